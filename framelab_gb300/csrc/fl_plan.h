@@ -223,6 +223,10 @@ inline int fl_plan_refl(const fl_plan* p)
 // voxel (x, y, z < nz/2) is at z*nx*ny + 16*((y/4)*(nx/4) + x/4) + 4*(y%4) +
 // x%4, so one 128-byte line holds a 4 x 4 patch of pairs (the gathers of a
 // warp's neighbouring rays share lines whatever the ray direction).
+// A reflection form's folded volume holds orbits instead: the eight images of
+// voxel (x < nx/2, y < ny/2, z < nz/2) under the flips of x, y and z side by
+// side, (voxel, z mirror) pairs ordered by (flip y, flip x), at 8 times
+// orbit_index (matched_dev.cuh: 2 x 2 tiles of orbits).
 // For other plans both layouts are the standard ones.
 enum {
     FL_LAY_X_FOLDED = 1,   // the volume operand is z-folded

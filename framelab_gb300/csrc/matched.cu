@@ -166,8 +166,17 @@ k_fwd_oct(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restri
 // (refl_image, rows ib and nb-1-ib), all with the walked ray's c_r. yfold
 // writes the backprojection's input layout for these plans (two planes,
 // ReflGeom; k_weight_packed_refl).
+// Bound: the L1 data pipe (86 % of its wavefront peak at 256^3, issue 54 %).
+// With one 8-byte gather per image from a volume of tiled pairs it was bound
+// there too (92 %, eight requests a step): 6.89 ms at 256^3 / 360 views,
+// 111.2 ms at 512^3 / 720. The orbit layout answers a step with one 32-byte
+// load (two for NR = 4): 5.86 and 92.9 ms with the orbits in 2 x 2 tiles
+// (row by row 6.70 / 103.5, two or four z planes per line 7.3 / 112 and 9.4 /
+// 146; as two 16-byte loads each 7.53 / 119). 7 (NR = 4) and 9 (NR = 2) blocks
+// per SM against 6 and 8: 5.83 / 90.7; lanes in 2 x 2 quads: 5.66 / 87.7.
+// Half turn, 90 views at 256^3: 2.26 -> 2.18 ms.
 template <typename TX, typename TY, int NR>
-__global__ void __launch_bounds__(128, NR == 4 ? 6 : 8)
+__global__ void __launch_bounds__(128, NR == 4 ? 7 : 9)
 k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
            const float* __restrict__ colr, const RowEntry* __restrict__ row, int nx, int ny,
            int nz, int na, int nb, int nv, long long nper, float scale, int cr_power,
@@ -175,9 +184,13 @@ k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
 {
     if (skip && *skip) return;
     const ReflGeom g = refl_geom(NR, nv, na, nb);
-    const int ia = blockIdx.x * blockDim.x + threadIdx.x;
+    // four consecutive lanes take 2 x 2 rays (blockDim.x and .y are even): the
+    // L1 serves a warp's 32-byte loads four lanes at a time
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, hbx = blockDim.x >> 1;
+    const int quad = tid >> 2, qrow = quad / hbx;
+    const int ia = blockIdx.x * blockDim.x + 2 * (quad - qrow * hbx) + (tid & 1);
     const int sl = blockIdx.y;                      // < g.slots
-    const int ib = blockIdx.z * blockDim.y + threadIdx.y;
+    const int ib = blockIdx.z * blockDim.y + 2 * qrow + ((tid >> 1) & 1);
     if (ia >= na || ib >= g.nbh) return;
     int v, vt, a, stride;
     long long off;
@@ -458,6 +471,41 @@ __global__ void k_fold(const T* __restrict__ src, T* __restrict__ dst, long long
         } else {
             const T a = src[lo], b = src[hi];
             dst[base + 2 * r] = a; dst[base + 2 * r + 1] = b;
+        }
+    }
+}
+
+// Fold / unfold of a reflection form's volume (one frame): orbit r (fl_plan.h)
+// holds the eight images of voxel (x < nx/2, y < ny/2, z < nz/2) under the
+// flips of x, y and z.
+template <typename T>
+__global__ void k_fold_orbit(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny,
+                             int nz, long long norbits, int unfold)
+{
+    const long long nn = (long long)nx * ny;
+    const int hx = nx >> 1, hxy = hx * (ny >> 1);
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < norbits;
+         r += (long long)gridDim.x * blockDim.x) {
+        const int z = (int)(r / hxy), rem = (int)(r - (long long)z * hxy);
+        const int y = rem / hx, x = rem - y * hx;
+        const long long q = 8 * (long long)orbit_index(x, y, z * hxy, hx);
+        struct alignas(4 * sizeof(T)) Half { T v[4]; } o[2];
+        if (unfold) {
+            o[0] = reinterpret_cast<const Half*>(src + q)[0];
+            o[1] = reinterpret_cast<const Half*>(src + q)[1];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const long long xy = (long long)(c & 2 ? ny - 1 - y : y) * nx + (c & 1 ? nx - 1 - x : x);
+            const long long lo = z * nn + xy, hi = (nz - 1 - z) * nn + xy;
+            T& a = o[c >> 1].v[2 * (c & 1)];
+            T& b = o[c >> 1].v[2 * (c & 1) + 1];
+            if (unfold) { dst[lo] = a; dst[hi] = b; }
+            else { a = src[lo]; b = src[hi]; }
+        }
+        if (!unfold) {
+            reinterpret_cast<Half*>(dst + q)[0] = o[0];
+            reinterpret_cast<Half*>(dst + q)[1] = o[1];
         }
     }
 }
@@ -1147,8 +1195,8 @@ __device__ __forceinline__ void adj_rows_refl(float2 (&P)[NR][TZ], float2 (&Q)[N
 // reflected slot j (view j nv/NR - w, column na-1-a) into D_{j-k}; a weight of
 // D_k, turn slot j into D_{k+j} and reflected slot j into C_{j-k}. One weight
 // thus feeds 4 NR (voxel, ray) pairs. yw is the packed input of
-// k_weight_packed_refl / k_fwd_refl (two planes); X the tiled folded volume
-// (xfold) or the standard one.
+// k_weight_packed_refl / k_fwd_refl (two planes); X the folded volume's
+// orbits (xfold) or the standard one.
 // View chunks: the walked views w0 .. w1 only. A launch that is not the
 // first continues the sums it finds in X (FP32, either layout) and one that
 // is not the last leaves them there, so a sequence of launches over
@@ -1211,7 +1259,7 @@ k_adj_refl(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
                     const float* Xf = (const float*)X;
                     float2 a;
                     if (xfold) {
-                        a = Store<float>::ld2(Xf + 2 * tiled_pair(qx, qy, zl, nx >> 2));
+                        a = Store<float>::ld2(Xf + orbit_pair(qx, qy, z0 + k, nx, ny));
                     } else {
                         const long long c = (long long)qy * nx + qx;
                         a = make_float2(Xf[zl + c], Xf[(long long)(nz - 1 - z0 - k) * nxy + c]);
@@ -1321,9 +1369,8 @@ k_adj_refl(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
                 } else {
                     a = Q[j - NR][k]; qx = dxs[j - NR]; qy = dys[j - NR];
                 }
-                if (xfold) {                  // the tiled folded volume
-                    const long long t = tiled_pair(qx, qy, (int)zl, nx >> 2);
-                    Store<TX>::st2(X + 2 * t, a.x, a.y);
+                if (xfold) {                  // the folded volume's orbits
+                    Store<TX>::st2(X + orbit_pair(qx, qy, z0 + k, nx, ny), a.x, a.y);
                 } else {
                     const long long c = (long long)qy * nx + qx;
                     Store<TX>::st(X + zl + c, a.x);
@@ -1734,7 +1781,10 @@ void launch_fold(fl_plan* p, const void* src, void* dst, int unfold, cudaStream_
     const long long nxy = (long long)s.nx * s.ny;
     const long long npf = nxy * (s.nz / 2), np = npf * s.nt;
     unsigned g = (unsigned)std::min<long long>((np + 255) / 256, 16LL * 152);
-    if (p->rot)                 // half- or quarter-turn plan: tiled (one frame)
+    if (fl_plan_refl(p))        // reflection form: orbits of eight (one frame)
+        k_fold_orbit<T><<<(unsigned)std::min<long long>((np / 4 + 255) / 256, 16LL * 152), 256, 0,
+                          st>>>((const T*)src, (T*)dst, s.nx, s.ny, s.nz, npf / 4, unfold);
+    else if (p->rot)            // half- or quarter-turn plan: tiled (one frame)
         k_fold_tiled<T><<<g, 256, 0, st>>>((const T*)src, (T*)dst, s.nx, s.ny, s.nz, npf,
                                            unfold);
     else

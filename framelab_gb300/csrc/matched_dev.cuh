@@ -411,6 +411,56 @@ __device__ __forceinline__ void walk_oct(const TX* __restrict__ x, const ColEntr
     for (int j = 0; j < 4; j++) acc[j] = b.acc[j];
 }
 
+// Orbit index of voxel (x, y, z) in the folded volume of a reflection form
+// (fl_plan.h), x < hx = nx/2, y < hy = ny/2, zb = z hx hy: the voxel's eight
+// images under the flips of x, y and z lie side by side at 8 times it, as
+// four (voxel, z mirror) pairs ordered by (flip y, flip x). Tiles of 2 x 2
+// orbits: one 128-byte line of FP32 holds a 2 x 2 patch, so neighbouring rays'
+// orbits share lines whatever the ray direction (hx and hy are even).
+__device__ __forceinline__ int orbit_index(int x, int y, int zb, int hx)
+{
+    return zb + (y & ~1) * hx + ((y & 1) << 1) + 2 * x - (x & 1);
+}
+
+// Element of the folded volume where the (voxel, mirror) pair of any (x, y) and
+// z < nz/2 starts.
+__device__ __forceinline__ int orbit_pair(int x, int y, int z, int nx, int ny)
+{
+    const int hx = nx >> 1, hy = ny >> 1;
+    const int q = orbit_index(min(x, nx - 1 - x), min(y, ny - 1 - y), z * hx * hy, hx);
+    return 8 * q + (y >= hy ? 4 : 0) + (x >= hx ? 2 : 0);   // < 2^31 (plan creation)
+}
+
+// The 8 values of one orbit (one 32- or 16-byte load), as (voxel, mirror) pairs.
+template <typename T>
+__device__ __forceinline__ void ld_orbit(const T* __restrict__ p, float2 (&v)[4]);
+template <>
+__device__ __forceinline__ void ld_orbit<float>(const float* __restrict__ p, float2 (&v)[4])
+{
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y),
+          "=f"(v[3].x), "=f"(v[3].y)
+        : "l"(p));
+}
+template <>
+__device__ __forceinline__ void ld_orbit<__half>(const __half* __restrict__ p, float2 (&v)[4])
+{
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+}
+template <>
+__device__ __forceinline__ void ld_orbit<__nv_bfloat16>(const __nv_bfloat16* __restrict__ p,
+                                                        float2 (&v)[4])
+{
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        v[k] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
+}
+
 // The z-mirror walk of a reflection form (fl_plan.h): NR = 4, the quarter
 // turns and the reflection (square grid); NR = 2, the half turn and the
 // reflection. Per step the folded pairs of the voxel's 2 NR images g_k =
@@ -418,49 +468,72 @@ __device__ __forceinline__ void walk_oct(const TX* __restrict__ x, const ColEntr
 // ny-1-y), R (x, y) = (n-1-y, x), R^2 (x, y) = (nx-1-x, ny-1-y); R M (x, y) =
 // (y, x). acc[k] gets the (voxel, mirror) sums of image k, the sums of the ray
 // g_k takes the walked ray to.
+//
+// The images are the flips of (x, y) and, for NR = 4, the flips of (y, x): the
+// orbits of the voxel's quadrant position (xx, yy) and of (yy, xx), one vector
+// load each, whatever the images' order. Which of an orbit's pairs is which
+// image depends on the quadrant the ray is in, so the sums are kept by
+// the pairs' places and exchanged when the ray crosses the middle of x or y (at
+// most once each). Every image's sum adds the same terms in the same order as
+// with one gather per image.
 template <typename TX, int NR>
 struct ReflBody {
     const TX* __restrict__ x;
     long long xlen;
-    int nx, ny, nxy, nx4;
-    float2 acc[2 * NR], xv[2 * NR];
-    __device__ __forceinline__ void load(int jx, int jy, int jz, float2 (&o)[2 * NR]) const
+    int nx, ny, hx, hy, hxy;
+    int flips = 0;                           // of the current voxel (bit 0 x, bit 1 y)
+    float2 A[4], B[4], va[4], vb[4];         // sums and values of the two orbits
+    __device__ __forceinline__ void load(int jx, int jy, int jz, float2 (&a)[4],
+                                         float2 (&b)[4]) const
     {
-        const int zb = jz * nxy, pi2 = 2 * zb + nxy - 1;  // q -> pi2 - q: the turn by pi
-        int q[2 * NR];
+        const int xx = min(jx, nx - 1 - jx), yy = min(jy, ny - 1 - jy), zb = jz * hxy;
+        const int q = orbit_index(xx, yy, zb, hx);
+        if (FL_IN(8 * (long long)q + 7, xlen)) ld_orbit<TX>(x + 8 * (long long)q, a);
         if (NR == 4) {
-            q[0] = tiled_pair(jx, jy, zb, nx4);
-            q[1] = tiled_pair(nx - 1 - jy, jx, zb, nx4);
-            q[4] = tiled_pair(jx, ny - 1 - jy, zb, nx4);
-            q[5] = tiled_pair(jy, jx, zb, nx4);
-            q[2] = pi2 - q[0];
-            q[3] = pi2 - q[1];
-            q[6] = pi2 - q[4];
-            q[7] = pi2 - q[5];
-        } else {
-            q[0] = tiled_pair(jx, jy, zb, nx4);
-            q[2] = tiled_pair(jx, ny - 1 - jy, zb, nx4);
-            q[1] = pi2 - q[0];
-            q[3] = pi2 - q[2];
-        }
-#pragma unroll
-        for (int j = 0; j < 2 * NR; j++) {
-            o[j] = make_float2(0.0f, 0.0f);
-            if (FL_IN(2 * (long long)q[j] + 1, xlen)) o[j] = Store<TX>::ld2(x + 2 * (long long)q[j]);
+            const int t = orbit_index(yy, xx, zb, hx);
+            if (FL_IN(8 * (long long)t + 7, xlen)) ld_orbit<TX>(x + 8 * (long long)t, b);
         }
     }
-    __device__ __forceinline__ void at(int jx, int jy, int jz) { load(jx, jy, jz, xv); }
+    // the sums follow the voxel into the quadrant of flips f (bit 0 x, bit 1 y)
+    __device__ __forceinline__ void quadrant(int f)
+    {
+        const int d = f ^ flips;
+        if (!d) return;
+        // exchanged through memory by a run-time index: swaps of the registers
+        // themselves made the compiler spill inside the walk
+        float2 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) t[j] = A[j];
+#pragma unroll
+        for (int j = 0; j < 4; j++) A[j] = t[j ^ d];
+        if (NR == 4) {
+            const int e = (d >> 1) | ((d & 1) << 1);    // (y, x): the flips trade places
+#pragma unroll
+            for (int j = 0; j < 4; j++) t[j] = B[j];
+#pragma unroll
+            for (int j = 0; j < 4; j++) B[j] = t[j ^ e];
+        }
+        flips = f;
+    }
+    __device__ __forceinline__ int flips_of(int jx, int jy) const
+    {
+        return (jx >= hx ? 1 : 0) | (jy >= hy ? 2 : 0);
+    }
+    __device__ __forceinline__ void at(int jx, int jy, int jz)
+    {
+        load(jx, jy, jz, va, vb);
+        quadrant(flips_of(jx, jy));
+    }
     __device__ __forceinline__ void take(float seg, bool more, int jx, int jy, int jz)
     {
-        float2 xn[2 * NR];
+        const float2 w = make_float2(seg, seg);
 #pragma unroll
-        for (int j = 0; j < 2 * NR; j++) xn[j] = make_float2(0.0f, 0.0f);
-        if (more) load(jx, jy, jz, xn);
-#pragma unroll
-        for (int j = 0; j < 2 * NR; j++) {
-            acc[j] = __ffma2_rn(make_float2(seg, seg), xv[j], acc[j]);
-            xv[j] = xn[j];
+        for (int j = 0; j < 4; j++) {
+            A[j] = __ffma2_rn(w, va[j], A[j]);
+            if (NR == 4) B[j] = __ffma2_rn(w, vb[j], B[j]);
         }
+        if (more) load(jx, jy, jz, va, vb);
+        if (more) quadrant(flips_of(jx, jy));
     }
 };
 
@@ -470,12 +543,21 @@ __device__ __forceinline__ void walk_refl(const TX* __restrict__ x, const ColEnt
                                           float2 (&acc)[2 * NR], long long xlen)
 {
     ReflBody<TX, NR> b;
-    b.x = x; b.xlen = xlen; b.nx = nx; b.ny = ny; b.nxy = nx * ny; b.nx4 = nx >> 2;
+    b.x = x; b.xlen = xlen; b.nx = nx; b.ny = ny;
+    b.hx = nx >> 1; b.hy = ny >> 1; b.hxy = b.hx * b.hy;
 #pragma unroll
-    for (int j = 0; j < 2 * NR; j++) { b.acc[j] = make_float2(0.0f, 0.0f); b.xv[j] = b.acc[j]; }
+    for (int j = 0; j < 4; j++)
+        b.A[j] = b.B[j] = b.va[j] = b.vb[j] = make_float2(0.0f, 0.0f);
     if (__ldg(&pZ->ih) < 0.0f) seg_walk<true>(ce, pZ, nx, ny, nz / 2, b);
-#pragma unroll
-    for (int j = 0; j < 2 * NR; j++) acc[j] = b.acc[j];
+    b.quadrant(0);                           // A, B by the images' own flips
+    if (NR == 4) {
+        acc[0] = b.A[0]; acc[2 % (2 * NR)] = b.A[3];          // I, R^2
+        acc[4 % (2 * NR)] = b.A[2]; acc[6 % (2 * NR)] = b.A[1];   // M, R^2 M
+        acc[1] = b.B[1]; acc[3] = b.B[2];                     // R, R^3
+        acc[5 % (2 * NR)] = b.B[0]; acc[7 % (2 * NR)] = b.B[3];   // R M, R^3 M
+    } else {
+        acc[0] = b.A[0]; acc[1] = b.A[3]; acc[2] = b.A[2]; acc[3] = b.A[1];
+    }
 }
 
 // Views and input layout of a reflection form (fl_plan.h). The walked views
