@@ -214,9 +214,9 @@ k_batch_weight(float* __restrict__ YW, const float* __restrict__ Y,
         const int NR = b.refl;
         const FanReflGeom g = fan_refl_geom(NR, b.nv, b.na);
         const int s = r / b.na, ia = r - s * b.na;
-        int v, vt, a, stride;
+        int v, vt, a;
         long long off;
-        if (s >= g.slots || !refl_slot(g, s, ia, v, vt, a, off, stride)) return;
+        if (s >= g.slots || !refl_slot(g, s, ia, v, vt, a, off)) return;
         const float cr = ray_cr(b.scale, b.colr[(long long)vt * b.na + a], 0.0f);
         for (int k = 0; k < 2 * NR; k++) {
             long long vk; int ak;

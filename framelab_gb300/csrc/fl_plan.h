@@ -122,9 +122,9 @@ struct fl_plan {
     // kernels; 0 keeps each kernel's built-in shape (set by fl_plan_autotune;
     // every thread's result is independent of the shape)
     int fwd_bx, fwd_by, adj_bx, adj_by;
-    // voxels per thread of the reflection backprojection (1 or 2; 0 = 2) and
-    // its row loop: 1 or 2 rows per iteration, 3 one pass over the run's rows
-    // (runs of 2; 0 = 1)
+    // reflection backprojection: columns per side of a warp's block (1 or 2; 0
+    // = fl_plan_adj_run's choice), and FL_TUNE_ADJ_ROWS (kept for callers; its
+    // row loop has one form)
     int adj_run, adj_rows;
     // launches over consecutive view chunks of the reflection backprojection
     // (FP32 output; 0 or 1: one launch), and the diagonal columns'
@@ -244,9 +244,14 @@ int fl_plan_fan_block(const fl_plan* p);
 // View groups of a fan plan's turn and reflection backprojections (8 or 16):
 // the plan's setting (FL_TUNE_FAN_GROUPS), else 8.
 int fl_plan_fan_groups(const fl_plan* p);
-// View chunks of a cone plan's reflection backprojection: the plan's setting
-// (FL_TUNE_ADJ_CHUNKS) where the output is FP32, else 1.
+// View chunks of a cone plan's reflection backprojection where the output is
+// FP32: the plan's setting (FL_TUNE_ADJ_CHUNKS), else one per half gigabyte of
+// packed input; otherwise 1.
 int fl_plan_adj_chunks(const fl_plan* p, bool f32_out);
+// Columns per side of the block a warp of the reflection backprojection owns
+// (1 or 2): the plan's setting (FL_TUNE_ADJ_RUN), else 2 once there are ten
+// warps of 2 x 2 columns per SM.
+int fl_plan_adj_run(const fl_plan* p);
 
 // The fan forward's transposed copy of x by TMA (fan_tma.cu): false, with
 // nothing launched, where the plan, the input address or the row sizes do
@@ -276,6 +281,9 @@ int fl_matched_adjoint_w(fl_plan* p, const float* yw, void* x, int xt, const int
 // the same with the input in FP32 or (cone plans) FP16, wt = FL_F32 / FL_F16
 int fl_matched_adjoint_wt(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
                           int layout, cudaStream_t st);
+// the reflection forms' kernels of it (refl_adjoint.cu)
+void fl_matched_adjoint_refl(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
+                             int xfold, cudaStream_t st);
 // volume (all frames) to the z-folded layout, or back with unfold = 1
 int fl_matched_fold(fl_plan* p, const void* src, void* dst, int dtype, int unfold,
                     cudaStream_t st);

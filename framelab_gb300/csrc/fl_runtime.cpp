@@ -410,7 +410,7 @@ extern "C" int fl_plan_query(const fl_plan* p, int option, int* value)
         return fl_set_error(FL_OK, "");
     }
     if (option == FL_TUNE_ADJ_RUN) {
-        *value = p->adj_run == 1 ? 1 : 2;
+        *value = fl_plan_refl(p) && p->s.ndim == 3 ? fl_plan_adj_run(p) : (p->adj_run == 1 ? 1 : 2);
         return fl_set_error(FL_OK, "");
     }
     if (option == FL_TUNE_ADJ_ROWS) {

@@ -192,31 +192,34 @@ k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
     const int sl = blockIdx.y;                      // < g.slots
     const int ib = blockIdx.z * blockDim.y + 2 * qrow + ((tid >> 1) & 1);
     if (ia >= na || ib >= g.nbh) return;
-    int v, vt, a, stride;
+    int v, vt, a;
     long long off;
-    if (!refl_slot(g, sl, ia, v, vt, a, off, stride)) return;
+    if (!refl_slot(g, sl, ia, v, vt, a, off)) return;
     const ColEntry* ce = col + (long long)vt * na + a;
     const RowEntry* re = row + (long long)vt * nb + ib;
     float2 acc[2 * NR];
     walk_refl<TX, NR>(X, ce, &re->z, nx, ny, nz, acc, nper);
     const float cr = ray_cr(scale, colr[(long long)vt * na + a], __ldg(&re->dz2));
     const float xs = xscale ? *xscale : 1.0f;
+    float o[2][2 * NR];                 // the orbit's two planes of 2 NR values
 #pragma unroll
     for (int k = 0; k < 2 * NR; k++) {
         float o0 = acc[k].x, o1 = acc[k].y;
         if (xscale) { o0 *= xs; o1 *= xs; }
         o0 = cr * o0; o1 = cr * o1;
         if (cr_power == 2) { o0 = cr * o0; o1 = cr * o1; }
-        if (yfold) {                    // the orbit's two planes of 2 NR values
-            Store<TY>::st2(y + (k < NR ? 0 : g.plane) + off +
-                               (long long)g.vpr * ((long long)ib * stride + ia) + 2 * (k % NR),
-                           o0, o1);
-        } else {
+        o[k / NR][2 * (k % NR)] = o0; o[k / NR][2 * (k % NR) + 1] = o1;
+        if (!yfold) {
             long long vk; int ak;
             refl_image<NR>(k, v, a, na, nv, vk, ak);
             Store<TY>::st(y + (vk * nb + ib) * na + ak, o0);
             Store<TY>::st(y + (vk * nb + (nb - 1 - ib)) * na + ak, o1);
         }
+    }
+    if (yfold) {
+        TY* at = y + off + (long long)g.vpr * ((long long)ia * g.nbh + ib);
+        st_out<TY, 2 * NR>(at, o[0]);
+        st_out<TY, 2 * NR>(at + g.plane, o[1]);
     }
 }
 
@@ -384,32 +387,33 @@ __global__ void k_weight_packed(float* __restrict__ yw, const TY* __restrict__ y
 // Packed yw of a reflection form: for each walked ray (refl_slot) and row ib
 // < nb/2 the 4 NR values c_r y of its images (refl_image, rows ib and
 // nb-1-ib), with c_r of the walked ray, in the two planes of ReflGeom.
+// A block takes 32 columns x 8 rows: the reads run along the columns, and the
+// eight rows of a column make 256 consecutive bytes of each plane.
 template <typename TY, int NR>
-__global__ void k_weight_packed_refl(float* __restrict__ yw, const TY* __restrict__ y,
-                                     const float* __restrict__ colr,
-                                     const RowEntry* __restrict__ row, int na, int nb, int nv,
-                                     long long npack, float scale)
+__global__ void __launch_bounds__(256)
+k_weight_packed_refl(float* __restrict__ yw, const TY* __restrict__ y,
+                     const float* __restrict__ colr, const RowEntry* __restrict__ row, int na,
+                     int nb, int nv, float scale)
 {
-    long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= npack) return;                         // npack = slots * nb/2 * na
     const ReflGeom g = refl_geom(NR, nv, na, nb);
-    const int ia = (int)(r % na);
-    const long long q = r / na;
-    const int ib = (int)(q % g.nbh);
-    const int sl = (int)(q / g.nbh);
-    int v, vt, a, stride;
+    const int ia = blockIdx.x * 32 + (threadIdx.x & 31);
+    const int ib = blockIdx.y * 8 + (threadIdx.x >> 5), sl = blockIdx.z;
+    if (ia >= na || ib >= g.nbh) return;
+    int v, vt, a;
     long long off;
-    if (!refl_slot(g, sl, ia, v, vt, a, off, stride)) return;
+    if (!refl_slot(g, sl, ia, v, vt, a, off)) return;
     const float cr = ray_cr(scale, colr[(long long)vt * na + a], row[(long long)vt * nb + ib].dz2);
-    const long long at = off + (long long)g.vpr * ((long long)ib * stride + ia);
+    float o[2][2 * NR];
 #pragma unroll
     for (int k = 0; k < 2 * NR; k++) {
         long long vk; int ak;
         refl_image<NR>(k, v, a, na, nv, vk, ak);
-        const float p0 = Store<TY>::ld_plain(y + (vk * nb + ib) * na + ak);
-        const float p1 = Store<TY>::ld_plain(y + (vk * nb + (nb - 1 - ib)) * na + ak);
-        Store<float>::st2(yw + (k < NR ? 0 : g.plane) + at + 2 * (k % NR), cr * p0, cr * p1);
+        o[k / NR][2 * (k % NR)] = cr * Store<TY>::ld_plain(y + (vk * nb + ib) * na + ak);
+        o[k / NR][2 * (k % NR) + 1] = cr * Store<TY>::ld_plain(y + (vk * nb + (nb - 1 - ib)) * na + ak);
     }
+    float* at = yw + off + (long long)g.vpr * ((long long)ia * g.nbh + ib);
+    st_out<float, 2 * NR>(at, o[0]);
+    st_out<float, 2 * NR>(at + g.plane, o[1]);
 }
 
 // Packed yw of a fan turn plan (G = 2 or 4): for r = (iv < nv/G, ia) the G
@@ -441,9 +445,9 @@ __global__ void k_weight_fan_refl(float* __restrict__ yw, const TY* __restrict__
     if (r >= nslot) return;                         // nslot = slots * na
     const FanReflGeom g = fan_refl_geom(NR, nv, na);
     const int sl = (int)(r / na), ia = (int)(r - (long long)sl * na);
-    int v, vt, a, stride;
+    int v, vt, a;
     long long off;
-    if (!refl_slot(g, sl, ia, v, vt, a, off, stride)) return;
+    if (!refl_slot(g, sl, ia, v, vt, a, off)) return;
     const float cr = ray_cr(scale, colr[(long long)vt * na + a], 0.0f);
 #pragma unroll
     for (int k = 0; k < 2 * NR; k++) {
@@ -622,69 +626,6 @@ k_adj_fan_turn(TX* __restrict__ X, const float* __restrict__ ywp,
 // with w_rV evaluated exactly as in the forward walk. The TZ accumulators are
 // registers (k is a compile-time index).
 // ---------------------------------------------------------------------------
-// The backprojection input (pre-weighted sinogram) is FP32, or FP16 in the
-// mixed CGLS form. ld_in<TW, N> reads N consecutive values of one orbit from
-// an address aligned to N elements, as one vector load, and widens them.
-template <typename TW, int N>
-__device__ __forceinline__ void ld_in(const TW* __restrict__ p, float (&v)[N]);
-
-template <>
-__device__ __forceinline__ void ld_in<float, 1>(const float* __restrict__ p, float (&v)[1])
-{
-    v[0] = __ldg(p);
-}
-template <>
-__device__ __forceinline__ void ld_in<float, 2>(const float* __restrict__ p, float (&v)[2])
-{
-    const float2 u = __ldg(reinterpret_cast<const float2*>(p));
-    v[0] = u.x; v[1] = u.y;
-}
-template <>
-__device__ __forceinline__ void ld_in<float, 4>(const float* __restrict__ p, float (&v)[4])
-{
-    const float4 u = __ldg(reinterpret_cast<const float4*>(p));
-    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
-}
-template <>
-__device__ __forceinline__ void ld_in<float, 8>(const float* __restrict__ p, float (&v)[8])
-{
-    // one 32-byte load (sm_100 and later; orbits are 32-byte aligned)
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
-          "=f"(v[7])
-        : "l"(p));
-}
-template <>
-__device__ __forceinline__ void ld_in<__half, 1>(const __half* __restrict__ p, float (&v)[1])
-{
-    v[0] = __half2float(__ldg(p));
-}
-template <>
-__device__ __forceinline__ void ld_in<__half, 2>(const __half* __restrict__ p, float (&v)[2])
-{
-    const float2 a = __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
-    v[0] = a.x; v[1] = a.y;
-}
-template <>
-__device__ __forceinline__ void ld_in<__half, 4>(const __half* __restrict__ p, float (&v)[4])
-{
-    const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
-    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-template <>
-__device__ __forceinline__ void ld_in<__half, 8>(const __half* __restrict__ p, float (&v)[8])
-{
-    const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
-    const unsigned w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
-        v[2 * k] = a.x; v[2 * k + 1] = a.y;
-    }
-}
-
 // Candidate rays of one detector column for the TZ voxels of a run. MODE +1:
 // the run lies above the source plane, so every ray that reaches it rises
 // (A_z increasing in k); MODE -1: below, every such ray falls; MODE 0: the run
@@ -1060,326 +1001,6 @@ k_adj_oct(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __restr
         }
 }
 
-// Reflection forms of adj_rows_oct: every weight multiplies the row pairs of
-// the walked ray's 2 NR images into the sums P[j] (turn images) and Q[j]
-// (reflected images); yt / yr hold them side by side (2 NR values per row and
-// column in each plane, rows rs columns apart), so each is one vector load
-// whose lanes read neighbouring columns' orbits. RU rows per iteration: RU =
-// 2 issues the loads of two rows before either's arithmetic (more loads in
-// flight per thread); RU = 0 loads each row of the run once for all its
-// voxels; the rows are added in order either way.
-template <int MODE, int TZ, int RU, typename TW, int NR>
-__device__ __forceinline__ void adj_rows_refl(float2 (&P)[NR][TZ], float2 (&Q)[NR][TZ], int nk,
-                                              int z0, float l, float h, float e1, float e2,
-                                              float s1, float s2,
-                                              const AxisEntry* __restrict__ rv, float bh,
-                                              float be, const TW* __restrict__ yt,
-                                              const TW* __restrict__ yr, int rs, int nb)
-{
-    float mn = fminf(e1, e2), mx = fmaxf(e1, e2);
-    float lo_e = e1 - 0.02f, hi_e = e2 + s2 + 0.02f;
-    if constexpr (RU == 0) {
-        // the run's rows once: each row in the union of the voxels' windows
-        // is loaded once and adds to every voxel whose window holds it (the
-        // same terms in the same order as one pass per voxel)
-        int blo[TZ], bhi[TZ];
-        int ulo = nb, uhi = -1;
-#pragma unroll
-        for (int k = 0; k < TZ; k++) {
-            if (MODE < 0) {
-                blo[k] = max(__float2int_ru(lo_e), 0);
-                bhi[k] = min(__float2int_rd(hi_e), nb - 1);
-                lo_e += s1; hi_e += s2;
-            } else {
-                e1 += s1; e2 += s2;
-                const float mn1 = fminf(e1, e2), mx1 = fmaxf(e1, e2);
-                blo[k] = max(__float2int_ru(fminf(mn, mn1) - 0.02f), 0);
-                bhi[k] = min(__float2int_rd(fmaxf(mx, mx1) + 0.02f), nb - 1);
-                mn = mn1; mx = mx1;
-            }
-            if (k >= nk) { blo[k] = nb; bhi[k] = -1; }
-            ulo = min(ulo, blo[k]); uhi = max(uhi, bhi[k]);
-        }
-        for (int ib = ulo; ib <= uhi; ib++) {
-            if (!FL_IN(ib, nb)) continue;
-            const AxisEntry re = rv[ib];
-            float o[4 * NR];
-            ld_in<TW, 2 * NR>(yt + 2 * NR * (long long)ib * rs,
-                              *reinterpret_cast<float(*)[2 * NR]>(o));
-            ld_in<TW, 2 * NR>(yr + 2 * NR * (long long)ib * rs,
-                              *reinterpret_cast<float(*)[2 * NR]>(o + 2 * NR));
-            const float cb = __fsub_rn(re.c, be);
-            float az[TZ + 1];
-#pragma unroll
-            for (int k = 0; k <= TZ; k++)
-                az[k] = xrel(re, __fsub_rn((float)(z0 + k), re.kq), bh, cb);
-#pragma unroll
-            for (int k = 0; k < TZ; k++) {
-                if (ib < blo[k] || ib > bhi[k]) continue;
-                float l2, h2;
-                if (MODE < 0) { l2 = fmaxf(l, az[k + 1]); h2 = fminf(h, az[k]); }
-                else {
-                    l2 = fmaxf(l, fminf(az[k], az[k + 1]));
-                    h2 = fminf(h, fmaxf(az[k], az[k + 1]));
-                }
-                const float w = fmaxf(h2 - l2, 0.0f);
-                const float2 w2 = make_float2(w, w);
-#pragma unroll
-                for (int j = 0; j < NR; j++) {
-                    P[j][k] = __ffma2_rn(w2, make_float2(o[2 * j], o[2 * j + 1]), P[j][k]);
-                    Q[j][k] = __ffma2_rn(w2, make_float2(o[2 * NR + 2 * j], o[2 * NR + 2 * j + 1]),
-                                         Q[j][k]);
-                }
-            }
-        }
-        return;
-    }
-    constexpr int RN = RU > 0 ? RU : 1;          // rows per iteration below
-#pragma unroll
-    for (int k = 0; k < TZ; k++) {
-        if (k >= nk) break;
-        int blo, bhi;
-        if (MODE < 0) {
-            blo = max(__float2int_ru(lo_e), 0);
-            bhi = min(__float2int_rd(hi_e), nb - 1);
-            lo_e += s1; hi_e += s2;
-        } else {
-            e1 += s1; e2 += s2;
-            const float mn1 = fminf(e1, e2), mx1 = fmaxf(e1, e2);
-            blo = max(__float2int_ru(fminf(mn, mn1) - 0.02f), 0);
-            bhi = min(__float2int_rd(fmaxf(mx, mx1) + 0.02f), nb - 1);
-            mn = mn1; mx = mx1;
-        }
-        const float fk0 = (float)(z0 + k), fk1 = (float)(z0 + k + 1);
-        for (int ib = blo; ib <= bhi; ib += RN) {
-            AxisEntry re[RN];
-            float o[RN][4 * NR];
-            bool on[RN];
-#pragma unroll
-            for (int u = 0; u < RN; u++) {
-                on[u] = ib + u <= bhi && FL_IN(ib + u, nb);
-                const long long r = on[u] ? ib + u : min(max(ib, 0), nb - 1);   // one that exists
-                re[u] = rv[r];
-                ld_in<TW, 2 * NR>(yt + 2 * NR * r * rs, *reinterpret_cast<float(*)[2 * NR]>(o[u]));
-                ld_in<TW, 2 * NR>(yr + 2 * NR * r * rs,
-                                  *reinterpret_cast<float(*)[2 * NR]>(o[u] + 2 * NR));
-            }
-#pragma unroll
-            for (int u = 0; u < RN; u++) {
-                const float2 az = row_planes(re[u], fk0, fk1, bh, be);
-                float l2, h2;
-                if (MODE < 0) { l2 = fmaxf(l, az.y); h2 = fminf(h, az.x); }
-                else { l2 = fmaxf(l, fminf(az.x, az.y)); h2 = fminf(h, fmaxf(az.x, az.y)); }
-                if (!on[u]) continue;
-                const float w = fmaxf(h2 - l2, 0.0f);
-                const float2 w2 = make_float2(w, w);
-#pragma unroll
-                for (int j = 0; j < NR; j++) {
-                    P[j][k] = __ffma2_rn(w2, make_float2(o[u][2 * j], o[u][2 * j + 1]), P[j][k]);
-                    Q[j][k] = __ffma2_rn(
-                        w2, make_float2(o[u][2 * NR + 2 * j], o[u][2 * NR + 2 * j + 1]), Q[j][k]);
-                }
-            }
-        }
-    }
-}
-
-// Reflection + z-mirror backprojections (fl_plan::refl). NR = 4 (quarter
-// turns, nx == ny == n): one thread per voxel column V0 = (x, y) of the octant
-// x <= y < n/2; NR = 2 (half turn): of the quadrant x < nx/2, y < ny/2. With
-// S = R^(4/NR) the thread owns the images C_k = S^k V0 and D_k = S^k M V0 (k
-// < NR; for NR = 4 and x == y, D_k = C_{k+3} and only the C_k are visited),
-// a run of TZ voxels of the lower half and their mirrors; one frame. It
-// visits the walked views w = 0 .. ov (refl_view). In view w a weight of
-// column C_k multiplies turn slot j (view w + j nv/NR) into C_{k+j} and
-// reflected slot j (view j nv/NR - w, column na-1-a) into D_{j-k}; a weight of
-// D_k, turn slot j into D_{k+j} and reflected slot j into C_{j-k}. One weight
-// thus feeds 4 NR (voxel, ray) pairs. yw is the packed input of
-// k_weight_packed_refl / k_fwd_refl (two planes); X the folded volume's
-// orbits (xfold) or the standard one.
-// View chunks: the walked views w0 .. w1 only. A launch that is not the
-// first continues the sums it finds in X (FP32, either layout) and one that
-// is not the last leaves them there, so a sequence of launches over
-// consecutive chunks adds every term in the order one launch would: the bits
-// are the same. On the diagonal (NR = 4, x == y) P and Q are carried apart
-// between chunks, P in X and Q in dq (dq[((x * dqz + z) * NR + j)] for the
-// voxel pair at height z < nz/2), and combined by the last.
-template <typename TX, int TZ, int RU, typename TW, int NR>
-__global__ void __launch_bounds__(128, TZ == 1 ? (RU == 2 ? 6 : 8) : (RU == 1 ? 6 : 5))
-k_adj_refl(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __restrict__ col,
-           const AxisEntry* __restrict__ rowz, const ViewEntry* __restrict__ view, DetGrid G,
-           int nx, int ny, int nz, int na, int nb, int nv, float dz,
-           const int* __restrict__ skip, int xfold, int w0, int w1, int first, int last,
-           float2* __restrict__ dq, int dqz)
-{
-    if (skip && *skip) return;
-    const ReflGeom g = refl_geom(NR, nv, na, nb);
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;    // < nx / 2
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;    // < ny / 2
-    const int z0 = blockIdx.z * TZ;
-    const int nzw = nz / 2, hx = nx / 2, hy = ny / 2;
-    const int nk = min(TZ, nzw - z0);
-    if (ix >= hx || iy >= hy || (NR == 4 && ix > iy)) return;
-    const bool diag = NR == 4 && ix == iy;
-    // P: the sums the turn slots feed, Q: the reflected slots' (rotated one
-    // place per column, in opposite directions; exchanged between the C and
-    // the D columns)
-    float2 P[NR][TZ], Q[NR][TZ];
-#pragma unroll
-    for (int j = 0; j < NR; j++)
-#pragma unroll
-        for (int k = 0; k < TZ; k++) { P[j][k] = make_float2(0.0f, 0.0f); Q[j][k] = P[j][k]; }
-    const float inv_dv = 1.0f / G.dv;
-    const int nsteps = diag ? NR : 2 * NR;
-    // C_j = S^j V0 and D_j = S^j M V0 of the thread's column (the stores
-    // below; the loads of a chunk after the first)
-    const long long nxy = (long long)nx * ny;
-    int cx[NR], cy[NR], dxs[NR], dys[NR];
-    if (NR == 4) {
-        cx[0] = ix; cx[1 % NR] = nx - 1 - iy; cx[2 % NR] = nx - 1 - ix; cx[3 % NR] = iy;
-        cy[0] = iy; cy[1 % NR] = ix; cy[2 % NR] = ny - 1 - iy; cy[3 % NR] = ny - 1 - ix;
-        dxs[0] = ix; dxs[1 % NR] = iy; dxs[2 % NR] = nx - 1 - ix; dxs[3 % NR] = nx - 1 - iy;
-        dys[0] = ny - 1 - iy; dys[1 % NR] = ix; dys[2 % NR] = iy; dys[3 % NR] = ny - 1 - ix;
-    } else {
-        cx[0] = ix; cx[1 % NR] = nx - 1 - ix; cy[0] = iy; cy[1 % NR] = ny - 1 - iy;
-        dxs[0] = ix; dxs[1 % NR] = nx - 1 - ix; dys[0] = ny - 1 - iy; dys[1 % NR] = iy;
-    }
-    if (!first) {                                    // continue the chunk before
-#pragma unroll
-        for (int k = 0; k < TZ; k++)
-            if (k < nk) {
-                const int zl = (z0 + k) * (int)nxy;
-#pragma unroll
-                for (int j = 0; j < 2 * NR; j++) {
-                    if (diag && j >= NR) {
-                        Q[j - NR][k] = dq[((long long)ix * dqz + z0 + k) * NR + (j - NR)];
-                        continue;
-                    }
-                    const int qx = j < NR ? cx[j] : dxs[j - NR], qy = j < NR ? cy[j] : dys[j - NR];
-                    const float* Xf = (const float*)X;
-                    float2 a;
-                    if (xfold) {
-                        a = Store<float>::ld2(Xf + orbit_pair(qx, qy, z0 + k, nx, ny));
-                    } else {
-                        const long long c = (long long)qy * nx + qx;
-                        a = make_float2(Xf[zl + c], Xf[(long long)(nz - 1 - z0 - k) * nxy + c]);
-                    }
-                    if (j < NR) P[j][k] = a; else Q[j - NR][k] = a;
-                }
-            }
-    }
-    for (int w = w0; w <= min(w1, g.ov); w++) {
-        int vt, rs, alim;
-        long long base;
-        refl_view(g, w, vt, base, rs, alim);
-        const ViewEntry ve = view[vt];
-        const ColEntry* cv = col + (long long)vt * na;
-        const AxisEntry* rv = rowz + (long long)vt * nb;
-        const TW* yv = yw + base;
-        const float zr0 = (float)(z0 - nz / 2) * dz - ve.sz;
-        const float zr1 = (float)(z0 + nk - nz / 2) * dz - ve.sz;
-        const float tol = 1e-3f * dz;
-        const int mode = (zr1 <= -tol) ? -1 : 0;               // lower half: never above
-        int px = ix, py = iy;                                  // C_0
-#pragma unroll 1
-        for (int k = 0; k < nsteps; k++) {
-            if (k == NR) {                                     // the D columns: D_0 = M V0
-                px = ix; py = ny - 1 - iy;
-#pragma unroll
-                for (int j = 0; j < NR; j++)
-#pragma unroll
-                    for (int z = 0; z < TZ; z++) {
-                        const float2 t = P[j][z];
-                        P[j][z] = Q[j][z]; Q[j][z] = t;
-                    }
-            }
-            int alo, ahi; float dmin, dmax;
-            column_window(G, ve.c, ve.s, (float)(px - hx), (float)(py - hy), 1.0f, 1.0f, na, alo,
-                          ahi, dmin, dmax);
-            ahi = min(ahi, alim - 1);
-            for (int ia = alo; ia <= ahi; ia++) {
-                if (!FL_IN(ia, na)) continue;
-                const ColEntry ce = cv[ia];
-                float bh, be, l, hh;
-                if (!cone_column(ce, px, py, nx, ny, bh, be, l, hh)) continue;
-                // absolute parameters of the column's ends (row windows only)
-                const float r1 = __fdividef(1.0f, __fadd_rn(bh, l) + ve.ac);
-                const float r2 = __fdividef(1.0f, __fadd_rn(bh, hh) + ve.ac);
-                const float s1 = dz * r1 * inv_dv, s2 = dz * r2 * inv_dv;
-                const float e1 = (zr0 * r1 - G.v0) * inv_dv, e2 = (zr0 * r2 - G.v0) * inv_dv;
-                const TW* yt = yv + g.vpr * ia;
-                if (mode < 0)
-                    adj_rows_refl<-1, TZ, RU, TW, NR>(P, Q, nk, z0, l, hh, e1, e2, s1, s2, rv, bh,
-                                                      be, yt, yt + g.plane, rs, g.nbh);
-                else
-                    adj_rows_refl<0, TZ, RU, TW, NR>(P, Q, nk, z0, l, hh, e1, e2, s1, s2, rv, bh,
-                                                     be, yt, yt + g.plane, rs, g.nbh);
-            }
-            // next column S (px, py); P rotates back one place, Q forward one
-            if (NR == 4) {
-                const int t = px;
-                px = nx - 1 - py; py = t;
-            } else {
-                px = nx - 1 - px; py = ny - 1 - py;
-            }
-#pragma unroll
-            for (int z = 0; z < TZ; z++) {
-                const float2 a = P[0][z];
-#pragma unroll
-                for (int j = 0; j + 1 < NR; j++) P[j][z] = P[j + 1][z];
-                P[NR - 1][z] = a;
-                const float2 b = Q[NR - 1][z];
-#pragma unroll
-                for (int j = NR - 1; j > 0; j--) Q[j][z] = Q[j - 1][z];
-                Q[0][z] = b;
-            }
-        }
-        if (!diag) {                                           // C sums back into P
-#pragma unroll
-            for (int j = 0; j < NR; j++)
-#pragma unroll
-                for (int z = 0; z < TZ; z++) {
-                    const float2 t = P[j][z];
-                    P[j][z] = Q[j][z]; Q[j][z] = t;
-                }
-        }
-    }
-    // C_j = S^j V0 holds P[j] (and, on the diagonal of NR = 4, Q[j + 1], the
-    // sums of D_{j+1} = C_j; before the last chunk they stay apart, Q in dq);
-    // D_j = S^j M V0 holds Q[j]
-#pragma unroll
-    for (int k = 0; k < TZ; k++)
-        if (k < nk) {
-            const long long zl = (long long)(z0 + k) * nxy, zh = (long long)(nz - 1 - z0 - k) * nxy;
-#pragma unroll
-            for (int j = 0; j < 2 * NR; j++) {
-                if (diag && j >= NR) {
-                    if (!last) dq[((long long)ix * dqz + z0 + k) * NR + (j - NR)] = Q[j - NR][k];
-                    continue;
-                }
-                float2 a;
-                int qx, qy;
-                if (j < NR) {
-                    a = P[j][k];
-                    if (diag && last) {
-                        const float2 b = Q[(j + 1) % NR][k];
-                        a.x += b.x; a.y += b.y;
-                    }
-                    qx = cx[j]; qy = cy[j];
-                } else {
-                    a = Q[j - NR][k]; qx = dxs[j - NR]; qy = dys[j - NR];
-                }
-                if (xfold) {                  // the folded volume's orbits
-                    Store<TX>::st2(X + orbit_pair(qx, qy, z0 + k, nx, ny), a.x, a.y);
-                } else {
-                    const long long c = (long long)qy * nx + qx;
-                    Store<TX>::st(X + zl + c, a.x);
-                    Store<TX>::st(X + zh + c, a.y);
-                }
-            }
-        }
-}
-
 // MIRROR: yw is the folded sinogram; the runs cover the lower half z < nz/2
 // only (the walked rows' rays never reach the upper half) and each thread also
 // produces the mirrored run, into the folded volume when xfold is set.
@@ -1469,16 +1090,6 @@ k_adj_cone(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
         }
 }
 
-DetGrid det_grid(const fl_plan* p)
-{
-    DetGrid G;
-    G.kind = p->det_kind; G.u0 = p->u0; G.du = p->du; G.g0 = p->g0; G.dg = p->dg;
-    G.v0 = p->v0; G.dv = p->dv; G.SO = p->s.SO; G.SD = p->SD;
-    G.rdu = p->du != 0.0f ? 1.0f / p->du : 0.0f;
-    G.rdg = p->dg != 0.0f ? 1.0f / p->dg : 0.0f;
-    return G;
-}
-
 }  // namespace
 
 // Tunables of fan plans (fl_plan.h).
@@ -1494,8 +1105,13 @@ int fl_plan_fan_lanes(const fl_plan* p)
 
 int fl_plan_adj_chunks(const fl_plan* p, bool f32_out)
 {
-    if (!f32_out || p->adj_chunks < 2) return 1;
+    if (!f32_out || p->adj_chunks == 1 || p->s.ndim != 3 || !fl_plan_refl(p)) return 1;
     if (fl_plan_refl(p) == 4 && !p->d_dq) return 1;        // no room for the diagonal's sums
+    // by default half a gigabyte of packed input per launch: the blocks
+    // resident together then drift over fewer views than L2 holds (512^3, 720
+    // views, 2.3 GB: 188.3 ms a CGLS iteration in one launch, 184.9 in 4, 183.9
+    // in 8, 186.5 in 16; 256^3, 360 views, 0.3 GB: 12.82, 12.86 in 4, 13.1 in 8)
+    if (!p->adj_chunks) return (int)std::min<long long>(16, std::max<long long>(1, p->n_rays * 4 >> 29));
     return p->adj_chunks;
 }
 
@@ -1525,6 +1141,14 @@ int fl_plan_fan_block(const fl_plan* p)
 
 namespace {
 
+template <typename T>
+constexpr int dtype_of()
+{
+    return std::is_same<T, float>::value    ? FL_F32
+           : std::is_same<T, __half>::value ? FL_F16
+                                            : FL_BF16;
+}
+
 // The fan forward's transposed copy of its input (walk_fan), in the plan's
 // buffer (allocated with the plan: nothing is allocated here, so a forward
 // can be captured in a CUDA graph): by TMA where it applies, else by a
@@ -1533,10 +1157,7 @@ template <typename TX>
 const TX* fan_transposed(fl_plan* p, const void* x, cudaStream_t st)
 {
     const fl_scan& s = p->s;
-    const int dt = std::is_same<TX, float>::value    ? FL_F32
-                   : std::is_same<TX, __half>::value ? FL_F16
-                                                     : FL_BF16;
-    if (fl_fan_transpose_tma(p, x, dt, st)) return (const TX*)p->d_xt;   // fan_tma.cu
+    if (fl_fan_transpose_tma(p, x, dtype_of<TX>(), st)) return (const TX*)p->d_xt;   // fan_tma.cu
     const dim3 grid(fl_div_up(s.nx, 32), fl_div_up(s.ny, 32), s.nt);
     k_transpose_fan<TX><<<grid, dim3(32, 8), 0, st>>>((const TX*)x, (TX*)p->d_xt, s.nx, s.ny,
                                                       p->n_vox_frame);
@@ -1637,37 +1258,7 @@ void launch_adj_cone(fl_plan* p, const TW* yw, void* x, const int* skip, int xfo
         const int nzw = p->zmirror ? s.nz / 2 : s.nz;
         int zruns = (nzw + TZ - 1) / TZ;
         if (fl_plan_refl(p)) {
-            // runs of 2 voxels or of 1; one or two rows per iteration, or (runs
-            // of 2) one pass over the run's rows: fl_plan_autotune
-            const int NR = fl_plan_refl(p);
-            const int run = p->adj_run == 1 ? 1 : 2;
-            const int ru = p->adj_rows == 2 ? 2 : (p->adj_rows == 3 && run == 2 ? 0 : 1);
-            zruns = (nzw + run - 1) / run;
-            const dim3 ab = p->adj_bx ? dim3(p->adj_bx, p->adj_by) : dim3(8, 16);
-            dim3 grid(fl_div_up(s.nx / 2, ab.x), fl_div_up(s.ny / 2, ab.y), (unsigned)zruns);
-            // view chunks (fl_plan_adj_chunks): launches over consecutive
-            // walked views, so the blocks resident together read the same
-            // views' rows from L2; FP32 output only
-            const int nch = fl_plan_adj_chunks(p, std::is_same<TX, float>::value);
-            const int wper = (refl_geom(NR, s.nv, s.na, s.nb).ov + nch) / nch;
-#define FL_ADJ_REFL(TZ_, RU_, NR_)                                                             \
-    for (int c = 0; c < nch; c++)                                                             \
-        k_adj_refl<TX, TZ_, RU_, TW, NR_><<<grid, ab, 0, st>>>(                                 \
-            (TX*)x, yw, p->d_col, p->d_rowz, p->d_view, G, s.nx, s.ny, s.nz, s.na, s.nb, s.nv,   \
-            s.dz, skip, xfold, c * wper, c * wper + wper - 1, c == 0, c == nch - 1, p->d_dq,    \
-            s.nz / 2)
-#define FL_ADJ_REFL_NR(NR_)                                                                    \
-    do {                                                                                       \
-        if (run == 1 && ru == 1) FL_ADJ_REFL(1, 1, NR_);                                      \
-        else if (run == 1) FL_ADJ_REFL(1, 2, NR_);                                            \
-        else if (ru == 1) FL_ADJ_REFL(2, 1, NR_);                                             \
-        else if (ru == 2) FL_ADJ_REFL(2, 2, NR_);                                             \
-        else FL_ADJ_REFL(2, 0, NR_);                                                          \
-    } while (0)
-            if (NR == 4) FL_ADJ_REFL_NR(4);
-            else FL_ADJ_REFL_NR(2);
-#undef FL_ADJ_REFL_NR
-#undef FL_ADJ_REFL
+            fl_matched_adjoint_refl(p, yw, dtype_of<TW>(), x, dtype_of<TX>(), skip, xfold, st);
         } else if (p->zmirror && p->rot && p->rot4) {
             // runs of 2: the four columns' 16 accumulators keep 8 blocks per SM
             constexpr int TO = 2;
@@ -1816,19 +1407,16 @@ void launch_weight_packed_refl(fl_plan* p, const void* y, int yt, float* yw, cud
 {
     const fl_scan& s = p->s;
     const ReflGeom gm = refl_geom(NR, s.nv, s.na, s.nb);
-    const long long npk = (long long)gm.slots * gm.nbh * s.na;
-    const unsigned g = fl_div_up(npk, 256);
+    const dim3 g(fl_div_up(s.na, 32), fl_div_up(gm.nbh, 8), gm.slots);
     if (yt == FL_F32)
         k_weight_packed_refl<float, NR><<<g, 256, 0, st>>>(yw, (const float*)y, p->d_colr,
-                                                           p->d_row, s.na, s.nb, s.nv, npk,
-                                                           s.scale);
+                                                           p->d_row, s.na, s.nb, s.nv, s.scale);
     else if (yt == FL_F16)
         k_weight_packed_refl<__half, NR><<<g, 256, 0, st>>>(yw, (const __half*)y, p->d_colr,
-                                                            p->d_row, s.na, s.nb, s.nv, npk,
-                                                            s.scale);
+                                                            p->d_row, s.na, s.nb, s.nv, s.scale);
     else
         k_weight_packed_refl<__nv_bfloat16, NR><<<g, 256, 0, st>>>(
-            yw, (const __nv_bfloat16*)y, p->d_colr, p->d_row, s.na, s.nb, s.nv, npk, s.scale);
+            yw, (const __nv_bfloat16*)y, p->d_colr, p->d_row, s.na, s.nb, s.nv, s.scale);
 }
 
 template <int G>
@@ -1983,10 +1571,9 @@ int fl_matched_adjoint_wt(fl_plan* p, const void* yw, int wt, void* x, int xt, c
 // below is timed (CUDA events, one launch after one untimed) on the plan's own
 // geometry, with the plan's scratch as input and output, and the fastest kept
 // for the forward and for the backprojection.
-// * Cone plans: the 128-thread block shapes of both kernels, and for the
-//   reflection backprojection runs of 1 or 2 voxels per thread with 1 or 2
-//   rows per iteration or one pass over a run's rows. A thread's result does
-//   not depend on these, so neither do the projections.
+// * Cone plans: the 128-thread block shapes of both kernels, for the reflection
+//   backprojection warps of one or 2 x 2 columns and its view chunks instead. A
+//   voxel's sum does not depend on these, so neither do the projections.
 // * Fan plans: the parts per walked ray of the turn forward (1, 4, 16: the
 //   order of a ray's additions, within FP32 rounding) and the pixel block of
 //   the backprojections (1 or 2: the same bits).
@@ -2030,21 +1617,19 @@ extern "C" int fl_plan_autotune(fl_plan* p, void* stream, int32_t* shapes)
     };
     if (cone) {
         static const int cand[4][2] = {{8, 16}, {16, 8}, {32, 4}, {4, 32}};
-        // the reflection backprojection also tries voxel runs of 2 and 1 per
-        // thread with one or two rows per iteration, and runs of 2 in one pass
-        // over their rows (variant r: run, rows)
-        static const int var[5][2] = {{2, 1}, {1, 1}, {2, 2}, {1, 2}, {2, 3}};
-        const int nvar = fl_plan_refl(p) ? 5 : 1;
+        // the reflection backprojection has no block shape; it tries warps of
+        // 2 x 2 columns and of one (FL_TUNE_ADJ_RUN)
+        const bool refl = fl_plan_refl(p) != 0;
         for (int pass = 0; pass < 2 && !st; pass++) {
             const bool fwd = pass == 0;
             float best = 3.0e38f;
             int bi = 0, br = 0;
-            for (int c = 0; c < 4 && !st; c++)
-                for (int r = 0; r < (fwd ? 1 : nvar) && !st; r++) {
+            for (int c = 0; c < (!fwd && refl ? 1 : 4) && !st; c++)
+                for (int r = !fwd && refl ? 1 : 0; r < (!fwd && refl ? 3 : 1) && !st; r++) {
                     if (fwd) { p->fwd_bx = cand[c][0]; p->fwd_by = cand[c][1]; }
                     else {
                         p->adj_bx = cand[c][0]; p->adj_by = cand[c][1];
-                        p->adj_run = var[r][0]; p->adj_rows = var[r][1];
+                        p->adj_run = r;
                     }
                     float ms = 0.0f;
                     st = timed(fwd, ms);
@@ -2053,7 +1638,7 @@ extern "C" int fl_plan_autotune(fl_plan* p, void* stream, int32_t* shapes)
             if (fwd) { p->fwd_bx = cand[bi][0]; p->fwd_by = cand[bi][1]; }
             else {
                 p->adj_bx = cand[bi][0]; p->adj_by = cand[bi][1];
-                p->adj_run = var[br][0]; p->adj_rows = var[br][1];
+                p->adj_run = br;
             }
         }
         // then the view chunks of the reflection backprojection (FP32 output)
@@ -2070,8 +1655,7 @@ extern "C" int fl_plan_autotune(fl_plan* p, void* stream, int32_t* shapes)
             p->adj_chunks = chunks[bi];
         }
         if (st)
-            p->fwd_bx = p->fwd_by = p->adj_bx = p->adj_by = p->adj_run = p->adj_rows =
-                p->adj_chunks = 0;
+            p->fwd_bx = p->fwd_by = p->adj_bx = p->adj_by = p->adj_run = p->adj_chunks = 0;
     } else {
         static const int parts[3] = {1, 4, 16};
         const bool turn = fl_plan_turns(p) > 1;
@@ -2124,13 +1708,15 @@ int fl_matched_count(fl_plan* p, int32_t* counts, cudaStream_t st)
 // ---------------------------------------------------------------------------
 FL_OOB_ACCESSOR(fl_oob_matched)
 extern "C" unsigned long long fl_oob_batch(int reset);
+extern "C" unsigned long long fl_oob_refl(int reset);
 
 extern "C" int fl_debug_bounds(int64_t* violations, int reset)
 {
     if (!violations) return fl_set_error(FL_ERR_INVALID, "fl_debug_bounds: null argument");
 #ifdef FL_BOUNDS_CHECK
     FL_CUDA(cudaDeviceSynchronize());
-    *violations = (int64_t)(fl_oob_matched(reset) + fl_oob_batch(reset));
+    *violations = (int64_t)(fl_oob_matched(reset) + fl_oob_batch(reset) +
+                            fl_oob_refl(reset));
     return fl_set_error(FL_OK, "");
 #else
     *violations = 0;

@@ -3,6 +3,8 @@
 // (batch.cu): the incremental ray walk, the per-ray weight c_r, and the
 // detector-column window of an xy box used by the gathers.
 #pragma once
+#include <type_traits>
+
 #include "fl_common.cuh"
 #include "fl_plan.h"
 
@@ -567,10 +569,11 @@ __device__ __forceinline__ void walk_refl(const TX* __restrict__ x, const ColEnt
 // (nv: the exact angle pi/4; nv + 1: the exact angle pi/2). The backprojection
 // input has two planes of nv nb na / 2 values (the turn images, the reflected
 // images), vpr = 2 NR values per walked ray and plane (NR images x two rows).
-// Per plane: with an end view, slots s < ov of nb/2 rows x na columns, slot 0
+// Per plane: with an end view, slots s < ov of na columns x nb/2 rows (rows
+// fastest: the backprojection's lanes read the rows of neighbouring voxels), slot 0
 // holding view 0 at columns < na/2 and view ov at columns >= na/2, slot s
 // view s; without one, slot s < ov holds view s + 1 and a half slot at the end
-// (rows of na/2 columns) view 0.
+// (na/2 columns) view 0.
 struct ReflGeom {
     int nv, na, nbh, ov, end, endrow, vpr, slots;   // slots: forward grid (whole and half)
     long long slot, plane;                          // values per slot / per plane
@@ -603,6 +606,7 @@ __host__ __device__ inline ReflGeom refl_geom(int NR, int nv, int na, int nb)
 // images'), in slots of na columns laid out as the cone's (refl_slot /
 // refl_view with one row): nv * na values in all.
 struct FanReflGeom {
+    static constexpr int nbh = 1;                   // one row
     int nv, na, ov, end, endrow, vpr, slots;
     long long slot;                                 // values per slot
 };
@@ -622,15 +626,15 @@ __host__ __device__ inline FanReflGeom fan_refl_geom(int NR, int nv, int na)
 }
 
 // Forward slot (s, column ia) of a reflection form: the walked view v, its
-// table row vt and column a, and where its values go in each plane (offset
-// off + vpr (ib stride + ia) + 2 k for row ib, image k mod NR). False for the
-// unused half of the last slot. (Geo: ReflGeom, or FanReflGeom with one row.)
+// table row vt and column a, and the offset of the slot in each plane (the
+// values of row ib, image k mod NR at off + vpr (ia nb/2 + ib) + 2 k). False
+// for the unused half of the last slot. (Geo: ReflGeom, or FanReflGeom.)
 template <typename Geo>
 __device__ __forceinline__ bool refl_slot(const Geo& g, int s, int ia, int& v, int& vt,
-                                          int& a, long long& off, int& stride)
+                                          int& a, long long& off)
 {
     const int h = g.na / 2;
-    a = ia; stride = g.na;
+    a = ia;
     if (g.end) {
         off = s * g.slot;
         v = vt = s;
@@ -639,7 +643,7 @@ __device__ __forceinline__ bool refl_slot(const Geo& g, int s, int ia, int& v, i
     }
     if (s == g.ov) {
         if (ia >= h) return false;
-        v = vt = 0; off = g.ov * g.slot; stride = h;
+        v = vt = 0; off = g.ov * g.slot;
         return true;
     }
     v = vt = s + 1; off = s * g.slot;
@@ -660,21 +664,21 @@ __device__ __forceinline__ void refl_image(int k, int v, int a, int na, int nv, 
 }
 
 // Backprojection view w of a reflection form: table row, the plane offset of
-// its values (column ia, row ib at base + vpr (ib stride + ia)), and the
-// number of its walked columns.
+// its values (column ia, row ib at base + vpr (ia nb/2 + ib)), and the number
+// of its walked columns.
 template <typename Geo>
 __device__ __forceinline__ void refl_view(const Geo& g, int w, int& vt, long long& base,
-                                          int& stride, int& alim)
+                                          int& alim)
 {
     const int h = g.na / 2;
-    stride = g.na; alim = g.na; vt = w;
+    alim = g.na; vt = w;
     if (g.end) {
         base = w * g.slot;
         if (w == 0) alim = h;
-        else if (w == g.ov) { vt = g.endrow; base = (long long)g.vpr * h; alim = h; }
+        else if (w == g.ov) { vt = g.endrow; base = (long long)g.vpr * h * g.nbh; alim = h; }
         return;
     }
-    if (w == 0) { base = g.ov * g.slot; stride = h; alim = h; }
+    if (w == 0) { base = g.ov * g.slot; alim = h; }
     else base = (w - 1) * g.slot;
 }
 // The fan walk in batches of kFanBatch steps: the crossings of a batch are
@@ -848,6 +852,86 @@ __device__ __forceinline__ void walk_fan_parts(const TX* __restrict__ x,
     for (int j = 0; j < NI; j++) acc[j] = sacc[j];
 }
 
+// The backprojection input (pre-weighted sinogram) is FP32, or FP16 in the
+// mixed CGLS form. ld_in<TW, N> reads N consecutive values of one orbit from
+// an address aligned to N elements, as one vector load, and widens them.
+template <typename TW, int N>
+__device__ __forceinline__ void ld_in(const TW* __restrict__ p, float (&v)[N]);
+
+template <>
+__device__ __forceinline__ void ld_in<float, 1>(const float* __restrict__ p, float (&v)[1])
+{
+    v[0] = __ldg(p);
+}
+template <>
+__device__ __forceinline__ void ld_in<float, 2>(const float* __restrict__ p, float (&v)[2])
+{
+    const float2 u = __ldg(reinterpret_cast<const float2*>(p));
+    v[0] = u.x; v[1] = u.y;
+}
+template <>
+__device__ __forceinline__ void ld_in<float, 4>(const float* __restrict__ p, float (&v)[4])
+{
+    const float4 u = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+}
+template <>
+__device__ __forceinline__ void ld_in<float, 8>(const float* __restrict__ p, float (&v)[8])
+{
+    // one 32-byte load (sm_100 and later; orbits are 32-byte aligned)
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+          "=f"(v[7])
+        : "l"(p));
+}
+template <>
+__device__ __forceinline__ void ld_in<__half, 1>(const __half* __restrict__ p, float (&v)[1])
+{
+    v[0] = __half2float(__ldg(p));
+}
+template <>
+__device__ __forceinline__ void ld_in<__half, 2>(const __half* __restrict__ p, float (&v)[2])
+{
+    const float2 a = __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
+    v[0] = a.x; v[1] = a.y;
+}
+template <>
+__device__ __forceinline__ void ld_in<__half, 4>(const __half* __restrict__ p, float (&v)[4])
+{
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+template <>
+__device__ __forceinline__ void ld_in<__half, 8>(const __half* __restrict__ p, float (&v)[8])
+{
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+        v[2 * k] = a.x; v[2 * k + 1] = a.y;
+    }
+}
+
+// st_out<T, N>: N consecutive values as one vector store (the address aligned
+// to N elements).
+template <typename T, int N>
+__device__ __forceinline__ void st_out(T* __restrict__ p, const float (&v)[N])
+{
+    if constexpr (std::is_same<T, float>::value && N == 8) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
+                        "f"(v[6]), "f"(v[7]) : "memory");
+    } else {
+        struct alignas(N * sizeof(T)) Vec { T e[N]; } o;
+#pragma unroll
+        for (int k = 0; k < N; k++) Store<T>::st(&o.e[k], v[k]);
+        *reinterpret_cast<Vec*>(p) = o;
+    }
+}
+
 // The xy part of a cone ray's crossings with the voxel column (cx, cy): the
 // frame of the column's segment (anchor bh + be) and the column's entry l and
 // exit h in it, the crossings the forward walk computes for the column's
@@ -888,6 +972,16 @@ struct DetGrid {
     float u0, du, g0, dg, v0, dv, SO, SD;
     float rdu, rdg;    // 1/du, 1/dg (column windows only: they carry 0.02 columns of slack)
 };
+
+inline DetGrid det_grid(const fl_plan* p)
+{
+    DetGrid G;
+    G.kind = p->det_kind; G.u0 = p->u0; G.du = p->du; G.g0 = p->g0; G.dg = p->dg;
+    G.v0 = p->v0; G.dv = p->dv; G.SO = p->s.SO; G.SD = p->SD;
+    G.rdu = p->du != 0.0f ? 1.0f / p->du : 0.0f;
+    G.rdg = p->dg != 0.0f ? 1.0f / p->dg : 0.0f;
+    return G;
+}
 
 // Column range [lo, hi] of rays that can cross the xy square [x0,x0+1]x[y0,y0+1]
 // in a view with cos/sin (c, s); also returns the depth range SO + t.
@@ -1325,10 +1419,10 @@ __device__ __forceinline__ void fan_refl_forward_block(const TX* __restrict__ X,
     const FanReflGeom g = fan_refl_geom(NR, nv, na);
     const int tx = threadIdx.x % nry, lane = threadIdx.x / nry;
     const long long r = r0 + tx;
-    int v = 0, vt = 0, a = 0, stride = 0;
+    int v = 0, vt = 0, a = 0;
     long long off = 0;
     const int sl = (int)(r / na), ia = (int)(r - (long long)sl * na);
-    const bool ray = r < (long long)g.slots * na && refl_slot(g, sl, ia, v, vt, a, off, stride);
+    const bool ray = r < (long long)g.slots * na && refl_slot(g, sl, ia, v, vt, a, off);
     float acc[NI];
 #pragma unroll
     for (int j = 0; j < NI; j++) acc[j] = 0.0f;
@@ -1469,9 +1563,9 @@ __device__ __forceinline__ void fan_refl_gather(float (&P)[NR][PB][PB], float (&
             }
     };
     for (int w = g; w <= geo.ov; w += NG) {
-        int vt, rs, alim;
+        int vt, alim;
         long long base;
-        refl_view(geo, w, vt, base, rs, alim);
+        refl_view(geo, w, vt, base, alim);
         const ViewEntry ve = view[vt];
         const ColEntry* cv = col + (long long)vt * na;
         const float* yv = ywp + base;

@@ -235,8 +235,8 @@ int fl_plan_query(const fl_plan *plan, int option, int *value);
  * candidate on the plan's own geometry, one launch each on `stream` after one
  * untimed, and keeps the fastest for the forward and for the backprojection.
  * Cone plans: the 128-thread block shapes (8x16, 16x8, 32x4, 4x32) of both
- * kernels and, on reflection plans, the backprojection's voxel run and row
- * loop (FL_TUNE_ADJ_RUN / _ROWS). Fan plans: the parts per walked ray of the
+ * kernels (on reflection plans the backprojection's FL_TUNE_ADJ_RUN and
+ * FL_TUNE_ADJ_CHUNKS instead). Fan plans: the parts per walked ray of the
  * turn and reflection forwards (FL_TUNE_FAN_PARTS: 1, 4, 16), the pixel block
  * of the backprojections (FL_TUNE_FAN_BLOCK: 1 or 2) and the view groups of
  * the turn and reflection backprojections (FL_TUNE_FAN_GROUPS: 8 or 16). Only
@@ -246,12 +246,12 @@ int fl_plan_query(const fl_plan *plan, int option, int *value);
  * backprojection x, y of a cone plan; for a fan plan the parts count, 0, the
  * pixel block and the view groups. */
 int fl_plan_autotune(fl_plan *plan, void *stream, int32_t *shapes);
-/* FL_TUNE_ADJ_RUN: voxels per thread of the reflection backprojection (1 or
- * 2); FL_TUNE_ADJ_ROWS: its row loop, 1 or 2 detector rows per iteration, or
- * 3: one pass over a run's rows, each row loaded once for all the run's
- * voxels (runs of 2; with runs of 1 it is 1). fl_plan_autotune times the
- * pairs and keeps the fastest; fl_plan_option sets them (other values are
- * refused), fl_plan_query reads them. The results do not depend on them. */
+/* FL_TUNE_ADJ_RUN: columns per side of the block of voxel columns a warp of the
+ * reflection backprojection owns (1 or 2; by default 2 once such warps fill the
+ * GPU). fl_plan_autotune times both and keeps the faster; fl_plan_option sets it
+ * (other values are refused), fl_plan_query reads the value in effect. The
+ * results do not depend on it. FL_TUNE_ADJ_ROWS (1 .. 3) is accepted and read
+ * back, and selects nothing: the kernel's row loop has one form. */
 enum { FL_TUNE_ADJ_RUN = 16, FL_TUNE_ADJ_ROWS = 17 };
 /* Fan plans. FL_TUNE_FAN_PARTS: threads per walked ray of the half- or
  * quarter-turn forward (1, 4 or 16), each walking a run of the ray's segments,
@@ -275,10 +275,10 @@ enum { FL_TUNE_FAN_PARTS = 18, FL_TUNE_FAN_BLOCK = 19 };
  * fl_plan_autotune times both on turn and reflection plans. */
 enum { FL_TUNE_FAN_GROUPS = 20 };
 /* FL_TUNE_ADJ_CHUNKS: the reflection backprojection of a cone plan runs as
- * this many launches over consecutive chunks of its walked views (1 .. 64;
- * default 1), each continuing the sums the one before left in the output, so
+ * this many launches over consecutive chunks of its walked views (1 .. 64; by
+ * default one per half gigabyte of packed input, at most 16), each continuing the sums the one before left in the output, so
  * the blocks resident together read the same views' detector rows and L2
- * serves them (512^3, 720 views: 16 chunks, 264 -> 256 ms per CGLS iteration).
+ * serves them (512^3, 720 views: 4 chunks, 188 -> 185 ms per CGLS iteration).
  * The sums are added in the same order: the results do not depend on it. It
  * applies where the backprojection writes FP32 (FP16 / BF16 outputs take one
  * launch). fl_plan_autotune times 1, 4, 8, 16. */
