@@ -209,8 +209,9 @@ inline int fl_plan_refl(const fl_plan* p)
 // Layouts of the matched launchers' operands. For a z-mirror plan the
 // z-folded volume stores, per frame, the pairs (voxel (ix, iy, iz),
 // voxel (ix, iy, nz-1-iz)) for iz < nz/2 at pair index (iz*ny + iy)*nx + ix;
-// the adjoint input (pre-weighted sinogram) is always folded the same way:
-// pairs (row ib, row nb-1-ib) for ib < nb/2 at pair index (iv*nb/2 + ib)*na + ia,
+// the adjoint input (pre-weighted sinogram) has its rows fastest: row ib at
+// (iv*na + ia)*nb + ib, or with the z mirror the pairs (row ib, row nb-1-ib) for
+// ib < nb/2 at pair index (iv*na + ia)*nb/2 + ib,
 // except on a half- (G = 2) or quarter-turn (G = 4) plan, where the 2 G values
 // of views iv + j nv/G (j < G), rows ib and nb-1-ib, lie side by side at
 // 2 G ((iv*nb/2 + ib)*na + ia) + 2 j for iv < nv/G. A reflection form packs
@@ -283,6 +284,9 @@ int fl_matched_adjoint_wt(fl_plan* p, const void* yw, int wt, void* x, int xt, c
                           int layout, cudaStream_t st);
 // the reflection forms' kernels of it (refl_adjoint.cu)
 void fl_matched_adjoint_refl(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
+                             int xfold, cudaStream_t st);
+// the general and z-mirror forms' kernels (cone_adjoint.cu)
+void fl_matched_adjoint_cone(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
                              int xfold, cudaStream_t st);
 // volume (all frames) to the z-folded layout, or back with unfold = 1
 int fl_matched_fold(fl_plan* p, const void* src, void* dst, int dtype, int unfold,

@@ -34,9 +34,11 @@ namespace {
 // MIRROR (scans symmetric about the source plane, fl_plan::zmirror): X is
 // z-folded; the block walks only the rows ib < nb/2 and also produces each
 // ray's mirrored companion, row nb-1-ib, from the same walk. yfold selects
-// the folded sinogram layout (pairs of rows ib and nb-1-ib) for the output.
+// the backprojection's input layout for the output (k_weight_cone's).
+// 7 blocks per SM with the mirror: 152 x 152 x 98, 211 views 1.33 -> 0.99 ms
+// against 8 (72 registers); without it 8 and 7 are alike.
 template <typename TX, typename TY, bool MIRROR>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, MIRROR ? 7 : 8)
 k_fwd_cone(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
            const float* __restrict__ colr, const RowEntry* __restrict__ row,
            const int* __restrict__ vframe, int nx, int ny, int nz, int na, int nb,
@@ -65,13 +67,14 @@ k_fwd_cone(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
         float om = cr * accm;
         if (cr_power == 2) om = cr * om;
         if (yfold) {
-            Store<TY>::st2(y + 2 * (((long long)iv * (nb / 2) + ib) * na + ia), out, om);
+            Store<TY>::st2(y + 2 * (((long long)iv * na + ia) * (nb / 2) + ib), out, om);
         } else {
             Store<TY>::st(y + ((long long)iv * nb + ib) * na + ia, out);
             Store<TY>::st(y + ((long long)iv * nb + (nb - 1 - ib)) * na + ia, om);
         }
     } else {
-        Store<TY>::st(y + ((long long)iv * nb + ib) * na + ia, out);
+        const unsigned q = yfold ? (unsigned)ia * nb + ib : (unsigned)ib * na + ia;
+        Store<TY>::st(y + (long long)iv * na * nb + q, out);
     }
 }
 
@@ -334,28 +337,37 @@ k_count(int32_t* __restrict__ cnt, const ColEntry* __restrict__ col,
     cnt[r] = c;
 }
 
-// Folded yw for a z-mirror plan: the pair (c_r y[ib], c_r y[nb-1-ib]) of rows
-// ib < nb/2, both with the walked row's c_r (equal to the mirror's: its d_z is
-// the exact negation).
-// pv: view iv takes c_r of view iv % pv, the ray it is defined by (pv = nv:
-// turn plans pack their input with k_weight_packed instead).
-template <typename TY>
-__global__ void k_weight_fold(float* __restrict__ yw, const TY* __restrict__ y,
-                              const float* __restrict__ colr, const RowEntry* __restrict__ row,
-                              int na, int nb, long long npairs, float scale, int pv)
+// yw of the general and (MIRROR) z-mirror forms of a cone plan, rows fastest:
+// c_r y of row ib at (iv na + ia) nb + ib; with the mirror the pair (c_r y[ib],
+// c_r y[nb-1-ib]) of rows ib < nb/2 at 2 ((iv na + ia) nb/2 + ib), both with the
+// walked row's c_r (equal to the mirror's: its d_z is the exact negation). 32 x
+// 32 tiles through shared memory: reads run along columns, writes along rows.
+template <typename TY, bool MIRROR>
+__global__ void __launch_bounds__(256)
+k_weight_cone(float* __restrict__ yw, const TY* __restrict__ y, const float* __restrict__ colr,
+              const RowEntry* __restrict__ row, int na, int nb, float scale)
 {
-    long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= npairs) return;
-    const int nbh = nb / 2;
-    int ia = (int)(r % na);
-    long long q = r / na;
-    int ib = (int)(q % nbh);
-    int iv = (int)(q / nbh);
-    const int ivc = iv % pv;
-    float cr = ray_cr(scale, colr[(long long)ivc * na + ia], row[(long long)ivc * nb + ib].dz2);
-    float a = Store<TY>::ld_plain(y + ((long long)iv * nb + ib) * na + ia);
-    float b = Store<TY>::ld_plain(y + ((long long)iv * nb + (nb - 1 - ib)) * na + ia);
-    Store<float>::st2(yw + 2 * r, cr * a, cr * b);
+    constexpr int V = MIRROR ? 2 : 1;
+    __shared__ float tile[V][32][33];
+    const int nbw = MIRROR ? nb / 2 : nb, iv = blockIdx.z;
+    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int ia = a0 + threadIdx.x, ib = b0 + k;
+        if (ia >= na || ib >= nbw) continue;
+        const float cr = ray_cr(scale, colr[(long long)iv * na + ia], row[(long long)iv * nb + ib].dz2);
+        tile[0][k][threadIdx.x] = cr * Store<TY>::ld_plain(y + ((long long)iv * nb + ib) * na + ia);
+        if (MIRROR)
+            tile[V - 1][k][threadIdx.x] =
+                cr * Store<TY>::ld_plain(y + ((long long)iv * nb + (nb - 1 - ib)) * na + ia);
+    }
+    __syncthreads();
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int ia = a0 + k, ib = b0 + threadIdx.x;
+        if (ia >= na || ib >= nbw) continue;
+        float* o = yw + V * (((long long)iv * na + ia) * nbw + ib);
+        if (MIRROR) Store<float>::st2(o, tile[0][threadIdx.x][k], tile[V - 1][threadIdx.x][k]);
+        else *o = tile[0][threadIdx.x][k];
+    }
 }
 
 // Packed yw of a half- (G = 2) or quarter-turn (G = 4) plan: for
@@ -540,23 +552,15 @@ __global__ void k_fold_tiled(const T* __restrict__ src, T* __restrict__ dst, int
     }
 }
 
-// yw = c_r * y  (the adjoint gathers pre-weighted sinogram values)
+// yw = c_r * y of a fan plan (the adjoint gathers pre-weighted sinogram values)
 template <typename TY>
 __global__ void k_weight(float* __restrict__ yw, const TY* __restrict__ y,
-                         const float* __restrict__ colr, const RowEntry* __restrict__ row,
-                         int na, int nb, long long nrays, float scale, int three)
+                         const float* __restrict__ colr, long long nrays, float scale)
 {
     long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nrays) return;
-    int ia = (int)(r % na);
-    long long q = r / na;
-    int ib = (int)(q % nb);
-    int iv = (int)(q / nb);
-    float dz2 = three ? row[(long long)iv * nb + ib].dz2 : 0.0f;
-    float cr = ray_cr(scale, colr[(long long)iv * na + ia], dz2);
-    yw[r] = cr * Store<TY>::ld_plain(y + r);
+    yw[r] = ray_cr(scale, colr[r], 0.0f) * Store<TY>::ld_plain(y + r);
 }
-
 
 // ---------------------------------------------------------------------------
 // Fan adjoint: one thread per (pixel, frame).
@@ -617,105 +621,21 @@ k_adj_fan_turn(TX* __restrict__ X, const float* __restrict__ ywp,
 }
 
 // ---------------------------------------------------------------------------
-// Cone adjoint: one thread per voxel column (ix, iy) and a run of TZ voxels in
-// z (block 32 x 4 columns). Per view, the thread finds the detector columns
-// whose rays can cross its column (projection of the column's four corners),
-// and per such column the xy crossing interval [l, h] of the ray family. For
-// each voxel k of the run it then visits only the detector rows whose ray is
-// inside that voxel's z range somewhere in [l, h], and adds w_rV * (c_r y_r)
-// with w_rV evaluated exactly as in the forward walk. The TZ accumulators are
-// registers (k is a compile-time index).
+// Half- and quarter-turn backprojections (the general, z-mirror and reflection
+// forms: cone_adjoint.cu, refl_adjoint.cu). One thread per voxel column and a
+// run of TZ voxels in z. Per view, the thread finds the detector columns whose
+// rays can cross its column (projection of the column's four corners), and per
+// such column the xy crossing interval [l, h] of the ray family. For each voxel
+// k of the run it then visits only the detector rows whose ray is inside that
+// voxel's z range somewhere in [l, h], and adds w_rV * (c_r y_r) with w_rV
+// evaluated exactly as in the forward walk. The walked rays lie below the
+// source plane. MODE -1 (every run except the one at the source plane): the
+// rays descend and the row grid rises (dv > 0 for any z-mirror plan), so e1 <=
+// e2 at every plane and both grow with k; voxel k's rows are then [e1(k), e2(k +
+// 1)] without per-plane min / max. MODE 0: the general window.
 // ---------------------------------------------------------------------------
-// Candidate rays of one detector column for the TZ voxels of a run. MODE +1:
-// the run lies above the source plane, so every ray that reaches it rises
-// (A_z increasing in k); MODE -1: below, every such ray falls; MODE 0: the run
-// straddles the source plane (general min/max). The other orientation's rays
-// get w <= 0 from the specialised formula, as they miss the run.
-template <int MODE, int TZ, typename TW>
-__device__ __forceinline__ void adj_rows(float (&acc)[TZ], int nk, int z0, float l, float h,
-                                         float e1, float e2, float s1, float s2,
-                                         const AxisEntry* __restrict__ rv, float bh, float be,
-                                         const TW* __restrict__ ycol, int na, int nb)
-{
-    float mn = fminf(e1, e2), mx = fmaxf(e1, e2);   // row span at plane k
-#pragma unroll
-    for (int k = 0; k < TZ; k++) {
-        if (k >= nk) break;
-        e1 += s1; e2 += s2;
-        const float mn1 = fminf(e1, e2), mx1 = fmaxf(e1, e2);   // plane k + 1
-        const int blo = max(__float2int_ru(fminf(mn, mn1) - 0.02f), 0);
-        const int bhi = min(__float2int_rd(fmaxf(mx, mx1) + 0.02f), nb - 1);
-        mn = mn1; mx = mx1;
-        const float fk0 = (float)(z0 + k), fk1 = (float)(z0 + k + 1);
-        for (int ib = blo; ib <= bhi; ib++) {
-            if (!FL_IN(ib, nb)) continue;
-            const AxisEntry re = rv[ib];                 // (inv_z, off_z) of row ib
-            float yv1[1];
-            ld_in<TW, 1>(ycol + (long long)ib * na, yv1);
-            const float yval = yv1[0];
-            const float2 azp = row_planes(re, fk0, fk1, bh, be);
-            const float az0 = azp.x, az1 = azp.y;
-            float l2, h2;
-            if (MODE > 0)      { l2 = fmaxf(l, az0); h2 = fminf(h, az1); }
-            else if (MODE < 0) { l2 = fmaxf(l, az1); h2 = fminf(h, az0); }
-            else { l2 = fmaxf(l, fminf(az0, az1)); h2 = fminf(h, fmaxf(az0, az1)); }
-            // w <= 0 (the ray misses voxel k) adds exactly 0 for finite y
-            acc[k] = fmaf(fmaxf(h2 - l2, 0.0f), yval, acc[k]);
-        }
-    }
-}
-
-// z-mirror form: rows limited to the walked half (nb here is nb/2); ycol
-// points into the folded sinogram (pairs of rows ib and nb-1-ib, row stride
-// 2*na); acc[k] holds the voxel k and its mirror, both updated by one paired
-// FMA (per lane the same rounding as fmaf). MODE -1 (every lower run except
-// the one at the source plane): the rays descend and the row grid rises
-// (dv > 0 for any z-mirror plan), so e1 <= e2 at every plane and both grow
-// with k; voxel k's rows are then [e1(k), e2(k + 1)] without per-plane
-// min / max. MODE 0: the general window. (MODE +1 does not occur: every run
-// of the lower half lies below the source.)
-template <int MODE, int TZ, typename TW>
-__device__ __forceinline__ void adj_rows_pair(float2 (&acc)[TZ], int nk, int z0, float l,
-                                              float h, float e1, float e2, float s1, float s2,
-                                              const AxisEntry* __restrict__ rv, float bh, float be,
-                                              const TW* __restrict__ ycol, int na, int nb)
-{
-    float mn = fminf(e1, e2), mx = fmaxf(e1, e2);
-    float lo_e = e1 - 0.02f, hi_e = e2 + s2 + 0.02f;
-#pragma unroll
-    for (int k = 0; k < TZ; k++) {
-        if (k >= nk) break;
-        int blo, bhi;
-        if (MODE < 0) {
-            blo = max(__float2int_ru(lo_e), 0);
-            bhi = min(__float2int_rd(hi_e), nb - 1);
-            lo_e += s1; hi_e += s2;
-        } else {
-            e1 += s1; e2 += s2;
-            const float mn1 = fminf(e1, e2), mx1 = fmaxf(e1, e2);
-            blo = max(__float2int_ru(fminf(mn, mn1) - 0.02f), 0);
-            bhi = min(__float2int_rd(fmaxf(mx, mx1) + 0.02f), nb - 1);
-            mn = mn1; mx = mx1;
-        }
-        const float fk0 = (float)(z0 + k), fk1 = (float)(z0 + k + 1);
-        for (int ib = blo; ib <= bhi; ib++) {
-            if (!FL_IN(ib, nb)) continue;
-            const AxisEntry re = rv[ib];
-            float tv[2];
-            ld_in<TW, 2>(ycol + 2 * (long long)ib * na, tv);
-            const float2 t = make_float2(tv[0], tv[1]);
-            const float2 az = row_planes(re, fk0, fk1, bh, be);
-            float l2, h2;
-            if (MODE < 0) { l2 = fmaxf(l, az.y); h2 = fminf(h, az.x); }
-            else { l2 = fmaxf(l, fminf(az.x, az.y)); h2 = fminf(h, fmaxf(az.x, az.y)); }
-            const float w = fmaxf(h2 - l2, 0.0f);
-            acc[k] = __ffma2_rn(make_float2(w, w), t, acc[k]);
-        }
-    }
-}
-
-// Half-turn form of adj_rows_pair: every weight also multiplies the row pair
-// of view v + nv/2 into the turned voxels' sums accr; y4 holds both row pairs
+// Half turn: every weight multiplies the row pair of view v into the voxels'
+// sums acc and the row pair of view v + nv/2 into the turned voxels' sums accr; y4 holds both row pairs
 // side by side (4 floats per row and column, 16-byte aligned).
 template <int MODE, int TZ, typename TW>
 __device__ __forceinline__ void adj_rows_quad(float2 (&acc)[TZ], float2 (&accr)[TZ], int nk,
@@ -852,7 +772,7 @@ k_adj_quad(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
         }
 }
 
-// Quarter-turn form of adj_rows_pair: every weight multiplies the row pairs of
+// Quarter turns: every weight multiplies the row pairs of
 // views v + j nv/4 into the sums a0..a3; y8 holds them side by side (8 floats
 // per row and column, 32-byte aligned).
 template <int MODE, int TZ, typename TW>
@@ -1001,95 +921,6 @@ k_adj_oct(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __restr
         }
 }
 
-// MIRROR: yw is the folded sinogram; the runs cover the lower half z < nz/2
-// only (the walked rows' rays never reach the upper half) and each thread also
-// produces the mirrored run, into the folded volume when xfold is set.
-template <typename TX, int TZ, bool MIRROR, typename TW>
-__global__ void __launch_bounds__(128, 8)
-k_adj_cone(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __restrict__ col,
-           const AxisEntry* __restrict__ rowz, const ViewEntry* __restrict__ view,
-           const int* __restrict__ idY, const int* __restrict__ Nv, int tmp_size, DetGrid G,
-           int nx, int ny, int nz, int na, int nb, float dz, int zruns,
-           const int* __restrict__ skip, int xfold)
-{
-    if (skip && *skip) return;
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    const int zr = blockIdx.z % zruns, it = blockIdx.z / zruns;
-    const int z0 = zr * TZ;
-    const int nzw = MIRROR ? nz / 2 : nz;      // voxels gathered directly
-    const int nbw = MIRROR ? nb / 2 : nb;      // rows evaluated
-    const int nk = min(TZ, nzw - z0);          // voxels of this run inside that range
-    if (ix >= nx || iy >= ny) return;
-    float acc[TZ];                 // general form
-    float2 acc2[TZ];               // mirror form: (voxel, mirrored voxel)
-#pragma unroll
-    for (int k = 0; k < TZ; k++) { acc[k] = 0.0f; acc2[k] = make_float2(0.0f, 0.0f); }
-    const float x0 = (float)(ix - nx / 2), y0 = (float)(iy - ny / 2);
-    const float inv_dv = 1.0f / G.dv;
-    const int nvf = Nv[it];
-    for (int j = 0; j < nvf; j++) {
-        const int iv = idY[it * tmp_size + j];
-        const ViewEntry ve = view[iv];
-        int alo, ahi; float dmin, dmax;
-        column_window(G, ve.c, ve.s, x0, y0, 1.0f, 1.0f, na, alo, ahi, dmin, dmax);
-        const ColEntry* cv = col + (long long)iv * na;
-        const AxisEntry* rv = rowz + (long long)iv * nb;
-        const TW* yv = yw + (long long)iv * nb * na;      // folded: nb/2 rows of pairs
-        // run planes relative to the source: lowest and highest
-        const float zr0 = (float)(z0 - nz / 2) * dz - ve.sz;
-        const float zr1 = (float)(z0 + nk - nz / 2) * dz - ve.sz;
-        // uniform per block; a run within rounding distance of the source plane
-        // takes the general path
-        const float tol = 1e-3f * dz;
-        const int mode = (zr0 >= tol) ? 1 : ((zr1 <= -tol) ? -1 : 0);
-        for (int ia = alo; ia <= ahi; ia++) {
-            if (!FL_IN(ia, na)) continue;
-            const ColEntry ce = cv[ia];
-            float bh, be, l, h;
-            if (!cone_column(ce, ix, iy, nx, ny, bh, be, l, h)) continue;
-            // A ray of row ib is at z = sz + (A + ac) * d_ib, d_ib ~ v0 + ib * dv. It is
-            // inside voxel k somewhere in [l, h] iff d_ib lies between the plane
-            // heights over (A + ac) at the two ends: in detector-row units the
-            // rows [e(k), e(k+1)], stepping by dz/(A + ac)/dv per plane.
-            const float r1 = __fdividef(1.0f, __fadd_rn(bh, l) + ve.ac);
-            const float r2 = __fdividef(1.0f, __fadd_rn(bh, h) + ve.ac);
-            const float s1 = dz * r1 * inv_dv, s2 = dz * r2 * inv_dv;
-            const float e1 = (zr0 * r1 - G.v0) * inv_dv, e2 = (zr0 * r2 - G.v0) * inv_dv;
-            if (MIRROR) {
-                const TW* ycol = yv + 2 * ia;
-                if (mode < 0)
-                    adj_rows_pair<-1, TZ, TW>(acc2, nk, z0, l, h, e1, e2, s1, s2, rv, bh, be, ycol, na, nbw);
-                else
-                    adj_rows_pair<0, TZ, TW>(acc2, nk, z0, l, h, e1, e2, s1, s2, rv, bh, be, ycol, na, nbw);
-            } else {
-                const TW* ycol = yv + ia;
-                if (mode > 0)
-                    adj_rows<1, TZ, TW>(acc, nk, z0, l, h, e1, e2, s1, s2, rv, bh, be, ycol, na, nbw);
-                else if (mode < 0)
-                    adj_rows<-1, TZ, TW>(acc, nk, z0, l, h, e1, e2, s1, s2, rv, bh, be, ycol, na, nbw);
-                else
-                    adj_rows<0, TZ, TW>(acc, nk, z0, l, h, e1, e2, s1, s2, rv, bh, be, ycol, na, nbw);
-            }
-        }
-    }
-    const long long frame = (long long)it * nx * ny * nz, col_ = (long long)iy * nx + ix;
-#pragma unroll
-    for (int k = 0; k < TZ; k++)
-        if (k < nk) {
-            if (MIRROR && xfold) {
-                Store<TX>::st2(X + frame + 2 * ((long long)(z0 + k) * nx * ny + col_),
-                               acc2[k].x, acc2[k].y);
-            } else if (MIRROR) {
-                Store<TX>::st(X + frame + (long long)(z0 + k) * nx * ny + col_, acc2[k].x);
-                Store<TX>::st(X + frame + (long long)(nz - 1 - z0 - k) * nx * ny + col_,
-                              acc2[k].y);
-            } else {
-                Store<TX>::st(X + frame + (long long)(z0 + k) * nx * ny + col_, acc[k]);
-            }
-        }
-}
-
 }  // namespace
 
 // Tunables of fan plans (fl_plan.h).
@@ -1200,7 +1031,7 @@ void launch_fwd(fl_plan* p, const void* x, void* y, int cr_power, const int* ski
         dim3 grid(fl_div_up(s.na, fb.x), s.nv, fl_div_up(s.nb, fb.y));
         k_fwd_cone<TX, TY, false><<<grid, fb, 0, st>>>(
             (const TX*)x, (TY*)y, p->d_col, p->d_colr, p->d_row, p->d_view_frame, s.nx, s.ny,
-            s.nz, s.na, s.nb, p->n_vox_frame, s.scale, cr_power, skip, xscale, 0);
+            s.nz, s.na, s.nb, p->n_vox_frame, s.scale, cr_power, skip, xscale, yfold);
     } else if (fl_plan_refl(p)) {
         const TX* xt = fan_transposed<TX>(p, x, st);
         const int NR = fl_plan_refl(p);
@@ -1254,9 +1085,8 @@ void launch_adj_cone(fl_plan* p, const TW* yw, void* x, const int* skip, int xfo
     const fl_scan& s = p->s;
     DetGrid G = det_grid(p);
     {
-        constexpr int TZ = 8;
-        const int nzw = p->zmirror ? s.nz / 2 : s.nz;
-        int zruns = (nzw + TZ - 1) / TZ;
+        const int nzw = s.nz / 2;
+        int zruns;
         if (fl_plan_refl(p)) {
             fl_matched_adjoint_refl(p, yw, dtype_of<TW>(), x, dtype_of<TX>(), skip, xfold, st);
         } else if (p->zmirror && p->rot && p->rot4) {
@@ -1277,18 +1107,8 @@ void launch_adj_cone(fl_plan* p, const TW* yw, void* x, const int* skip, int xfo
             k_adj_quad<TX, TQ, TW><<<grid, ab, 0, st>>>(
                 (TX*)x, yw, p->d_col, p->d_rowz, p->d_view, G, s.nx, s.ny, s.nz, s.na, s.nb, s.nv,
                 s.dz, zruns, skip, xfold);
-        } else if (p->zmirror) {
-            const dim3 ab = p->adj_bx ? dim3(p->adj_bx, p->adj_by) : dim3(16, 8);
-            dim3 grid(fl_div_up(s.nx, ab.x), fl_div_up(s.ny, ab.y), (unsigned)zruns * s.nt);
-            k_adj_cone<TX, TZ, true, TW><<<grid, ab, 0, st>>>(
-                (TX*)x, yw, p->d_col, p->d_rowz, p->d_view, p->d_idY, p->d_Nv, p->tmp_size, G,
-                s.nx, s.ny, s.nz, s.na, s.nb, s.dz, zruns, skip, xfold);
         } else {
-            const dim3 ab = p->adj_bx ? dim3(p->adj_bx, p->adj_by) : dim3(32, 4);
-            dim3 grid(fl_div_up(s.nx, ab.x), fl_div_up(s.ny, ab.y), (unsigned)zruns * s.nt);
-            k_adj_cone<TX, TZ, false, TW><<<grid, ab, 0, st>>>(
-                (TX*)x, yw, p->d_col, p->d_rowz, p->d_view, p->d_idY, p->d_Nv, p->tmp_size, G,
-                s.nx, s.ny, s.nz, s.na, s.nb, s.dz, zruns, skip, 0);
+            fl_matched_adjoint_cone(p, yw, dtype_of<TW>(), x, dtype_of<TX>(), skip, xfold, st);
         }
     }
 }
@@ -1477,10 +1297,9 @@ int fl_matched_forward(fl_plan* p, const void* x, int xt, void* y, int yt, int c
             if ((e = fl_matched_fold(p, x, w, xt, 0, st))) return e;
             x = w;
         }
-        yfold = (layout & FL_LAY_Y_ADJ) ? 1 : 0;
-    } else if (p->s.ndim == 2 && fl_plan_turns(p) > 1) {
-        yfold = (layout & FL_LAY_Y_ADJ) ? 1 : 0;      // the packed fan layout
     }
+    // the backprojection's input layout (fl_plan.h)
+    if (p->s.ndim == 3 || fl_plan_turns(p) > 1) yfold = (layout & FL_LAY_Y_ADJ) ? 1 : 0;
     if (xt == FL_F32) launch_fwd_y<float>(p, x, y, yt, cr_power, skip, xscale, yfold, st);
     else if (xt == FL_F16) launch_fwd_y<__half>(p, x, y, yt, cr_power, skip, xscale, yfold, st);
     else launch_fwd_y<__nv_bfloat16>(p, x, y, yt, cr_power, skip, xscale, yfold, st);
@@ -1513,32 +1332,32 @@ int fl_matched_weight(fl_plan* p, const void* y, int yt, float* yw, cudaStream_t
         else launch_weight_fan_packed<2>(p, y, yt, yw, st);
         return fl_check_launch("matched adjoint weighting");
     }
-    if (three && p->zmirror) {
-        long long np = (long long)s.nv * (s.nb / 2) * s.na;
-        unsigned g = fl_div_up(np, 256);
-        const int hv = s.nv;            // view period: every view has its own rays here
-        if (yt == FL_F32)
-            k_weight_fold<float><<<g, 256, 0, st>>>(yw, (const float*)y, p->d_colr, p->d_row,
-                                                    s.na, s.nb, np, s.scale, hv);
-        else if (yt == FL_F16)
-            k_weight_fold<__half><<<g, 256, 0, st>>>(yw, (const __half*)y, p->d_colr, p->d_row,
-                                                     s.na, s.nb, np, s.scale, hv);
-        else
-            k_weight_fold<__nv_bfloat16><<<g, 256, 0, st>>>(yw, (const __nv_bfloat16*)y,
-                                                            p->d_colr, p->d_row, s.na, s.nb, np,
-                                                            s.scale, hv);
+    if (three) {
+        const dim3 g(fl_div_up(s.na, 32), fl_div_up(p->zmirror ? s.nb / 2 : s.nb, 32), s.nv);
+        const dim3 blk(32, 8);
+#define FL_WEIGHT_CONE(TY)                                                                   \
+    do {                                                                                     \
+        if (p->zmirror)                                                                      \
+            k_weight_cone<TY, true><<<g, blk, 0, st>>>(yw, (const TY*)y, p->d_colr, p->d_row, \
+                                                       s.na, s.nb, s.scale);                 \
+        else                                                                                 \
+            k_weight_cone<TY, false><<<g, blk, 0, st>>>(yw, (const TY*)y, p->d_colr, p->d_row, \
+                                                        s.na, s.nb, s.scale);                \
+    } while (0)
+        if (yt == FL_F32) FL_WEIGHT_CONE(float);
+        else if (yt == FL_F16) FL_WEIGHT_CONE(__half);
+        else FL_WEIGHT_CONE(__nv_bfloat16);
+#undef FL_WEIGHT_CONE
         return fl_check_launch("matched adjoint weighting");
     }
     unsigned g = fl_div_up(nr, 256);
     if (yt == FL_F32)
-        k_weight<float><<<g, 256, 0, st>>>(yw, (const float*)y, p->d_colr, p->d_row, s.na,
-                                           s.nb, nr, s.scale, three);
+        k_weight<float><<<g, 256, 0, st>>>(yw, (const float*)y, p->d_colr, nr, s.scale);
     else if (yt == FL_F16)
-        k_weight<__half><<<g, 256, 0, st>>>(yw, (const __half*)y, p->d_colr, p->d_row, s.na,
-                                            s.nb, nr, s.scale, three);
+        k_weight<__half><<<g, 256, 0, st>>>(yw, (const __half*)y, p->d_colr, nr, s.scale);
     else
-        k_weight<__nv_bfloat16><<<g, 256, 0, st>>>(yw, (const __nv_bfloat16*)y, p->d_colr,
-                                                   p->d_row, s.na, s.nb, nr, s.scale, three);
+        k_weight<__nv_bfloat16><<<g, 256, 0, st>>>(yw, (const __nv_bfloat16*)y, p->d_colr, nr,
+                                                   s.scale);
     return fl_check_launch("matched adjoint weighting");
 }
 
@@ -1709,6 +1528,7 @@ int fl_matched_count(fl_plan* p, int32_t* counts, cudaStream_t st)
 FL_OOB_ACCESSOR(fl_oob_matched)
 extern "C" unsigned long long fl_oob_batch(int reset);
 extern "C" unsigned long long fl_oob_refl(int reset);
+extern "C" unsigned long long fl_oob_cone(int reset);
 
 extern "C" int fl_debug_bounds(int64_t* violations, int reset)
 {
@@ -1716,7 +1536,7 @@ extern "C" int fl_debug_bounds(int64_t* violations, int reset)
 #ifdef FL_BOUNDS_CHECK
     FL_CUDA(cudaDeviceSynchronize());
     *violations = (int64_t)(fl_oob_matched(reset) + fl_oob_batch(reset) +
-                            fl_oob_refl(reset));
+                            fl_oob_refl(reset) + fl_oob_cone(reset));
     return fl_set_error(FL_OK, "");
 #else
     *violations = 0;
