@@ -107,6 +107,8 @@ int fl_set_error(int code, const char* fmt, ...);
 // Every device allocation of the library goes through fl_malloc, so a test can
 // make the n-th one fail (fl_debug_fail_alloc) and check the error paths.
 cudaError_t fl_malloc(void** p, size_t bytes);
+// the same from a memory pool, in stream order
+cudaError_t fl_malloc_async(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
 int fl_check_cuda(cudaError_t e, const char* what);
 int fl_check_launch(const char* what);
 #define FL_CUDA(call)                                                     \

@@ -55,6 +55,8 @@ struct fl_plan {
     float *d_cos_det2, *d_sin_det2; // [na+1] bin-edge trig (finite-beam backprojector)
     float *d_fb_edges;             // [nv*na*6] finite-beam edge lines (Px, Py, Pd) x 2
     int32_t *d_view_frame, *d_idY, *d_Nv;
+    cudaMemPool_t pool;            // cone: stream-ordered scratch of single calls (kept, freed with the plan)
+    float zdet_min, zdet_max;      // smallest non-zero and largest |z_det| (cone)
     // matched-model tables (device); rows nv and nv + 1 (two extra views) hold
     // view nv/8 at the exact angle pi/4 and view nv/4 at the exact angle pi/2
     // for the reflection forms

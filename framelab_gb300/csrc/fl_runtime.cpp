@@ -47,19 +47,30 @@ static std::atomic<long long> g_fail_countdown{0};
 
 extern "C" void fl_debug_fail_alloc(int64_t nth) { g_fail_countdown.store(nth > 0 ? nth : 0); }
 
-cudaError_t fl_malloc(void** p, size_t bytes)
+// whether this allocation is the one to fail
+static bool alloc_fails(void** p)
 {
     long long c = g_fail_countdown.load();
     while (c > 0) {
         if (g_fail_countdown.compare_exchange_weak(c, c - 1)) {
             if (c == 1) {
                 *p = nullptr;
-                return cudaErrorMemoryAllocation;
+                return true;
             }
             break;
         }
     }
-    return cudaMalloc(p, bytes);
+    return false;
+}
+
+cudaError_t fl_malloc(void** p, size_t bytes)
+{
+    return alloc_fails(p) ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+}
+
+cudaError_t fl_malloc_async(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st)
+{
+    return alloc_fails(p) ? cudaErrorMemoryAllocation : cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
 extern "C" int fl_last_status(void) { return g_status; }
@@ -90,6 +101,24 @@ static void free_plan_arrays(fl_plan* p)
                     p->d_dq, p->d_tma_err};
     for (void* q : ptrs)
         if (q) cudaFree(q);
+    if (p->pool) cudaMemPoolDestroy(p->pool);
+}
+
+// A memory pool of the current device that keeps what it was given until it is
+// destroyed: concurrent calls get memory of their own, a call after another on
+// one stream the same memory again.
+static int make_pool(cudaMemPool_t* pool)
+{
+    cudaMemPoolProps pr;
+    std::memset(&pr, 0, sizeof pr);
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    int st = fl_check_cuda(cudaGetDevice(&pr.location.id), "cudaGetDevice");
+    if (!st) st = fl_check_cuda(cudaMemPoolCreate(pool, &pr), "cudaMemPoolCreate");
+    uint64_t keep = ~0ull;
+    if (!st) st = fl_check_cuda(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep),
+                                "cudaMemPoolSetAttribute");
+    return st;
 }
 
 // Nudge a direction component away from zero so 1/d stays finite; the ray
@@ -605,6 +634,15 @@ extern "C" int fl_plan_create(const fl_scan* scan, fl_plan** out)
     if (!st && !fbe.empty()) st = upload(&p->d_fb_edges, fbe.data(), fbe.size());
     if (!st) st = upload(&p->d_idY, idY.data(), idY.size());
     if (!st) st = upload(&p->d_Nv, Nvv.data(), nt);
+    if (!st && s.ndim == 3) {
+        st = make_pool(&p->pool);
+        p->zdet_min = 3.0e38f;
+        for (int ib = 0; ib < nb; ib++) {
+            const float z = std::fabs(s.z_det[ib]);
+            if (z > 0.0f) p->zdet_min = std::fmin(p->zdet_min, z);
+            p->zdet_max = std::fmax(p->zdet_max, z);
+        }
+    }
     if (!st) st = build_tables(p, phi, s.sd_z ? sdz.data() : nullptr, s.y_det, s.z_det);
     // host copies of the arrays are not kept: clear the caller's pointers
     p->s.sd_phi = p->s.sd_z = p->s.y_det = p->s.z_det = nullptr;

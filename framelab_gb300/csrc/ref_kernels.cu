@@ -317,54 +317,120 @@ __device__ float chord_box(float px, float py, float pz, float qx, float qy, flo
     return fsqrt(fadd(fadd(fmul(ex, ex), fmul(ey, ey)), fmul(ez, ez)));
 }
 
-// chord_box for a unit cube (w = h = t = 1) when the in-plane direction
-// (a, b) has no zero component, with the x- and y-face families' in-plane
-// crossings u0x, u1x (the b / a family) and u0y, u1y (the a / b family)
-// computed by the caller once per detector column. Every value is the same
-// float expression chord_box evaluates, so the result has the same bits.
-__device__ float chord_box_col(float a, float b, float c, float u0x, float u1x, float u0y,
-                               float u1y, float rx, float ry, float rz)
+// One detector column of a voxel column's window in one view: what find_l_3d
+// (w = h = t = 1) needs of it, and where its rays pass (k_ref_cone_chord_adj).
+struct alignas(16) ChordCol {
+    float a, b;                    // direction
+    float t0, k, half;             // parameter nearest the voxel column, reach, 1/2 + margin
+    float cmin, cmax;              // row directions c for which the reach holds
+    int ia, flags, pad;
+    union {
+        struct {                   // any column
+            float uxm, uxp, uym, uyp;   // crossings at the faces x = -+1/2 (y) and y = -+1/2 (x)
+            float x2, y2;               // detector point
+        };
+        struct {                   // kTwo: the two faces the rays pass, in the order tested
+            float d1, i1, o1, h1;       // direction component, its reciprocal, source offset, -+1/2
+            float d2, i2, o2, h2;
+            float p1x, p1y, p2x, p2y;   // where the rays pass them
+            float e2;                   // (p2x - p1x)^2 + (p2y - p1y)^2
+        };
+    };
+};
+enum { kXm = 1, kXp = 2, kYm = 4, kYp = 8,    // the crossing lies within the face's width
+       kXFirst = 16,                          // |a| > |b|: the x faces are tested first
+       kAxis = 32,                            // a = 0 or b = 0: find_l_3d's 2-D cases
+       kRowsSafe = 64,                        // every row's direction is in [cmin, cmax] or 0
+       kTwo = 128 };                          // chord_two applies to every row
+
+// n / d, correctly rounded, from the correctly rounded reciprocal i of d: with q
+// = RN(n i) within an ulp of n / d and the remainder n - q d exact, RN(q + (n -
+// q d) i) is RN(n / d) (P. Markstein, IBM J. Res. Dev. 34, 1990, theorem 8). Both
+// operands and the quotient are far from the ends of the exponent range here
+// (kRowsSafe); n = 0 gives 0.
+__device__ __forceinline__ float div_by(float n, float d, float i)
 {
-    const float hw = 0.5f, hh = 0.5f, ht = 0.5f;          // fdiv(1, 2), exact
+    const float q = fmul(n, i);
+    return __fmaf_rn(__fmaf_rn(-q, d, n), i, q);
+}
+
+// find_l_3d for a column whose rays pass exactly two faces in the plane, with
+// |c| below |a| or |b| / 1.2 in every row: the two faces' hits, or one of them
+// and a z face's (two z hits alone are a run (a / c, b / c) of more than one
+// voxel: none, or a third hit: no chord). The same float expressions as
+// chord_box, in its order.
+__device__ __forceinline__ float chord_two(const ChordCol& q, float c, float rx, float ry, float rz)
+{
+    const float s1 = div_by(c, q.d1, q.i1), s2 = div_by(c, q.d2, q.i2);
+    const float v1 = fadd(fadd(fmul(s1, -q.o1), rz), fmul(s1, q.h1));
+    const float v2 = fadd(fadd(fmul(s2, -q.o2), rz), fmul(s2, q.h2));
+    const bool k1 = fabs_ref(v1) <= 0.5f, k2 = fabs_ref(v2) <= 0.5f;
+    if (k1 && k2) {
+        const float ez = fsub(v2, v1);
+        return fsqrt(fadd(q.e2, fmul(ez, ez)));
+    }
+    if (!k1 && !k2) return 0.0f;
+    const float px = k1 ? q.p1x : q.p2x, py = k1 ? q.p1y : q.p2y, pz = k1 ? v1 : v2;
+    const float ic = fdiv(1.0f, c);
+    const float su = div_by(q.a, c, ic), sv = div_by(q.b, c, ic);
+    const float u0 = fadd(fmul(su, -rz), rx), u1 = fmul(su, 0.5f);
+    const float v0 = fadd(fmul(sv, -rz), ry), w1 = fmul(sv, 0.5f);
+    const float um = fsub(u0, u1), vm = fsub(v0, w1), up = fadd(u0, u1), vp = fadd(v0, w1);
+    const bool lo = fabs_ref(um) <= 0.5f && fabs_ref(vm) <= 0.5f;
+    const bool hi = fabs_ref(up) <= 0.5f && fabs_ref(vp) <= 0.5f;
+    if (!lo && !hi) return 0.0f;
+    const float ex = fsub(lo ? um : up, px), ey = fsub(lo ? vm : vp, py);
+    const float ez = fsub(lo ? -0.5f : 0.5f, pz);
+    return fsqrt(fadd(fadd(fmul(ex, ex), fmul(ey, ey)), fmul(ez, ez)));
+}
+
+// chord_box for a unit cube when the in-plane direction (a, b) has no zero
+// component: every value is the same float expression chord_box evaluates, in
+// its order of faces, so the result has the same bits. The in-plane crossings
+// and whether they pass come with the column; a family whose two crossings both
+// fail has no hit and needs no division. Two hits on the z faces alone are a
+// chord whose in-plane run (a / c, b / c) is at most one voxel in x and y, so
+// without a hit before them the z faces are only tested where |c| can be as
+// large as |a| and |b| (one hit gives no chord).
+__device__ __forceinline__ float chord_box_col(const ChordCol& q, float c, float rx, float ry,
+                                               float rz)
+{
     float P0[3] = {0, 0, 0}, P1[3] = {0, 0, 0};
     int nh = 0;
-    int f0 = (fabs_ref(a) > fabs_ref(b)) ? 0 : 1;
-#pragma unroll
-    for (int pass = 0; pass < 3; pass++) {
-        if (pass > 0 && nh >= 2) break;
-        int fam = (pass == 0) ? f0 : (pass == 1 ? 1 - f0 : 2);
-        float u0, u1, v0, v1, lim0, lim1;
-        if (fam == 0) {
-            u0 = u0x; u1 = u1x;
-            float s = fdiv(c, a); v0 = fadd(fmul(s, -rx), rz); v1 = fmul(s, hw);
-            lim0 = hh; lim1 = ht;
-        } else if (fam == 1) {
-            u0 = u0y; u1 = u1y;
-            float s = fdiv(c, b); v0 = fadd(fmul(s, -ry), rz); v1 = fmul(s, hh);
-            lim0 = hw; lim1 = ht;
-        } else {
-            float s = fdiv(a, c); u0 = fadd(fmul(s, -rz), rx); u1 = fmul(s, ht);
-            s = fdiv(b, c);       v0 = fadd(fmul(s, -rz), ry); v1 = fmul(s, ht);
-            lim0 = hw; lim1 = hh;
-        }
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-            if (pass > 0 && side == 1 && nh >= 2) break;
-            float uu = side ? fadd(u0, u1) : fsub(u0, u1);
-            float vv = side ? fadd(v0, v1) : fsub(v0, v1);
-            if (fabs_ref(uu) <= lim0 && fabs_ref(vv) <= lim1) {
-                float q0, q1, q2;
-                if (fam == 0)      { q0 = side ? hw : -hw; q1 = uu; q2 = vv; }
-                else if (fam == 1) { q0 = uu; q1 = side ? hh : -hh; q2 = vv; }
-                else               { q0 = uu; q1 = vv; q2 = side ? ht : -ht; }
-                if (nh == 0) { P0[0] = q0; P0[1] = q1; P0[2] = q2; }
-                else         { P1[0] = q0; P1[1] = q1; P1[2] = q2; }
-                nh++;
-            }
-        }
+    auto hit = [&](float x, float y, float z) {
+        if (nh == 0) { P0[0] = x; P0[1] = y; P0[2] = z; }
+        else         { P1[0] = x; P1[1] = y; P1[2] = z; }
+        nh++;
+    };
+    const int f = q.flags;
+    auto xfaces = [&](bool all) {
+        if (!(f & (kXm | kXp))) return;
+        const float s = fdiv(c, q.a), v0 = fadd(fmul(s, -rx), rz), v1 = fmul(s, 0.5f);
+        const float vm = fsub(v0, v1), vp = fadd(v0, v1);
+        if ((f & kXm) && fabs_ref(vm) <= 0.5f) hit(-0.5f, q.uxm, vm);
+        if ((all || nh < 2) && (f & kXp) && fabs_ref(vp) <= 0.5f) hit(0.5f, q.uxp, vp);
+    };
+    auto yfaces = [&](bool all) {
+        if (!(f & (kYm | kYp))) return;
+        const float s = fdiv(c, q.b), v0 = fadd(fmul(s, -ry), rz), v1 = fmul(s, 0.5f);
+        const float vm = fsub(v0, v1), vp = fadd(v0, v1);
+        if ((f & kYm) && fabs_ref(vm) <= 0.5f) hit(q.uym, -0.5f, vm);
+        if ((all || nh < 2) && (f & kYp) && fabs_ref(vp) <= 0.5f) hit(q.uyp, 0.5f, vp);
+    };
+    if (f & kXFirst) { xfaces(true); if (nh < 2) yfaces(false); }
+    else             { yfaces(true); if (nh < 2) xfaces(false); }
+    if (nh == 0 && fmaxf(fabsf(q.a), fabsf(q.b)) > 1.2f * fabsf(c)) return 0.0f;
+    if (nh < 2) {
+        float s = fdiv(q.a, c);
+        const float u0 = fadd(fmul(s, -rz), rx), u1 = fmul(s, 0.5f);
+        s = fdiv(q.b, c);
+        const float v0 = fadd(fmul(s, -rz), ry), v1 = fmul(s, 0.5f);
+        const float um = fsub(u0, u1), up = fadd(u0, u1), vm = fsub(v0, v1), vp = fadd(v0, v1);
+        if (fabs_ref(um) <= 0.5f && fabs_ref(vm) <= 0.5f) hit(um, vm, -0.5f);
+        if (nh < 2 && fabs_ref(up) <= 0.5f && fabs_ref(vp) <= 0.5f) hit(up, vp, 0.5f);
     }
     if (nh != 2) return 0.0f;
-    float ex = fsub(P1[0], P0[0]), ey = fsub(P1[1], P0[1]), ez = fsub(P1[2], P0[2]);
+    const float ex = fsub(P1[0], P0[0]), ey = fsub(P1[1], P0[1]), ez = fsub(P1[2], P0[2]);
     return fsqrt(fadd(fadd(fmul(ex, ex), fmul(ey, ey)), fmul(ez, ez)));
 }
 
@@ -412,104 +478,253 @@ k_ref_fan_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
     x[(long long)it * nx * ny + (long long)iy * nx + ix] = fmul(acc, scale);
 }
 
-// Cone-beam chord backprojection, restating Atx_cone_mf_cpu_new.cpp:23-85
-// (unit-cube chord, z window half-width sqrt(1 + dz^2/2)). Per view, the
-// detector columns of a voxel's window (up to kChordCols of them) get their
-// row-independent find_l_3d terms once, in shared memory (one slot per
-// thread), and every row of the window reuses them; wider windows take the
-// plain per-(column, row) evaluation. The sums run in the reference's order.
-constexpr int kChordCols = 8;
-
-__global__ void __launch_bounds__(128)
-k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
-                     const float* __restrict__ cos_phi, const float* __restrict__ sin_phi,
-                     const float* __restrict__ sdz, const float* __restrict__ ydet,
-                     const float* __restrict__ zdet, const int* __restrict__ idY,
-                     const int* __restrict__ Nv, int tmp_size, float SO, float OD, float scale,
-                     float dy_det, float y_os, float dz_det, float dz, int nx, int ny, int nz,
-                     int na, int nb)
+// Rows-fastest copy of a cone sinogram for the backprojection below: yt[(iv na +
+// ia) nb + ib] = y[(iv nb + ib) na + ia], 32 x 32 tiles through shared memory;
+// *bad is set when a value is not finite.
+__global__ void __launch_bounds__(256)
+k_ref_rows_fastest(const float* __restrict__ y, float* __restrict__ yt, int* bad, int na, int nb)
 {
-    int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    int iy = blockIdx.y;
-    int izt = blockIdx.z;            // iz + nz * it
-    int iz = izt % nz, it = izt / nz;
-    // the window columns' row-independent terms, one slot per thread
-    __shared__ float cols[6][kChordCols][128];
-    const int t = threadIdx.x;
-    if (ix >= nx) return;
-    float SD = fadd(SO, OD);
-    int na2 = na / 2, nb2 = nb / 2, nx2 = nx / 2, ny2 = ny / 2, nz2 = nz / 2;
-    long long nd = (long long)na * nb;
-    float dwin = fsqrt(fadd(1.0f, fdiv(fmul(dz, dz), 2.0f)));
-    float zc = fmul((float)(iz - nz2) + 0.5f, dz);
-    float yc = (float)(iy - ny2) + 0.5f;
-    float xc = (float)(ix - nx2) + 0.5f;
+    __shared__ float tile[32][33];
+    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
+    const long long base = (long long)blockIdx.z * na * nb;
+    bool fin = true;
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int ia = a0 + threadIdx.x, ib = b0 + k;
+        if (ia >= na || ib >= nb) continue;
+        const float v = y[base + (long long)ib * na + ia];
+        tile[k][threadIdx.x] = v;
+        fin = fin && isfinite(v);
+    }
+    if (!__syncthreads_and(fin) && threadIdx.x == 0 && threadIdx.y == 0) *bad = 1;
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int ia = a0 + k, ib = b0 + threadIdx.x;
+        if (ia < na && ib < nb) yt[base + (long long)ia * nb + ib] = tile[threadIdx.x][k];
+    }
+}
+
+constexpr int kChordWarps = 4;     // neighbouring voxel columns per thread block
+
+// Cone-beam chord backprojection, restating Atx_cone_mf_cpu_new.cpp:23-85
+// (unit-cube chord, z window half-width sqrt(1 + dz^2/2)). A warp takes one
+// voxel column, a lane one voxel (groups of 2^lz lanes where the volume is
+// low): the detector columns of a view's window and their row-independent
+// find_l_3d terms are the same for all its voxels, so the lanes compute them
+// once, one column each, for several views together. The sums run in the
+// reference's order: rows, then columns.
+//
+// Rays that miss the voxel are not evaluated. The reference's window is about
+// 5 x 6 rays per voxel and view at a magnification of two, of which about 5
+// meet it; the others get l = 0 from find_l_3d and add an exact zero (unless a
+// value is not finite: *bad turns the skipping off). A line that misses the
+// voxel's box grown by a margin m on every side passes none of the reference's
+// face tests: a test computes u = s (h - r) + r' for a slope s of the direction
+// (a, b, c) and offsets r, r' of the source, with an error of at most 2^-22
+// (|s| (|r| + 1/2) + |r'|); where the test could pass, |u| <= 1/2, so |s r| <=
+// |r'| + |s| / 2 + 1. With slopes and offsets below L that is 2^-22 (3 L / 2 +
+// 1) and the comparisons below carry less than 2^-21 L themselves: under 0.02
+// for L = 1e4 and 0.12 for L = 1e5, the two margins used. Rays with a larger
+// slope (a row at c = 0 exactly fails the z faces by inf or NaN) take the full
+// test.
+//   in xy: |a ry - b rx| > (|a| + |b|) (1/2 + m);
+//   in z:  every point of the line inside the grown square lies within 0.88 of
+//          the one nearest its centre, at t0: |rz + c t0| > 1/2 + m + |c| k,
+//          k = 0.88 / |(a, b)|.
+// zmin, zmax: the smallest non-zero and the largest |z_det|. Y has its rows
+// fastest.
+// Bound: issue (82-85 %; 871 warp instructions per column of 32 voxels and
+// view). 128^3, 120 views, 192 x 160 panel: 27.6 ms with a thread per voxel,
+// the window's columns set up by each and every ray of it evaluated; 14.2 with
+// this mapping and the skipping ray by ray; 10.1 with the rows narrowed first
+// and no division for faces that fail in the plane; 8.30 with chord_two; 6.43
+// with the margin of 0.02 and without the per-ray test where chord_two applies.
+// 6 and 10 blocks per SM 6.68 and 6.61. 200^3, 40 views, 400 x 300: 51.8 -> 10.6.
+__global__ void __launch_bounds__(kChordWarps * 32, 8)
+k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
+                     const int* __restrict__ bad, const float* __restrict__ cos_phi,
+                     const float* __restrict__ sin_phi, const float* __restrict__ sdz,
+                     const float* __restrict__ ydet, const float* __restrict__ zdet,
+                     const int* __restrict__ idY, const int* __restrict__ Nv, int tmp_size,
+                     float SO, float OD, float scale, float dy_det, float y_os, float dz_det,
+                     float dz, int nx, int ny, int nz, int na, int nb, float zmin, float zmax,
+                     int rows_uniform, float dv0, float inv_dv, int zruns, int lz)
+{
+    __shared__ ChordCol cols[kChordWarps][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int ZL = 1 << lz, g0 = lane & ~(ZL - 1), sub = lane & (ZL - 1);
+    const unsigned gm = (0xffffffffu >> (32 - ZL)) << g0;
+    const int ix = ((blockIdx.x * kChordWarps + wp) << (5 - lz)) + (g0 >> lz);
+    const int iy = blockIdx.y;
+    const int iz = ((int)(blockIdx.z % zruns) << lz) + sub, it = blockIdx.z / zruns;
+    if (ix >= nx) return;                               // whole groups
+    const bool on = iz < nz;
+    const bool skip = !*bad;
+    const float SD = fadd(SO, OD);
+    const int na2 = na / 2, nb2 = nb / 2, nx2 = nx / 2, ny2 = ny / 2, nz2 = nz / 2;
+    const long long nd = (long long)na * nb;
+    const float dwin = fsqrt(fadd(1.0f, fdiv(fmul(dz, dz), 2.0f)));
+    const float zc = fmul((float)(iz - nz2) + 0.5f, dz);
+    const float yc = (float)(iy - ny2) + 0.5f, xc = (float)(ix - nx2) + 0.5f;
     float acc = 0.0f;
-    int nvf = Nv[it];
-    for (int j = 0; j < nvf; j++) {
-        int iv = idY[it * tmp_size + j];
-        const float* yv = Y + (long long)iv * nd;
-        float c = cos_phi[iv], s = sin_phi[iv];
-        float xr = fadd(fmul(c, xc), fmul(s, yc));
-        float yr = fadd(fmul(-s, xc), fmul(c, yc));
-        float g = fdiv(SD, fmul(fadd(xr, SO), dy_det));
-        int amax = (int)floorf(fadd(fsub(fmul(fadd(yr, 1.0f), g), y_os), (float)na2));
-        int amin = (int)floorf(fadd(fsub(fmul(fsub(yr, 1.0f), g), y_os), (float)na2));
-        g = fdiv(SD, fmul(fadd(xr, SO), dz_det));
-        int bmax = (int)floorf(fadd(fmul(fadd(zc, dwin), g), (float)nb2));
-        int bmin = (int)floorf(fadd(fmul(fsub(zc, dwin), g), (float)nb2));
-        amin = max(amin, 0); amax = min(amax, na - 1);
-        bmin = max(bmin, 0); bmax = min(bmax, nb - 1);
-        float x1 = fmul(c, -SO), y1 = fmul(s, -SO), z1 = sdz[iv];
-        float cOD = fmul(c, OD), sOD = fmul(s, OD);
-        const int W = amax - amin + 1;
-        if (W >= 1 && W <= kChordCols) {
-            // chord_box's offsets of the source from the voxel centre
-            const float rx = fsub(x1, xc), ry = fsub(y1, yc), rz = fsub(z1, zc);
-            for (int k = 0; k < W; k++) {
-                const float u = __ldg(ydet + amin + k);
-                const float x2 = fsub(cOD, fmul(s, u)), y2 = fadd(sOD, fmul(c, u));
-                const float a = fsub(x2, x1), b = fsub(y2, y1);
-                float u0x = 0.0f, u1x = 0.0f, u0y = 0.0f, u1y = 0.0f;
-                if (a != 0.0f && b != 0.0f) {
-                    float q = fdiv(b, a);
-                    u0x = fadd(fmul(q, -rx), ry); u1x = fmul(q, 0.5f);
-                    q = fdiv(a, b);
-                    u0y = fadd(fmul(q, -ry), rx); u1y = fmul(q, 0.5f);
-                }
-                cols[0][k][t] = x2; cols[1][k][t] = y2;
-                cols[2][k][t] = u0x; cols[3][k][t] = u1x;
-                cols[4][k][t] = u0y; cols[5][k][t] = u1y;
-            }
-            for (int ib = bmin; ib <= bmax; ib++) {
-                const float z2 = fadd(__ldg(zdet + ib), z1);
-                const float cz = fsub(z2, z1);
-                const float* yr_ = yv + (long long)ib * na + amin;
-                for (int k = 0; k < W; k++) {
-                    const float x2 = cols[0][k][t], y2 = cols[1][k][t];
-                    const float a = fsub(x2, x1), b = fsub(y2, y1);
-                    const float l =
-                        (a == 0.0f || b == 0.0f)
-                            ? chord_box(x1, y1, z1, x2, y2, z2, 1.0f, 1.0f, 1.0f, xc, yc, zc)
-                            : chord_box_col(a, b, cz, cols[2][k][t], cols[3][k][t],
-                                            cols[4][k][t], cols[5][k][t], rx, ry, rz);
-                    acc = fadd(acc, fmul(l, __ldg(yr_ + k)));
-                }
-            }
-            continue;
+    const int nvf = Nv[it];
+    for (int jb = 0; jb < nvf; jb += ZL) {
+        // this lane's view and its window of detector columns
+        int iv = 0, amin = 0, amax = -1;
+        if (jb + sub < nvf) {
+            iv = idY[it * tmp_size + jb + sub];
+            const float c = cos_phi[iv], s = sin_phi[iv];
+            const float xr = fadd(fmul(c, xc), fmul(s, yc));
+            const float yr = fadd(fmul(-s, xc), fmul(c, yc));
+            const float g = fdiv(SD, fmul(fadd(xr, SO), dy_det));
+            amax = (int)floorf(fadd(fsub(fmul(fadd(yr, 1.0f), g), y_os), (float)na2));
+            amin = (int)floorf(fadd(fsub(fmul(fsub(yr, 1.0f), g), y_os), (float)na2));
+            amin = max(amin, 0); amax = min(amax, na - 1);
         }
-        for (int ib = bmin; ib <= bmax; ib++) {
-            float z2 = fadd(__ldg(zdet + ib), z1);
-            for (int ia = amin; ia <= amax; ia++) {
-                float u = __ldg(ydet + ia);
-                float x2 = fsub(cOD, fmul(s, u));
-                float y2 = fadd(sOD, fmul(c, u));
-                float l = chord_box(x1, y1, z1, x2, y2, z2, 1.0f, 1.0f, 1.0f, xc, yc, zc);
-                acc = fadd(acc, fmul(l, __ldg(yv + (long long)ib * na + ia)));
+        const int maxw = __reduce_max_sync(gm, amax - amin + 1);
+        if (maxw <= 0) continue;
+        int lg = 2;                                     // 4 .. ZL columns per view
+        while (lg < lz && (1 << lg) < maxw) lg++;
+        const int W = 1 << lg;
+        for (int v0 = 0; v0 < min(ZL, nvf - jb); v0 += ZL >> lg) {
+            const int vm = g0 + v0 + (sub >> lg);
+            const int lo = __shfl_sync(gm, amin, vm), hi = __shfl_sync(gm, amax, vm);
+            const int ivm = __shfl_sync(gm, iv, vm);
+            const int ia = lo + (sub & (W - 1));
+            bool ok = ia <= hi;
+            __syncwarp(gm);
+            if (ok) {
+                const float c = cos_phi[ivm], s = sin_phi[ivm];
+                const float x1 = fmul(c, -SO), y1 = fmul(s, -SO), z1 = sdz[ivm];
+                const float rx = fsub(x1, xc), ry = fsub(y1, yc);
+                const float u = __ldg(ydet + ia);
+                ChordCol q;
+                q.x2 = fsub(fmul(c, OD), fmul(s, u)); q.y2 = fadd(fmul(s, OD), fmul(c, u));
+                q.a = fsub(q.x2, x1); q.b = fsub(q.y2, y1);
+                const float aa = fabsf(q.a), bb = fabsf(q.b);
+                q.flags = (q.a == 0.0f || q.b == 0.0f) ? kAxis : aa > bb ? kXFirst : 0;
+                q.uxm = q.uxp = q.uym = q.uyp = 0.0f;
+                if (!(q.flags & kAxis)) {
+                    float w = fdiv(q.b, q.a);
+                    float u0 = fadd(fmul(w, -rx), ry), u1 = fmul(w, 0.5f);
+                    q.uxm = fsub(u0, u1); q.uxp = fadd(u0, u1);
+                    w = fdiv(q.a, q.b);
+                    u0 = fadd(fmul(w, -ry), rx); u1 = fmul(w, 0.5f);
+                    q.uym = fsub(u0, u1); q.uyp = fadd(u0, u1);
+                    q.flags |= (fabsf(q.uxm) <= 0.5f ? kXm : 0) | (fabsf(q.uxp) <= 0.5f ? kXp : 0) |
+                               (fabsf(q.uym) <= 0.5f ? kYm : 0) | (fabsf(q.uyp) <= 0.5f ? kYp : 0);
+                }
+                const float big = fmaxf(aa, bb), small = fminf(aa, bb);
+                const float far = fmaxf(fmaxf(fabsf(rx), fabsf(ry)), fabsf(z1) + fabsf(dz) * (float)nz);
+                const float err = 2.4e-7f * (fabsf(z1) + zmax);
+                // slopes and offsets below 1e4 in every row: margin 0.02; below
+                // 1e5: 0.12, row by row
+                const bool near = 1e4f * fminf(small, zmin - err) >= fmaxf(big, zmax + err) && far < 1e4f;
+                const float L = near ? 1e4f : 1e5f;
+                q.half = near ? 0.52f : 0.62f;
+                q.t0 = 0.0f; q.k = 3.0e38f;             // no reach: every row is evaluated
+                q.cmin = big / L; q.cmax = L * small;
+                if (skip && L * small >= big && far < L && big > 1e-3f) {
+                    const float d2 = q.a * q.a + q.b * q.b;
+                    q.t0 = -__fdividef(q.a * rx + q.b * ry, d2);
+                    q.k = 0.88f * rsqrtf(d2);
+                    if (zmin - err >= q.cmin && zmax + err <= q.cmax) {
+                        q.flags |= kRowsSafe;
+                        // the rays of the whole column miss
+                        if (fabsf(q.a * ry - q.b * rx) > q.half * (aa + bb)) ok = false;
+                        const int in = q.flags & (kXm | kXp | kYm | kYp);
+                        if (__popc(in) == 2 && big > 1.2f * (zmax + err)) {
+                            // the two faces in the order they are tested
+                            const bool xf = q.flags & kXFirst;
+                            const int order = xf ? in : (in >> 2) | ((in & 3) << 2);
+                            const int f1 = __ffs(order) - 1, f2 = 31 - __clz(order);
+                            const float uxm = q.uxm, uxp = q.uxp, uym = q.uym, uyp = q.uyp;
+                            auto face = [&](int f, float& d, float& i, float& o, float& h, float& px,
+                                            float& py) {
+                                const bool x = (f < 2) == xf, m = !(f & 1);
+                                d = x ? q.a : q.b; i = fdiv(1.0f, d); o = x ? rx : ry;
+                                h = m ? -0.5f : 0.5f;
+                                px = x ? h : (m ? uym : uyp);
+                                py = x ? (m ? uxm : uxp) : h;
+                            };
+                            face(f1, q.d1, q.i1, q.o1, q.h1, q.p1x, q.p1y);
+                            face(f2, q.d2, q.i2, q.o2, q.h2, q.p2x, q.p2y);
+                            const float ex = fsub(q.p2x, q.p1x), ey = fsub(q.p2y, q.p1y);
+                            q.e2 = fadd(fmul(ex, ex), fmul(ey, ey));
+                            q.flags |= kTwo;
+                        }
+                    }
+                }
+                q.ia = ia;
+                cols[wp][lane] = q;
+            }
+            const unsigned mask = __ballot_sync(gm, ok) >> g0;
+            __syncwarp(gm);
+#pragma unroll 1
+            for (int k = 0; k < ZL >> lg; k++) {
+                const int wide = __shfl_sync(gm, amax - amin + 1, g0 + v0 + k);
+                const int ivk = __shfl_sync(gm, iv, g0 + v0 + k);
+                const int ak = __shfl_sync(gm, amin, g0 + v0 + k);
+                const unsigned todo = (mask >> (k << lg)) & (0xffffffffu >> (32 - W));
+                if ((!todo && wide <= W) || !on) continue;
+                const float c = cos_phi[ivk], s = sin_phi[ivk];
+                const float xr = fadd(fmul(c, xc), fmul(s, yc));
+                const float x1 = fmul(c, -SO), y1 = fmul(s, -SO), z1 = sdz[ivk];
+                const float rx = fsub(x1, xc), ry = fsub(y1, yc), rz = fsub(z1, zc);
+                const float g = fdiv(SD, fmul(fadd(xr, SO), dz_det));
+                int bmax = (int)floorf(fadd(fmul(fadd(zc, dwin), g), (float)nb2));
+                int bmin = (int)floorf(fadd(fmul(fsub(zc, dwin), g), (float)nb2));
+                bmin = max(bmin, 0); bmax = min(bmax, nb - 1);
+                const float* yv = Y + ivk * nd;
+                // rows within the columns' reach (uniform rows with safe
+                // directions only; 0.03 of a row to spare for the estimate
+                // and the 0.005 that plan creation allows from uniform, and the
+                // rounding of c)
+                if (rows_uniform && wide <= W) {
+                    float lo = 3.0e38f, hi = -3.0e38f;
+                    for (unsigned t = todo; t; t &= t - 1) {
+                        const ChordCol& q = cols[wp][g0 + (k << lg) + __ffs(t) - 1];
+                        const float mid = __fdividef(-rz, q.t0);
+                        const float d = __fdividef(fmaf(fabsf(mid), q.k, q.half), q.t0 - q.k);
+                        if (!(q.flags & kRowsSafe) || !(q.t0 > 2.0f * q.k)) { lo = -3.0e38f; hi = 3.0e38f; }
+                        else { lo = fminf(lo, mid - d); hi = fmaxf(hi, mid + d); }
+                    }
+                    const float e1 = (lo - dv0) * inv_dv, e2 = (hi - dv0) * inv_dv;
+                    const float more = 0.03f + 5e-7f * (fabsf(z1) + zmax) * fabsf(inv_dv);
+                    bmin = max(bmin, (int)fmaxf(ceilf(fminf(e1, e2) - more), -1.0f));
+                    bmax = min(bmax, (int)fminf(floorf(fmaxf(e1, e2) + more), (float)nb));
+                }
+                for (int ib = bmin; ib <= bmax; ib++) {
+                    const float z2 = fadd(__ldg(zdet + ib), z1);
+                    const float cz = fsub(z2, z1);
+                    const float* yb = yv + ib;
+                    if (wide > W) {                     // more columns than lanes: one by one
+                        const float cOD = fmul(c, OD), sOD = fmul(s, OD);
+                        for (int ia2 = ak; ia2 < ak + wide; ia2++) {
+                            const float u = __ldg(ydet + ia2);
+                            const float l = chord_box(x1, y1, z1, fsub(cOD, fmul(s, u)),
+                                                      fadd(sOD, fmul(c, u)), z2, 1.0f, 1.0f, 1.0f,
+                                                      xc, yc, zc);
+                            acc = fadd(acc, fmul(l, __ldg(yb + (long long)ia2 * nb)));
+                        }
+                        continue;
+                    }
+                    const float ac = fabsf(cz);
+#pragma unroll 1
+                    for (unsigned t = todo; t; t &= t - 1) {
+                        const ChordCol& q = cols[wp][g0 + (k << lg) + __ffs(t) - 1];
+                        if (!(q.flags & kTwo) && ac >= q.cmin && ac <= q.cmax &&
+                            fabsf(fmaf(cz, q.t0, rz)) > fmaf(ac, q.k, q.half)) continue;
+                        const float l =
+                            (q.flags & kTwo) ? chord_two(q, cz, rx, ry, rz)
+                            : (q.flags & kAxis)
+                                ? chord_box(x1, y1, z1, q.x2, q.y2, z2, 1.0f, 1.0f, 1.0f, xc, yc, zc)
+                                : chord_box_col(q, cz, rx, ry, rz);
+                        acc = fadd(acc, fmul(l, __ldg(yb + (long long)q.ia * nb)));
+                    }
+                }
             }
         }
     }
-    x[(long long)it * nx * ny * nz + ((long long)iz * ny + iy) * nx + ix] = fmul(acc, scale);
+    if (on) x[(long long)it * nx * ny * nz + ((long long)iz * ny + iy) * nx + ix] = fmul(acc, scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -839,11 +1054,31 @@ int fl_ref_adjoint(fl_plan* p, const float* y, float* x, cudaStream_t st)
     } else {
         if ((long long)s.nz * s.nt > 65535)
             return fl_set_error(FL_ERR_UNSUPPORTED, "reference backprojector: nz * nt > 65535");
-        dim3 grid(fl_div_up(s.nx, 128), s.ny, (unsigned)s.nz * s.nt);
-        k_ref_cone_chord_adj<<<grid, 128, 0, st>>>(
-            x, y, p->d_cos_phi, p->d_sin_phi, p->d_sd_z, p->d_y_det, p->d_z_det, p->d_idY,
-            p->d_Nv, p->tmp_size, s.SO, s.OD, s.scale, s.dy_det, s.y_os, s.dz_det, s.dz, s.nx,
-            s.ny, s.nz, s.na, s.nb);
+        // scratch of this call, in stream order: the non-finite flag and the
+        // rows-fastest copy of y (a warp's lanes read neighbouring rows)
+        void* w = nullptr;
+        FL_CUDA(fl_malloc_async(&w, 256 + (size_t)p->n_rays * sizeof(float), p->pool, st));
+        int* bad = (int*)w;
+        float* yt = (float*)((char*)w + 256);
+        int e = fl_check_cuda(cudaMemsetAsync(bad, 0, sizeof(int), st), "cudaMemsetAsync");
+        const dim3 tg(fl_div_up(s.na, 32), fl_div_up(s.nb, 32), s.nv);
+        if (!e) k_ref_rows_fastest<<<tg, dim3(32, 8), 0, st>>>(y, yt, bad, s.na, s.nb);
+        // 16 or 8 lanes per voxel column where that leaves at least a quarter
+        // fewer lanes without a voxel
+        int lz = 5;
+        auto lanes = [&](int l) { return fl_div_up(s.nz, 1 << l) << l; };
+        while (lz > 3 && 4 * lanes(lz - 1) <= 3 * lanes(lz)) lz--;
+        const int zruns = fl_div_up(s.nz, 1 << lz);
+        const dim3 grid(fl_div_up(s.nx, kChordWarps << (5 - lz)), s.ny, zruns * s.nt);
+        if (!e)
+            k_ref_cone_chord_adj<<<grid, kChordWarps * 32, 0, st>>>(
+                x, yt, bad, p->d_cos_phi, p->d_sin_phi, p->d_sd_z, p->d_y_det, p->d_z_det, p->d_idY,
+                p->d_Nv, p->tmp_size, s.SO, s.OD, s.scale, s.dy_det, s.y_os, s.dz_det, s.dz, s.nx,
+                s.ny, s.nz, s.na, s.nb, p->zdet_min, p->zdet_max, p->det_kind != -2, p->v0,
+                1.0f / p->dv, zruns, lz);
+        if (!e) e = fl_check_launch("reference chord backprojection");
+        const int f = fl_check_cuda(cudaFreeAsync(w, st), "cudaFreeAsync");
+        return e ? e : f;
     }
     return fl_check_launch("reference chord backprojection");
 }
