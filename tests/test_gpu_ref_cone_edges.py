@@ -100,3 +100,17 @@ def test_chord_backprojection_can_be_captured_and_overlap():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(x, want[k])
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_gao_forward_edges_bit_exact(name):
+    import torch
+    from framelab_gb300.projector import Plan
+    p = _case(name)
+    P = Plan(p)
+    x = np.random.default_rng(9).standard_normal(P.n_vox).astype(np.float32)
+    x[P.n_vox // 2] = np.inf
+    y, yn = P.forward_gao(torch.from_numpy(x).cuda())
+    want, wantn = O.cone_gao_f32(x, p, threads=TH)
+    assert np.array_equal(y.cpu().numpy().reshape(-1), want, equal_nan=True)
+    assert np.array_equal(yn.cpu().numpy().reshape(-1), wantn, equal_nan=True)
