@@ -42,7 +42,6 @@
 namespace {
 
 constexpr int kRayChunk = 128;
-constexpr int kPixChunk = 128;
 constexpr int kVecThreads = 256;
 constexpr int kVecChunk = kVecThreads * 16;
 
@@ -280,22 +279,22 @@ k_batch_adj_refl(float* __restrict__ X, const float* __restrict__ YW,
 #undef FL_BATCH_ADJ_REFL
 }
 
-// x = A^T (pre-weighted yw), one block per chunk of 2 image rows x
-// 2*kPixChunk columns, one thread per 2 x 2 pixel block (all view groups in
-// the thread: the single-scan kernel's bits)
-__global__ void __launch_bounds__(kPixChunk)
+// x = A^T (pre-weighted yw), one block per chunk of kFanX 2 x 2 pixel blocks of
+// two image rows x kFanGroups view groups (the single-scan kernel's bits)
+__global__ void __launch_bounds__(kFanX * kFanGroups)
 k_batch_adj(float* __restrict__ X, const float* __restrict__ YW,
             const BatchSlice* __restrict__ sl, const int4* __restrict__ chunks,
             const BatchScal* __restrict__ S)
 {
     const int4 ch = chunks[blockIdx.x];       // (slice, iy0, ix0, -)
-    if (S && S[ch.x].done) return;
+    if (S && S[ch.x].done) return;            // uniform in the block
     const BatchSlice& b = sl[ch.x];
     const int ix0 = ch.z + 2 * threadIdx.x, iy0 = ch.y;
-    if (ix0 >= b.nx) return;
-    float acc[2][2];
-    fan_block_gather_all<2, 2>(acc, YW + b.woff, b.col, b.view, b.views, b.nvf, b.G, ix0, iy0,
-                               b.nx, b.ny, b.na);
+    float acc[2][2] = {};
+    if (ix0 < b.nx)
+        fan_block_gather<2, 2>(acc, YW + b.woff, b.col, b.view, b.views, b.nvf, b.G, ix0, iy0,
+                               b.nx, b.ny, b.na, threadIdx.y);
+    if (!fan_combine_groups<2, kFanX>(acc) || ix0 >= b.nx) return;
     float* xs = X + b.xoff;
 #pragma unroll
     for (int j = 0; j < 2; j++)
@@ -571,7 +570,7 @@ extern "C" int fl_batch_create(fl_plan* const* plans, int32_t n_plans, fl_batch*
         const BatchSlice& c = sl[i];
         if (c.turns == 1) {
             for (int iy = 0; iy < c.ny; iy += 2)
-                for (int ix = 0; ix < c.nx; ix += 2 * kPixChunk)
+                for (int ix = 0; ix < c.nx; ix += 2 * kFanX)
                     pix.push_back(make_int4(i, iy, ix, 0));
         } else if (c.refl) {              // kFanX primary pixel blocks per chunk (block units)
             const int hxb = (c.refl == 1 ? c.nx : c.nx / 2) / c.pblk, hyb = (c.ny / 2) / c.pblk;
@@ -730,7 +729,7 @@ static int batch_adj_w(fl_batch* b, const float* yw, float* x, const BatchScal* 
         k_batch_adj_turn<<<b->n_pix_t_chunks, dim3(kFanX, kTurnGroups), 0, s2>>>(
             x, yw, b->d_sl, b->d_pix_t, S);
     if (g)
-        k_batch_adj<<<b->n_pix_chunks, kPixChunk, 0, s>>>(x, yw, b->d_sl, b->d_pix, S);
+        k_batch_adj<<<b->n_pix_chunks, dim3(kFanX, kFanGroups), 0, s>>>(x, yw, b->d_sl, b->d_pix, S);
     int st = fl_check_launch("batched adjoint");
     if (!st) st = join_from(s, s2, b->evj);
     if (!st) st = join_from(s, s3, b->evj3);

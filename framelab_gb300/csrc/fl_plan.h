@@ -135,11 +135,10 @@ struct fl_plan {
     int adj_chunks;
     float2 *d_dq;
     // fan plans: parts per walked ray of the turn forward (1, 4 or 16; 0 =
-    // the scan's default, fl_plan_fan_lanes) and pixels per thread side of
-    // the backprojections (1 or 2; 0 = 2 once there are 4 waves of blocks)
+    // the scan's default, fl_plan_fan_lanes), pixels per thread side of the
+    // backprojections (1 or 2; 0 = fl_plan_fan_block) and thread rows of the
+    // turn and reflection backprojections (8 or 16; 0 = fl_plan_fan_groups)
     int fan_lanes, fan_block;
-    // fan plans: view groups of the turn and reflection backprojections (8
-    // or 16; 0 = 8)
     int fan_groups;
     // scale of an FP16 backprojection input (the mixed CGLS form): the largest
     // power of two with y16_scale * c_r^2 <= 1 for every ray, so c_r^2 * (a
@@ -237,15 +236,16 @@ enum {
 };
 
 // Parts per walked ray of a fan turn plan's forward: the plan's setting
-// (FL_TUNE_FAN_PARTS), else 16 for scans of fewer than 65,536 walks and 1
-// above (a batch takes its slices' values when it is built).
+// (FL_TUNE_FAN_PARTS), else fan_turn_lanes' choice (a batch takes its slices'
+// values when it is built).
 int fl_plan_fan_lanes(const fl_plan* p);
 // Pixels per thread side of a fan plan's backprojection (1 or 2): the plan's
 // setting (FL_TUNE_FAN_BLOCK), else 2 once the 2 x 2 blocks make four waves
 // of thread blocks on 152 SMs.
 int fl_plan_fan_block(const fl_plan* p);
-// View groups of a fan plan's turn and reflection backprojections (8 or 16):
-// the plan's setting (FL_TUNE_FAN_GROUPS), else 8.
+// Thread rows of a fan plan's turn and reflection backprojections (8 or 16):
+// the plan's setting (FL_TUNE_FAN_GROUPS), else 16 (batches take 8; the bits
+// are the same).
 int fl_plan_fan_groups(const fl_plan* p);
 // View chunks of a cone plan's reflection backprojection where the output is
 // FP32: the plan's setting (FL_TUNE_ADJ_CHUNKS), else one per half gigabyte of

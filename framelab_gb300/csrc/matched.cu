@@ -288,7 +288,7 @@ k_adj_fan_refl(TX* __restrict__ X, const float* __restrict__ ywp,
                int nx, int ny, int na, int nv, const int* __restrict__ skip)
 {
     if (skip && *skip) return;
-    __shared__ float smem[NG * 2 * NR * PB * PB * kFanX];
+    __shared__ float smem[kTurnGroups * 2 * NR * PB * PB * kFanX];
     fan_refl_adjoint_block<TX, NR, PB, NG>(X, ywp, col, view, G, nx, ny, na, nv,
                                            blockIdx.x * kFanX, blockIdx.y, smem);
 }
@@ -563,40 +563,31 @@ __global__ void k_weight(float* __restrict__ yw, const TY* __restrict__ y,
 }
 
 // ---------------------------------------------------------------------------
-// Fan adjoint: one thread per (pixel, frame).
+// Fan adjoint of one P x P pixel block of one frame and one view group per
+// thread: blocks of kFanX x kFanGroups threads, thread (x, g) gathers view group
+// g and group 0 writes the combined sums. P = 1 and 2 give the same bits.
+// Bound: issue. 501 x 383, 451 views, 701 bins: 769 us with a pixel per thread,
+// 374 with 2 x 2 (a ray's crossings with three planes a side serve four pixels),
+// 354 with the window taken from the block's centre; 640 x 600, 719 views: 1379
+// us with a 2 x 2 block and all four groups in one thread, 909 with a thread per
+// group.
 // ---------------------------------------------------------------------------
-// Fan adjoint of one P x P pixel block of one frame per thread. Small images
-// (GROUPED, P = 1): blocks of kFanX x kFanGroups threads, thread (x, g)
-// gathers view group g and group 0 writes the combined sums, so that four
-// times as many threads share the views. Large images (P = 2): blocks of 128
-// threads, each gathering all groups itself. Both give the same bits.
-
-template <typename TX, int P, bool GROUPED>
-__global__ void __launch_bounds__(128)
+template <typename TX, int P>
+__global__ void __launch_bounds__(kFanX * kFanGroups)
 k_adj_fan(TX* __restrict__ X, const float* __restrict__ yw, const ColEntry* __restrict__ col,
           const ViewEntry* __restrict__ view, const int* __restrict__ idY,
           const int* __restrict__ Nv, int tmp_size, DetGrid G, int nx, int ny, int na,
           const int* __restrict__ skip)
 {
     if (skip && *skip) return;                 // uniform (one flag for the launch)
-    const int ix0 = P * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int ix0 = P * (blockIdx.x * kFanX + threadIdx.x);
     const int iy0 = P * blockIdx.y;
     const int it = blockIdx.z;
-    float acc[P][P];
-    if (GROUPED) {
-#pragma unroll
-        for (int j = 0; j < P; j++)
-#pragma unroll
-            for (int i = 0; i < P; i++) acc[j][i] = 0.0f;
-        if (ix0 < nx)
-            fan_block_gather<P, P>(acc, yw, col, view, idY + it * tmp_size, Nv[it], G, ix0, iy0,
-                                   nx, ny, na, threadIdx.y);
-        if (!fan_combine_groups<P, kFanX>(acc) || ix0 >= nx) return;
-    } else {
-        if (ix0 >= nx) return;
-        fan_block_gather_all<P, P>(acc, yw, col, view, idY + it * tmp_size, Nv[it], G, ix0, iy0,
-                                   nx, ny, na);
-    }
+    float acc[P][P] = {};
+    if (ix0 < nx)
+        fan_block_gather<P, P>(acc, yw, col, view, idY + it * tmp_size, Nv[it], G, ix0, iy0,
+                               nx, ny, na, threadIdx.y);
+    if (!fan_combine_groups<P, kFanX>(acc) || ix0 >= nx) return;
     TX* xf = X + (long long)it * nx * ny;
 #pragma unroll
     for (int j = 0; j < P; j++)
@@ -930,8 +921,9 @@ int fl_plan_fan_lanes(const fl_plan* p)
     const int G = fl_plan_turns(p);
     if (G <= 1 || p->s.ndim != 2) return 1;
     if (const int NR = fl_plan_refl(p))           // walked rays: slots x columns
-        return fan_turn_lanes((long long)p->s.na * fan_refl_geom(NR, p->s.nv, p->s.na).slots);
-    return fan_turn_lanes((long long)p->s.na * (p->s.nv / G));
+        return fan_turn_lanes((long long)p->s.na * fan_refl_geom(NR, p->s.nv, p->s.na).slots, p->s.nx,
+                              p->s.ny);
+    return fan_turn_lanes((long long)p->s.na * (p->s.nv / G), p->s.nx, p->s.ny);
 }
 
 int fl_plan_adj_chunks(const fl_plan* p, bool f32_out)
@@ -948,11 +940,10 @@ int fl_plan_adj_chunks(const fl_plan* p, bool f32_out)
 
 int fl_plan_fan_groups(const fl_plan* p)
 {
-    // the quarter-turn reflection backprojection with 2 x 2 blocks keeps 8
-    // (16 would need 64 KB of shared memory per thread block)
-    const int NR = p->s.ndim == 2 ? fl_plan_refl(p) : 0;
-    if (NR == 4 && fan_refl_pblock(NR, p->s.nx, p->s.ny) == 2) return kTurnGroups;
-    return p->fan_groups ? p->fan_groups : kTurnGroups;
+    // 256^2, 360 views: 74.1 us with 8 thread rows, 53.9 with 16; 640^2, 720
+    // views: 322, 313; 64^2, 90 views: 19.1, 14.7
+    if (p->fan_groups) return p->fan_groups;
+    return p->s.ndim == 2 && fl_plan_turns(p) > 1 ? kTurnViews : kTurnGroups;
 }
 
 int fl_plan_fan_block(const fl_plan* p)
@@ -960,14 +951,18 @@ int fl_plan_fan_block(const fl_plan* p)
     if (p->fan_block) return p->fan_block;
     const fl_scan& s = p->s;
     const int T = fl_plan_turns(p);
+    // threads of 2 x 2 blocks: one per block and view group
     long long blocks2;
     if (T > 1) {
         const int hx = T == 2 ? s.nx : s.nx / 2, hy = s.ny / 2;
-        blocks2 = (long long)fl_div_up(hx, 2 * kFanX) * fl_div_up(hy, 2);
+        blocks2 = (long long)fl_div_up(hx, 2) * fl_div_up(hy, 2) * fl_plan_fan_groups(p);
     } else {
-        blocks2 = (long long)fl_div_up(s.nx, 2 * 128) * ((s.ny + 1) / 2) * s.nt;
+        blocks2 = (long long)fl_div_up(s.nx, 2) * ((s.ny + 1) / 2) * s.nt * kFanGroups;
     }
-    return blocks2 >= 4LL * 152 ? 2 : 1;
+    // 256^2, 360 views (65,536): 72.7 us with pixels, 53.9 with 2 x 2; 128 x
+    // 200, 250 views (51,200): 43.9, 31.3; 128^2, 360 views (16,384): 31.5, 54.2;
+    // general 255^2 (65,024): 113, 68; 63 x 61 (3,968): 31, 37
+    return blocks2 >= 32768 ? 2 : 1;
 }
 
 namespace {
@@ -1137,7 +1132,7 @@ void launch_adj(fl_plan* p, const float* yw, void* x, const int* skip, int xfold
         if (NG == 16) FL_ADJ_FAN_REFL(NN, PP, 16);                                           \
         else FL_ADJ_FAN_REFL(NN, PP, kTurnGroups);                                           \
     } while (0)
-        if (NR == 4 && PB == 2) FL_ADJ_FAN_REFL(4, 2, kTurnGroups);   // fl_plan_fan_groups
+        if (NR == 4 && PB == 2) FL_ADJ_FAN_REFL_G(4, 2);
         else if (NR == 4) FL_ADJ_FAN_REFL_G(4, 1);
         else if (NR == 2 && PB == 2) FL_ADJ_FAN_REFL_G(2, 2);
         else if (NR == 2) FL_ADJ_FAN_REFL_G(2, 1);
@@ -1169,19 +1164,12 @@ void launch_adj(fl_plan* p, const float* yw, void* x, const int* skip, int xfold
 #undef FL_ADJ_FAN_TURN_G
 #undef FL_ADJ_FAN_TURN
     } else {
-        // 2 x 2 pixel blocks, one thread each, once there are at least 4 waves
-        // of 128-thread blocks; else one pixel per view group
-        if (fl_plan_fan_block(p) == 2) {
-            dim3 grid(fl_div_up(s.nx, 2 * 128), (s.ny + 1) / 2, s.nt);
-            k_adj_fan<TX, 2, false><<<grid, 128, 0, st>>>((TX*)x, yw, p->d_col, p->d_view,
-                                                           p->d_idY, p->d_Nv, p->tmp_size, G,
-                                                           s.nx, s.ny, s.na, skip);
-        } else {
-            dim3 grid(fl_div_up(s.nx, kFanX), s.ny, s.nt);
-            k_adj_fan<TX, 1, true><<<grid, dim3(kFanX, kFanGroups), 0, st>>>(
-                (TX*)x, yw, p->d_col, p->d_view, p->d_idY, p->d_Nv, p->tmp_size, G, s.nx, s.ny,
-                s.na, skip);
-        }
+        // 2 x 2 pixel blocks or pixels (fl_plan_fan_block), a thread per view group
+        const int P = fl_plan_fan_block(p);
+        const dim3 grid(fl_div_up(s.nx, P * kFanX), fl_div_up(s.ny, P), s.nt), blk(kFanX, kFanGroups);
+        auto* k = P == 2 ? k_adj_fan<TX, 2> : k_adj_fan<TX, 1>;
+        k<<<grid, blk, 0, st>>>((TX*)x, yw, p->d_col, p->d_view, p->d_idY, p->d_Nv, p->tmp_size, G,
+                                s.nx, s.ny, s.na, skip);
     }
 }
 

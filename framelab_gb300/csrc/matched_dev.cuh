@@ -989,21 +989,35 @@ __device__ __forceinline__ void column_window(const DetGrid& G, float c, float s
                                               float y0, float wx, float wy, int na, int& lo,
                                               int& hi, float& dmin, float& dmax)
 {
-    float umin = 3.0e38f, umax = -3.0e38f;
-    dmin = 3.0e38f; dmax = -3.0e38f;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        float px = x0 + ((k & 1) ? wx : 0.0f);
-        float py = y0 + ((k & 2) ? wy : 0.0f);
-        float depth = G.SO + (c * px + s * py);        // distance from source along the axis
-        float lat = -s * px + c * py;
-        float u = (G.kind == 0) ? G.SD * __fdividef(lat, depth) : atan2f(lat, depth);
-        umin = fminf(umin, u); umax = fmaxf(umax, u);
-        dmin = fminf(dmin, depth); dmax = fmaxf(dmax, depth);
-    }
     float f0, f1;
-    if (G.kind == 0) { f0 = (umin - G.u0) * G.rdu; f1 = (umax - G.u0) * G.rdu; }
-    else             { f0 = (umin - G.g0) * G.rdg; f1 = (umax - G.g0) * G.rdg; }
+    if (G.kind == 0) {
+        // From the box's centre: with t = lat / depth there, a corner offset
+        // (ex wx, ey wy) / 2 moves the detector position by SD ((-s - t c) ex wx
+        // + (c - t s) ey wy) / 2 over the corner's own depth, so the shadow lies
+        // within SD (|s + t c| wx + |c - t s| wy) / (2 dmin) of the centre's (two
+        // divisions instead of the four corners' and no comparisons).
+        const float px = x0 + 0.5f * wx, py = y0 + 0.5f * wy;
+        const float depth = G.SO + (c * px + s * py);  // distance from source along the axis
+        const float lat = -s * px + c * py;
+        const float rad = 0.5f * (fabsf(c) * wx + fabsf(s) * wy);
+        dmin = depth - rad; dmax = depth + rad;
+        const float t = __fdividef(lat, depth);
+        const float uc = G.SD * t;
+        const float hw = __fdividef(0.5f * G.SD, dmin) * (fabsf(s + t * c) * wx + fabsf(c - t * s) * wy);
+        f0 = (uc - hw - G.u0) * G.rdu; f1 = (uc + hw - G.u0) * G.rdu;
+    } else {
+        float umin = 3.0e38f, umax = -3.0e38f;
+        dmin = 3.0e38f; dmax = -3.0e38f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float px = x0 + ((k & 1) ? wx : 0.0f), py = y0 + ((k & 2) ? wy : 0.0f);
+            const float depth = G.SO + (c * px + s * py);
+            const float u = atan2f(-s * px + c * py, depth);
+            umin = fminf(umin, u); umax = fmaxf(umax, u);
+            dmin = fminf(dmin, depth); dmax = fmaxf(dmax, depth);
+        }
+        f0 = (umin - G.g0) * G.rdg; f1 = (umax - G.g0) * G.rdg;
+    }
     if (f0 > f1) { float t = f0; f0 = f1; f1 = t; }
     // the rays of columns whose detector position lies in the shadow [f0, f1];
     // 0.02 column of slack covers the float evaluation and the tolerance
@@ -1097,57 +1111,6 @@ __device__ __forceinline__ void fan_block_gather(float (&acc)[PY][PX],
     }
 }
 
-// Every view group in one thread: the views in order, each into its group's
-// own sums (register sets rotated once per view), then
-// ((S_0 + S_1) + S_2) + S_3 -- the same bits as one thread per group and
-// fan_combine_groups, without the extra threads (for launches that fill the
-// GPU anyway).
-template <int PX, int PY>
-__device__ __forceinline__ void fan_block_gather_all(float (&acc)[PY][PX],
-                                                     const float* __restrict__ yw,
-                                                     const ColEntry* __restrict__ col,
-                                                     const ViewEntry* __restrict__ view,
-                                                     const int* __restrict__ views, int nvf,
-                                                     const DetGrid& G, int ix0, int iy0, int nx,
-                                                     int ny, int na)
-{
-    // part[0] always holds the group of the next view: after each view the
-    // groups rotate one place, and after the loop back into group order
-    float part[kFanGroups][PY][PX];
-#pragma unroll
-    for (int g = 0; g < kFanGroups; g++)
-#pragma unroll
-        for (int j = 0; j < PY; j++)
-#pragma unroll
-            for (int i = 0; i < PX; i++) part[g][j][i] = 0.0f;
-    auto rotate = [&]() {
-#pragma unroll
-        for (int j = 0; j < PY; j++)
-#pragma unroll
-            for (int i = 0; i < PX; i++) {
-                const float t = part[0][j][i];
-#pragma unroll
-                for (int g = 0; g < kFanGroups - 1; g++) part[g][j][i] = part[g + 1][j][i];
-                part[kFanGroups - 1][j][i] = t;
-            }
-    };
-    for (int jv = 0; jv < nvf; jv++) {
-        const int iv = views[jv];
-        fan_view_gather<PX, PY>(part[0], yw, col, view[iv], iv, G, ix0, iy0, nx, ny, na);
-        rotate();
-    }
-    for (int k = (kFanGroups - nvf % kFanGroups) % kFanGroups; k > 0; k--) rotate();
-#pragma unroll
-    for (int j = 0; j < PY; j++)
-#pragma unroll
-        for (int i = 0; i < PX; i++) {
-            float s = part[0][j][i];
-#pragma unroll
-            for (int g = 1; g < kFanGroups; g++) s += part[g][j][i];
-            acc[j][i] = s;
-        }
-}
-
 // Pixel p0 = (ix, iy) of a fan turn plan and its turns p_k = R^k p0
 // (walk_fan's R).
 template <int G>
@@ -1164,10 +1127,10 @@ __device__ __forceinline__ void fan_turn_pixels(int ix, int iy, int nx, int ny, 
     }
 }
 
-// View groups of the fan turn and reflection backprojections: 8 in batches
-// and by default; a plan may take 16 (FL_TUNE_FAN_GROUPS), which changes the
-// order of a pixel's additions.
-constexpr int kTurnGroups = 8;
+// View groups of the fan turn and reflection backprojections, and the thread
+// rows they are added in: 8 rows take two groups each (batches, which fill the
+// GPU), 16 rows one (FL_TUNE_FAN_GROUPS). The sums are the same either way.
+constexpr int kTurnViews = 16, kTurnGroups = 8;
 
 // Turn k of a P x P block of primary pixels with lower corner (ix0, iy0):
 // R^k maps the block onto the P x P block with lower corner (X0, Y0) (the
@@ -1197,7 +1160,7 @@ __host__ __device__ constexpr int turn_local_j(int k, int a, int b)
 
 // Fan adjoint of a turn plan (G = 2 or 4, one frame): the P x P block of
 // primary pixels at (ix0, iy0) and its turns, over the views iv = g, g + NG,
-// ... < nv/G of view group g. In view iv the weight of a turned pixel R^k p
+// ... < nv/G (view group g of NG). In view iv the weight of a turned pixel R^k p
 // and ray (iv, ia), from the same crossing table as the walk, multiplies the
 // value of ray (iv + j nv/G, ia) into R^{k+j mod G} p: A[(iv + j nv/G, a),
 // R^j p] = A[(iv, a), p]. acc[m][j][i] collects turn m of primary pixel
@@ -1261,16 +1224,23 @@ __device__ __forceinline__ void fan_turn_gather(float (&acc)[G][P][P],
 
 // Pixels per block row of the grouped fan backprojections.
 constexpr int kFanX = 32;
-// Parts per ray of the fan turn forward: kFanLanes for scans with fewer
-// than kFanSplitWalks walks (nv/G views x na columns), else 1. A function of
-// the scan alone, so a plan and a batch holding it choose alike.
+// Parts per ray of the fan turn forward: 4, or kFanLanes for scans of few walks
+// (nv/G views x na columns) of rays long enough for them (segments of 16
+// planes). Four threads to a ray also pay where there are rays enough: the
+// threads of a warp then walk the same part of neighbouring rays and end closer
+// together (512^2, 720 views: 262 us with whole rays, 218 with 4 parts, 263 with
+// 16; 256^2 / 360: 75, 45, 52; 128^2 / 360: 35, 21, 31; 96^2 / 180, 6,750 walks:
+// 30, 17.4, 15.5; 64^2 / 90: 21, 11.9, 12.5; 64 uneven slices: 6.49 ms, 6.51,
+// 9.65). A function of the scan alone, so a plan and a batch holding it choose
+// alike.
 constexpr int kFanLanes = 16;
-constexpr long long kFanSplitWalks = 1LL << 16;
+constexpr long long kFanSplitWalks = 1LL << 13;
 constexpr int kFanBlock = 256;       // threads per block of the fan turn forward
 
-__host__ __device__ inline int fan_turn_lanes(long long walks)
+__host__ __device__ inline int fan_turn_lanes(long long walks, int nx, int ny)
 {
-    return walks < kFanSplitWalks ? kFanLanes : 1;
+    const int n = nx > ny ? nx : ny;
+    return walks < kFanSplitWalks && n > 5 * (1 << kSegFan) ? kFanLanes : 4;
 }
 
 // One block of kFanBlock threads of the fan turn forward (G = 2 or 4, one
@@ -1343,12 +1313,13 @@ __device__ __forceinline__ void fan_turn_forward_block(const TX* __restrict__ X,
 }
 
 // One block of the fan turn backprojection (G = 2 or 4, one frame): thread
-// (x, g) of a block of kFanX x kTurnGroups threads takes the P x P block of
-// primary pixels at (ix0 + P x, iy0) -- G = 2: rows y < ny/2; G = 4: x, y <
-// n/2 -- with its turns, over view group g of the views iv < nv/G
-// (fan_turn_gather). The groups' sums meet in shared memory and are added in
-// the order g = 0, 1, ...; group 0 stores the pixels. Every thread of the
-// block must call it (it synchronises the block).
+// (x, g) of a block of kFanX x NG threads takes the P x P block of primary
+// pixels at (ix0 + P x, iy0) -- G = 2: rows y < ny/2; G = 4: x, y < n/2 -- with
+// its turns, over view group g (NG = 8: and then g + 8) of the views iv < nv/G
+// (fan_turn_gather). The groups' sums meet in shared memory and are added as
+// (S_0 + S_8) + (S_1 + S_9) + ..., so 8 and 16 threads give the same bits;
+// thread row 0 stores the pixels. Every thread of the block must call it (it
+// synchronises the block).
 template <typename TX, int G, int P, int NG = kTurnGroups>
 __device__ __forceinline__ void fan_turn_adjoint_block(TX* __restrict__ X,
                                                        const float* __restrict__ ywp,
@@ -1359,22 +1330,34 @@ __device__ __forceinline__ void fan_turn_adjoint_block(TX* __restrict__ X,
 {
     const int hx = G == 2 ? nx : nx / 2, hy = ny / 2;
     const int tx = threadIdx.x, g = threadIdx.y, bx = ix0 + P * tx;
-    float acc[G][P][P];
+    __shared__ float part[kTurnGroups][G * P * P][kFanX];
+    // NG = 16: one group per thread, the second eight added to the first's
+    // sums; NG = 8: both groups of a pair in turn
+#pragma unroll 1
+    for (int h = g; h < kTurnViews; h += NG) {
+        float acc[G][P][P];
 #pragma unroll
-    for (int m = 0; m < G; m++)
+        for (int m = 0; m < G; m++)
 #pragma unroll
-        for (int j = 0; j < P; j++)
+            for (int j = 0; j < P; j++)
 #pragma unroll
-            for (int i = 0; i < P; i++) acc[m][j][i] = 0.0f;
-    if (bx < hx)
-        fan_turn_gather<G, P>(acc, ywp, col, view, D, bx, iy0, nx, ny, na, nv, g, NG);
-    __shared__ float part[NG][G * P * P][kFanX];
+                for (int i = 0; i < P; i++) acc[m][j][i] = 0.0f;
+        if (bx < hx)
+            fan_turn_gather<G, P>(acc, ywp, col, view, D, bx, iy0, nx, ny, na, nv, h, kTurnViews);
+        const bool add = h >= kTurnGroups;
+        if (NG > kTurnGroups && add) __syncthreads();  // the first eight are there (uniform in a warp)
+        float(*mine)[kFanX] = part[h % kTurnGroups];
 #pragma unroll
-    for (int m = 0; m < G; m++)
+        for (int m = 0; m < G; m++)
 #pragma unroll
-        for (int j = 0; j < P; j++)
+            for (int j = 0; j < P; j++)
 #pragma unroll
-            for (int i = 0; i < P; i++) part[g][(m * P + j) * P + i][tx] = acc[m][j][i];
+                for (int i = 0; i < P; i++) {
+                    float& q = mine[(m * P + j) * P + i][tx];
+                    q = add ? q + acc[m][j][i] : acc[m][j][i];
+                }
+        if (NG > kTurnGroups && !add) __syncthreads();
+    }
     __syncthreads();
     if (g != 0) return;
 #pragma unroll
@@ -1388,7 +1371,7 @@ __device__ __forceinline__ void fan_turn_adjoint_block(TX* __restrict__ X,
             for (int m = 0; m < G; m++) {
                 float sum = part[0][(m * P + j) * P + i][tx];
 #pragma unroll
-                for (int k = 1; k < NG; k++) sum += part[k][(m * P + j) * P + i][tx];
+                for (int k = 1; k < kTurnGroups; k++) sum += part[k][(m * P + j) * P + i][tx];
                 Store<TX>::st(X + (long long)py[m] * nx + px[m], sum);
             }
         }
@@ -1669,13 +1652,13 @@ __device__ __forceinline__ void fan_refl_gather(float (&P)[NR][PB][PB], float (&
 constexpr int kFanReflShared = kTurnGroups * 2 * 4 * 4 * kFanX;
 
 // One block of a fan reflection backprojection: thread (x, g) of a block of
-// kFanX x kTurnGroups threads takes the PB x PB block of primary pixels with
-// lower corner (PB (bx0 + x), PB by) where it is a primary block (in block
-// units: x < the domain's width; NR = 4: x <= by) over view group g of the
-// walked views (fan_refl_gather). The groups' sums meet in shared memory
-// (smem: NG 2 NR PB^2 kFanX floats) and are added in the order g = 0, 1, ...;
-// group 0 stores the images. Every thread of the block must call it (it
-// synchronises the block).
+// kFanX x NG threads takes the PB x PB block of primary pixels with lower corner
+// (PB (bx0 + x), PB by) where it is a primary block (in block units: x < the
+// domain's width; NR = 4: x <= by) over view group g (NG = 8: and then g + 8) of
+// the walked views (fan_refl_gather). The groups' sums meet in shared memory
+// (smem: 8 2 NR PB^2 kFanX floats) and are added as the turn form's; thread row
+// 0 stores the images. Every thread of the block must call it (it synchronises
+// the block).
 template <typename TX, int NR, int PB, int NG = kTurnGroups>
 __device__ __forceinline__ void fan_refl_adjoint_block(TX* __restrict__ X,
                                                        const float* __restrict__ ywp,
@@ -1689,31 +1672,40 @@ __device__ __forceinline__ void fan_refl_adjoint_block(TX* __restrict__ X,
     const int hxb = (NR == 1 ? nx : nx / 2) / PB, hyb = (ny / 2) / PB;
     const bool prim = bx < hxb && by < hyb && (NR != 4 || bx <= by);
     const int X0 = PB * bx, Y0 = PB * by;
-    float P[NR][PB][PB], Q[NR][PB][PB];
-#pragma unroll
-    for (int j = 0; j < NR; j++)
-#pragma unroll
-        for (int b = 0; b < PB; b++)
-#pragma unroll
-            for (int a = 0; a < PB; a++) { P[j][b][a] = 0.0f; Q[j][b][a] = 0.0f; }
-    if (prim)
-        fan_refl_gather<NR, PB>(P, Q, ywp, col, view, D, X0, Y0, nx, ny, na, nv, g, NG);
     float(*part)[2 * NV][kFanX] = reinterpret_cast<float(*)[2 * NV][kFanX]>(smem);
+#pragma unroll 1
+    for (int h = g; h < kTurnViews; h += NG) {        // as in fan_turn_adjoint_block
+        float P[NR][PB][PB], Q[NR][PB][PB];
 #pragma unroll
-    for (int j = 0; j < NR; j++)
+        for (int j = 0; j < NR; j++)
 #pragma unroll
-        for (int b = 0; b < PB; b++)
+            for (int b = 0; b < PB; b++)
 #pragma unroll
-            for (int a = 0; a < PB; a++) {
-                part[g][(j * PB + b) * PB + a][tx] = P[j][b][a];
-                part[g][NV + (j * PB + b) * PB + a][tx] = Q[j][b][a];
-            }
+                for (int a = 0; a < PB; a++) { P[j][b][a] = 0.0f; Q[j][b][a] = 0.0f; }
+        if (prim)
+            fan_refl_gather<NR, PB>(P, Q, ywp, col, view, D, X0, Y0, nx, ny, na, nv, h, kTurnViews);
+        const bool add = h >= kTurnGroups;
+        if (NG > kTurnGroups && add) __syncthreads();
+        float(*mine)[kFanX] = part[h % kTurnGroups];
+#pragma unroll
+        for (int j = 0; j < NR; j++)
+#pragma unroll
+            for (int b = 0; b < PB; b++)
+#pragma unroll
+                for (int a = 0; a < PB; a++) {
+                    float& p = mine[(j * PB + b) * PB + a][tx];
+                    float& q = mine[NV + (j * PB + b) * PB + a][tx];
+                    p = add ? p + P[j][b][a] : P[j][b][a];
+                    q = add ? q + Q[j][b][a] : Q[j][b][a];
+                }
+        if (NG > kTurnGroups && !add) __syncthreads();
+    }
     __syncthreads();
     if (g != 0 || !prim) return;
     auto sum = [&](int k) {
         float t = part[0][k][tx];
 #pragma unroll
-        for (int m = 1; m < NG; m++) t += part[m][k][tx];
+        for (int m = 1; m < kTurnGroups; m++) t += part[m][k][tx];
         return t;
     };
     const bool diag = NR == 4 && X0 == Y0;

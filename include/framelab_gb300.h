@@ -240,8 +240,8 @@ int fl_plan_query(const fl_plan *plan, int option, int *value);
  * turn and reflection forwards (FL_TUNE_FAN_PARTS: 1, 4, 16), the pixel block
  * of the backprojections (FL_TUNE_FAN_BLOCK: 1 or 2) and the view groups of
  * the turn and reflection backprojections (FL_TUNE_FAN_GROUPS: 8 or 16). Only
- * the fan parts and groups change any bit of a result (the order of a ray's
- * or a pixel's additions, not the matrix). Synchronises `stream`; uses the
+ * the fan parts change any bit of a result (the order of a ray's additions, not
+ * the matrix). Synchronises `stream`; uses the
  * plan's scratch buffers. shapes (optional, [4]): the chosen forward x, y and
  * backprojection x, y of a cone plan; for a fan plan the parts count, 0, the
  * pixel block and the view groups. */
@@ -255,23 +255,21 @@ int fl_plan_autotune(fl_plan *plan, void *stream, int32_t *shapes);
 enum { FL_TUNE_ADJ_RUN = 16, FL_TUNE_ADJ_ROWS = 17 };
 /* Fan plans. FL_TUNE_FAN_PARTS: threads per walked ray of the half- or
  * quarter-turn forward (1, 4 or 16), each walking a run of the ray's segments,
- * their sums added in order; by default 16 for scans of fewer than 65,536
- * walks (nv/G views x na columns), else 1. It sets the order of a ray's
+ * their sums added in order; by default 4, or 16 for scans of fewer than 8,192
+ * walks (nv/G views x na columns) of images more than 80 pixels wide. It sets the order of a ray's
  * additions: the forward's bits (within FP32 rounding), not its matrix. A batch
  * takes each turn slice's count when it is created, so batched and single-plan
  * results stay equal bit for bit. FL_TUNE_FAN_BLOCK: pixels per thread side of
  * the fan backprojections, 1 (one pixel, view groups over threads) or 2 (a 2x2
- * block); by default 2 once there are four waves of blocks. The results do not
+ * block); by default 2 once there are enough blocks. The results do not
  * depend on it. fl_plan_option sets them (other values are refused),
  * fl_plan_query reads the values in effect. */
 enum { FL_TUNE_FAN_PARTS = 18, FL_TUNE_FAN_BLOCK = 19 };
-/* FL_TUNE_FAN_GROUPS: view groups of a fan plan's turn and reflection
- * backprojections, 8 (the default) or 16: each thread block's threads split a
- * pixel block's views into that many interleaved groups, added in order at
- * the end. It sets the order of a pixel's additions (its bits within FP32
- * rounding); batches take 8, so batched and single-plan results are equal bit
- * for bit with 8. The quarter-turn reflection form with 2 x 2 pixel blocks
- * always takes 8 (fl_plan_query reports the value in effect).
+/* FL_TUNE_FAN_GROUPS: thread rows of a fan plan's turn and reflection
+ * backprojections, 8 or 16 (the default of these forms; 8 for the general form,
+ * which has groups of its own): a pixel block's views are split into sixteen
+ * interleaved groups, one or two to a thread, added as (S_0 + S_8) + (S_1 + S_9)
+ * + ... at the end, so the results do not depend on it. Batches take 8.
  * fl_plan_autotune times both on turn and reflection plans. */
 enum { FL_TUNE_FAN_GROUPS = 20 };
 /* FL_TUNE_ADJ_CHUNKS: the reflection backprojection of a cone plan runs as
