@@ -207,14 +207,22 @@ struct Pass {
 // z-streaming 3-D level kernels for the three-tap banks (linear, Haar). A
 // block owns a column tile (warp = one row y, lane = x) and walks the slices
 // z = r, r + s, r + 2s, ... of one residue class r mod s (s = 2^level), up to
-// kSegZ output slices. The z taps of an output slice are the slices z - s, z,
+// seg_len output slices. The z taps of an output slice are the slices z - s, z,
 // z + s of its own class, so each thread keeps the z-pass inputs of its
 // sample in a three-slot register window and every slice is read once per
 // block. Every value is the same fmaf chain as in the separable pass kernels
 // above (taps in order, filters in order), so both forms give identical bits.
 constexpr int kSX = 32, kSY = 8, kST = kSX * kSY;   // column tile, threads per block
-constexpr int kSegZ = 32;                            // output slices of one class per block
+constexpr int kRowMax = 512, kRowTile = 256;         // k_syn_zx: longest whole row; columns of a part
 constexpr int kMaxStreamStep = 8;                    // dilations the streaming kernels take
+
+// element of a plane: a base that all threads share and a 32-bit byte offset,
+// which the load and store instructions add themselves
+template <typename T>
+__device__ __forceinline__ T* at(T* plane, unsigned off)
+{
+    return (T*)((const char*)plane + off);
+}
 
 // slices of residue class r in [0, nz): r, r + s, ...
 __host__ __device__ inline int class_len(int nz, int s, int r)
@@ -222,24 +230,36 @@ __host__ __device__ inline int class_len(int nz, int s, int r)
     return r < nz ? (nz - 1 - r) / s + 1 : 0;
 }
 
+// resident blocks of k_ana_stream per SM: three, and two where 27 values of v
+// are held as well as the window
+__host__ __device__ constexpr int ana_resident(int nf, int mode) { return nf == 3 && mode == 1 ? 2 : 3; }
+
 // One analysis level: the y and x passes of each slice in shared memory, the
-// z pass from the register window, fused with the coefficient write (mode 0)
-// or the Bregman update (mode 1) exactly as k_split_last.
-template <int NF, int S>
-__global__ void __launch_bounds__(kST, 2)
-k_ana_stream(const float* __restrict__ in, int nx, int ny, int nz, int nseg, Filters F,
-             BandPtrs coef, BandPtrs tout, float* __restrict__ low, int last, int mode, float tau)
+// z pass from the register window, fused with the coefficient write (MODE 0)
+// or the Bregman update (MODE 1) exactly as k_split_last. The stores of 27
+// arrays bound it. MODE 0 needs 72 registers, so three blocks fit; the window
+// is used by turns (no moves), a store adds a 32-bit offset to its band's plane,
+// and the x pass reads its own warp's row only, so one barrier a slice is left:
+// 256^3, two levels, linear bank 692 -> 624 us (5.9 of 6.7 TB/s). MODE 1 reads
+// all v of the next output before the slice's barrier, ahead of every store
+// (the band pointers may alias as far as the compiler knows): with the
+// synthesis 2757 -> 2530 us; v by groups of channels, as few as three in flight
+// beside as many in use, gave 2570-3290 us, also with three blocks.
+template <int NF, int S, int MODE>
+__global__ void __launch_bounds__(kST, ana_resident(NF, MODE))
+k_ana_stream(const float* __restrict__ in, int nx, int ny, int nz, int nseg, int seg_len, Filters F,
+             BandPtrs coef, BandPtrs tout, float* __restrict__ low, int last, float tau)
 {
     constexpr int RX = kSX + 2 * S, RY = kSY + 2 * S;   // in-plane region (halo S)
     constexpr int XR = RX - 32;                        // lanes holding a second column
     constexpr int LR = (RY + kSY - 1) / kSY;           // region rows per warp
     constexpr int NC = NF * NF;                        // channels into the z pass
     __shared__ float s_in[2][RY][RX];
-    __shared__ float s_p1[2][NF][kSY][RX];
+    __shared__ float s_p1[NF][kSY][RX];               // a warp writes and reads only its own row
     const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
     const int x0 = blockIdx.x * kSX, y0 = blockIdx.y * kSY;
     const int seg = blockIdx.z % nseg, r = blockIdx.z / nseg;
-    const int nfirst = seg * kSegZ, nend = min(nfirst + kSegZ, class_len(nz, S, r));
+    const int nfirst = seg * seg_len, nend = min(nfirst + seg_len, class_len(nz, S, r));
     if (nfirst >= nend) return;                        // uniform per block
     const int xa = wrapi(x0 - S + lane, nx);
     const int xb = lane < XR ? wrapi(x0 - S + 32 + lane, nx) : 0;
@@ -259,132 +279,166 @@ k_ana_stream(const float* __restrict__ in, int nx, int ny, int nz, int nseg, Fil
                 pb[m] = lane < XR ? __ldg(row + xb) : 0.0f;
             }
     };
-    float win[3][NC];
+    const long long plane = (long long)ny * nx;
+    const unsigned off = 4u * ((unsigned)y * nx + x);
+    float vv[MODE ? NC * NF : 1];                      // mode 1: v of the next output
+    float win[3][NC];                                  // the slices z - S, z, z + S by turns
     fetch(nfirst - 1);
-    for (int n = nfirst - 1, it = 0; n <= nend; n++, it++) {
-        const int b = it & 1;
+    for (int n = nfirst - 1, b = 0;;) {
 #pragma unroll
-        for (int m = 0; m < LR; m++)
-            if (wy + kSY * m < RY) {
-                s_in[b][wy + kSY * m][lane] = pa[m];
-                if (lane < XR) s_in[b][wy + kSY * m][32 + lane] = pb[m];
+        for (int u = 0; u < 3; u++, n++, b ^= 1) {
+            if (n > nend) return;                      // uniform per block
+#pragma unroll
+            for (int m = 0; m < LR; m++)
+                if (wy + kSY * m < RY) {
+                    s_in[b][wy + kSY * m][lane] = pa[m];
+                    if (lane < XR) s_in[b][wy + kSY * m][32 + lane] = pb[m];
+                }
+            if (n < nend) fetch(n + 1);
+            const long long zo = (r + S * (n - 1)) * plane;   // slots: z - S, z, z + S
+            if (MODE == 1 && n > nfirst && ok) {
+#pragma unroll
+                for (int band = 0; band < NC * NF; band++)
+                    if (band || last) vv[band] = *at(coef.p[band] + zo, off);
             }
-        if (n < nend) fetch(n + 1);
-        __syncthreads();
+            __syncthreads();
 #pragma unroll
-        for (int i = 0; i < NF; i++) {                 // y pass (D_i)
-            float s0 = 0.0f;
-#pragma unroll
-            for (int t = 0; t < 3; t++) s0 = fmaf(F.f[i][t], s_in[b][wy + t * S][lane], s0);
-            s_p1[b][i][wy][lane] = s0;
-            if (lane < XR) {
-                float s1 = 0.0f;
-#pragma unroll
-                for (int t = 0; t < 3; t++) s1 = fmaf(F.f[i][t], s_in[b][wy + t * S][32 + lane], s1);
-                s_p1[b][i][wy][32 + lane] = s1;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < NC; c++) { win[0][c] = win[1][c]; win[1][c] = win[2][c]; }
-#pragma unroll
-        for (int i = 0; i < NF; i++)                   // x pass (D_j) into the newest slot
-#pragma unroll
-            for (int j = 0; j < NF; j++) {
+            for (int i = 0; i < NF; i++) {             // y pass (D_i)
                 float s0 = 0.0f;
 #pragma unroll
-                for (int t = 0; t < 3; t++) s0 = fmaf(F.f[j][t], s_p1[b][i][wy][lane + t * S], s0);
-                win[2][NF * i + j] = s0;
-            }
-        if (n < nfirst + 1 || !ok) continue;           // window filling, or outside the volume
-        const int z = r + S * (n - 1);                 // slots: z - S, z, z + S
-        const long long q = ((long long)z * ny + y) * nx + x;
-        // every v of this sample is read before the first store (the band
-        // pointers may alias as far as the compiler knows), so the loads are
-        // in flight together
-        float vv[NC * NF];
+                for (int t = 0; t < 3; t++) s0 = fmaf(F.f[i][t], s_in[b][wy + t * S][lane], s0);
+                s_p1[i][wy][lane] = s0;
+                if (lane < XR) {
+                    float s1 = 0.0f;
 #pragma unroll
-        for (int band = 0; band < NC * NF; band++)
-            vv[band] = (mode == 0 || (band == 0 && !last)) ? 0.0f : coef.p[band][q];
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int k = 0; k < NF; k++) {             // z pass (D_k)
-                const int band = NF * c + k;
-                float w = 0.0f;
-#pragma unroll
-                for (int t = 0; t < 3; t++) w = fmaf(F.f[k][t], win[t][c], w);
-                if (band == 0 && !last) {
-                    if (low) low[q] = w;
-                    continue;
+                    for (int t = 0; t < 3; t++) s1 = fmaf(F.f[i][t], s_in[b][wy + t * S][32 + lane], s1);
+                    s_p1[i][wy][32 + lane] = s1;
                 }
-                if (mode == 0) {
-                    coef.p[band][q] = w;
-                } else {
-                    const float sv = vv[band] + w;         // v + W u
-                    float a = sv;                          // alpha
-                    if (!(band == 0 && last)) {
-                        const float mg = fabsf(sv) - tau;
-                        a = mg > 0.0f ? copysignf(mg, sv) : 0.0f;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < NF; i++)               // x pass (D_j) into the newest slot
+#pragma unroll
+                for (int j = 0; j < NF; j++) {
+                    float s0 = 0.0f;
+#pragma unroll
+                    for (int t = 0; t < 3; t++) s0 = fmaf(F.f[j][t], s_p1[i][wy][lane + t * S], s0);
+                    win[u][NF * i + j] = s0;
+                }
+            if (n < nfirst + 1 || !ok) continue;       // window filling, or outside the volume
+#pragma unroll
+            for (int c = 0; c < NC; c++)
+#pragma unroll
+                for (int k = 0; k < NF; k++) {         // z pass (D_k)
+                    const int band = NF * c + k;
+                    float w = 0.0f;
+#pragma unroll
+                    for (int t = 0; t < 3; t++) w = fmaf(F.f[k][t], win[(u + 1 + t) % 3][c], w);
+                    if (band == 0 && !last) {
+                        if (low) *at(low + zo, off) = w;
+                        continue;
                     }
-                    const float vn = sv - a;               // v + W u - alpha
-                    coef.p[band][q] = vn;
-                    tout.p[band][q] = a - vn;              // alpha - v_new
+                    if (MODE == 0) {
+                        *at(coef.p[band] + zo, off) = w;
+                    } else {
+                        const float sv = vv[band] + w; // v + W u
+                        float a = sv;                  // alpha
+                        if (!(band == 0 && last)) {
+                            const float mg = fabsf(sv) - tau;
+                            a = mg > 0.0f ? copysignf(mg, sv) : 0.0f;
+                        }
+                        const float vn = sv - a;       // v + W u - alpha
+                        *at(coef.p[band] + zo, off) = vn;
+                        *at(tout.p[band] + zo, off) = a - vn;   // alpha - v_new
+                    }
                 }
-            }
+        }
     }
 }
 
 // The z and x merges of one synthesis level (k_merge along z into NF^2
 // arrays, then along x into the NF arrays A_i), band 0 taken from `low` when
-// non-null. A warp covers one row y: its lanes hold the columns from S before
-// its kSX - 2S outputs to S after them, and the x taps come from the
-// neighbouring lanes. blockIdx.z = seg + nseg (i + NF r).
+// non-null. Threads along x hold aligned runs of columns: a whole row where it
+// fits in kRowMax threads (`whole`, several rows a block when it is short),
+// else kRowTile columns and one warp more for the columns beside them. The x
+// taps come from shared memory. blockIdx.z = seg + nseg (i + NF r).
+// The 27 bands' reads bound it; issue slots came next. Warps of 32 - 2S outputs
+// whose taps came by shuffles read rows from unaligned columns, and moving the
+// window and adding 64-bit addresses took half of the 135 instructions a
+// slice: 256^3, two levels, with the y merge 916 -> 759 us. Copies into a ring in
+// shared memory, four slices deep, were slower (968 us).
 template <int NF, int S>
-__global__ void __launch_bounds__(kST)
+__global__ void __launch_bounds__(kRowMax, 2)
 k_syn_zx(BandPtrs bands, const float* __restrict__ low, float* __restrict__ A, long long N,
-         int nx, int ny, int nz, int nseg, Filters R)
+         int nx, int ny, int nz, int nseg, int seg_len, int whole, Filters R)
 {
-    constexpr int OX = kSX - 2 * S, NB = NF * NF;      // outputs per warp, bands per thread
-    const int lane = threadIdx.x & 31;
-    const int y = blockIdx.y * kSY + (threadIdx.x >> 5);
+    constexpr int NB = NF * NF;                        // bands per thread
+    extern __shared__ float s_bm[];                    // [2][NF][rows][blockDim.x]
+    const int W = blockDim.x, rows = blockDim.y, tx = threadIdx.x;
+    const int y = blockIdx.y * rows + threadIdx.y;
     const int seg = blockIdx.z % nseg, ir = blockIdx.z / nseg, i = ir % NF, r = ir / NF;
-    const int nfirst = seg * kSegZ, nend = min(nfirst + kSegZ, class_len(nz, S, r));
-    if (nfirst >= nend || y >= ny) return;             // whole warps (no block barrier here)
-    const int xl = blockIdx.x * OX - S + lane;         // this lane's column, unwrapped
-    const long long col = (long long)y * nx + wrapi(xl, nx);
-    const bool out_ok = lane >= S && lane < kSX - S && xl < nx;
+    const int nfirst = seg * seg_len, nend = min(nfirst + seg_len, class_len(nz, S, r));
+    if (nfirst >= nend) return;                        // uniform per block
+    // this thread's column and the places of its x neighbours in its row
+    int x, left, right;
+    bool out_ok = y < ny;
+    if (whole) {
+        x = min(tx, nx - 1);
+        left = wrapi(x - S, nx);
+        right = wrapi(x + S, nx);
+        out_ok = out_ok && tx < nx;
+    } else {
+        // the last warp holds the S columns before the tile, then the S after it
+        const int x0 = blockIdx.x * kRowTile, h = tx - kRowTile;
+        const int off = h < 0 ? tx : h < S ? h - S : min(h - S, S - 1) + kRowTile;
+        x = wrapi(x0 + off, nx);
+        left = h < 0 ? (tx < S ? kRowTile + tx : tx - S) : tx;
+        right = h < 0 ? (tx + S < kRowTile ? tx + S : tx + S + S) : tx;
+        out_ok = out_ok && h < 0 && x0 + off < nx;
+    }
     const long long plane = (long long)ny * nx;
+    const unsigned off = 4u * ((unsigned)min(y, ny - 1) * nx + x);
     auto src = [&](int b) -> const float* {            // b = NF j + k: band NF (NF i + j) + k
         const int band = NF * NF * i + b;
         return (band == 0 && low) ? low : bands.p[band];
     };
-    float win[3][NB], nxt[NB];
+    const int row = threadIdx.y * W, step = rows * W;
+    float w[4][NB];                                    // three taps and the next slice, by turns
     auto fetch = [&](int n, float (&d)[NB]) {
-        const long long o = (long long)wrapi(r + S * n, nz) * plane + col;
+        const long long zo = wrapi(r + S * n, nz) * plane;
 #pragma unroll
-        for (int b = 0; b < NB; b++) d[b] = __ldg(src(b) + o);
+        for (int b = 0; b < NB; b++) d[b] = __ldg(at(src(b) + zo, off));
     };
-    fetch(nfirst - 1, win[1]);
-    fetch(nfirst, win[2]);
-    fetch(nfirst + 1, nxt);
-    for (int n = nfirst + 1; n <= nend; n++) {
+    fetch(nfirst - 1, w[0]);
+    fetch(nfirst, w[1]);
+    fetch(nfirst + 1, w[2]);
+    for (int n = nfirst + 1;;) {
 #pragma unroll
-        for (int b = 0; b < NB; b++) { win[0][b] = win[1][b]; win[1][b] = win[2][b]; win[2][b] = nxt[b]; }
-        if (n < nend) fetch(n + 1, nxt);
-        float a = 0.0f;                                // output slice r + S (n - 1)
+        for (int u = 0; u < 4; u++, n++) {
+            if (n > nend) return;                      // uniform per block
+            if (n < nend) fetch(n + 1, w[(u + 3) & 3]);
+            float* bm = s_bm + (u & 1) * NF * step + row;   // double-buffered: one barrier a slice
+            float own[NF];
 #pragma unroll
-        for (int j = 0; j < NF; j++) {
-            float bm = 0.0f;                           // z merge (R_k) of channel NF i + j
+            for (int j = 0; j < NF; j++) {
+                float m = 0.0f;                        // z merge (R_k) of channel NF i + j
 #pragma unroll
-            for (int k = 0; k < NF; k++)
+                for (int k = 0; k < NF; k++)
 #pragma unroll
-                for (int t = 0; t < 3; t++) bm = fmaf(R.f[k][t], win[t][NF * j + k], bm);
+                    for (int t = 0; t < 3; t++) m = fmaf(R.f[k][t], w[(u + t) & 3][NF * j + k], m);
+                own[j] = m;
+                bm[j * step + tx] = m;
+            }
+            __syncthreads();
+            float a = 0.0f;                            // output slice r + S (n - 1)
 #pragma unroll
-            for (int t = 0; t < 3; t++)                // x merge (R_j)
-                a = fmaf(R.f[j][t], __shfl_sync(0xffffffffu, bm, lane + (t - 1) * S), a);
+            for (int j = 0; j < NF; j++) {             // x merge (R_j)
+                a = fmaf(R.f[j][0], bm[j * step + left], a);
+                a = fmaf(R.f[j][1], own[j], a);
+                a = fmaf(R.f[j][2], bm[j * step + right], a);
+            }
+            if (out_ok) *at(A + i * N + (r + S * (n - 1)) * plane, off) = a;
         }
-        if (out_ok) A[i * N + (long long)(r + S * (n - 1)) * plane + (long long)y * nx + xl] = a;
     }
 }
 
@@ -392,7 +446,8 @@ k_syn_zx(BandPtrs bands, const float* __restrict__ low, float* __restrict__ A, l
 // = base + scale * result), streaming along y: a thread owns one column
 // (x, z) and walks the rows of one residue class mod S, the three y taps of
 // each output row held in a register window per input array.
-constexpr int kSegY = 32;                            // output rows of one class per thread
+constexpr int kSegY = 8;                             // output rows of one class per thread: 32 left
+                                                     // too few threads (77 x 61 x 45: 69 -> 44 us)
 
 template <int NF, int S>
 __global__ void __launch_bounds__(128)
@@ -459,6 +514,7 @@ struct fl_framelet {
     Filters D, R;
     int axes[3];                    // analysis pass order
     int fused;                      // 3-D levels through the z-streaming kernels
+    int sms;                        // multiprocessors of the device
     float* work;                    // intermediates: nf^(dim-1) + nf^(dim-2) arrays + low
     long long work_elems;
     std::vector<long long> level_base;   // first coefficient band of each level
@@ -535,6 +591,10 @@ extern "C" int fl_framelet_create(int nx, int ny, int nz, int levels, int kind, 
     int st = fl_check_cuda(fl_malloc((void**)&w->work, w->work_elems * sizeof(float)),
                            "fl_malloc(framelet)");
     if (st) { delete w; return st; }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || w->sms < 1)
+        w->sms = 152;
     *out = w;
     return fl_set_error(FL_OK, "");
 }
@@ -631,34 +691,58 @@ static void synthesis_level(fl_framelet* w, const BandPtrs& cb, const float* low
 // one kernel and the y merge (with the final base + scale) streaming along y.
 static bool stream_ok(const fl_framelet* w, int step)
 {
-    return w->fused && w->dim == 3 && w->D.nt == 3 && step <= kMaxStreamStep;
+    // offsets inside a plane are 32-bit byte counts
+    return w->fused && w->dim == 3 && w->D.nt == 3 && step <= kMaxStreamStep &&
+           (long long)w->nx * w->ny < (1LL << 30);
 }
 
-static int stream_nseg(const fl_framelet* w, int step)
+// Slices per block for `columns` blocks of one segment each, `resident` to an
+// SM: the count whose whole waves read the fewest slices (two more per segment
+// than it writes). 32 slices left the third wave half empty at 200 x 176 x 144
+// (analysis of two levels 224 us, 204 us by this rule) and most of the chip
+// idle at 77 x 61 x 45 (three levels 71 us, 32 us); at 256^3 all are alike.
+static int stream_seg_len(const fl_framelet* w, int step, long long columns, int resident)
 {
-    return fl_div_up(class_len(w->nz, step, 0), kSegZ);
+    const int len = class_len(w->nz, step, 0);
+    const long long slots = (long long)w->sms * resident;
+    int best = len;
+    long long least = -1;
+    for (int nseg = 1; nseg <= fl_div_up(len, 4); nseg++) {
+        const int sl = fl_div_up(len, nseg);
+        const long long read = (columns * nseg + slots - 1) / slots * (sl + 2);
+        if (least < 0 || read < least) { least = read; best = sl; }
+    }
+    return best;
 }
 
 template <int NF, int S>
 static void ana_stream(fl_framelet* w, const float* in, const BandPtrs& cb, const BandPtrs& tb,
                        float* low_out, int last, int mode, float tau, cudaStream_t s)
 {
-    const int nseg = stream_nseg(w, S);
-    const dim3 grid(fl_div_up(w->nx, kSX), fl_div_up(w->ny, kSY), (unsigned)(nseg * S));
-    k_ana_stream<NF, S><<<grid, kST, 0, s>>>(in, w->nx, w->ny, w->nz, nseg, w->D, cb, tb,
-                                             low_out, last, mode, tau);
+    const unsigned gx = fl_div_up(w->nx, kSX), gy = fl_div_up(w->ny, kSY);
+    const int sl = stream_seg_len(w, S, (long long)gx * gy * S, ana_resident(NF, mode));
+    const int nseg = fl_div_up(class_len(w->nz, S, 0), sl);
+    const dim3 grid(gx, gy, (unsigned)(nseg * S));
+    if (mode == 0)
+        k_ana_stream<NF, S, 0><<<grid, kST, 0, s>>>(in, w->nx, w->ny, w->nz, nseg, sl, w->D, cb, tb, low_out, last, tau);
+    else
+        k_ana_stream<NF, S, 1><<<grid, kST, 0, s>>>(in, w->nx, w->ny, w->nz, nseg, sl, w->D, cb, tb, low_out, last, tau);
 }
 
 template <int NF, int S>
 static void syn_stream(fl_framelet* w, const BandPtrs& cb, const float* low, float* dst,
                        const float* base, float scale, int final_, cudaStream_t s)
 {
-    const int nseg = stream_nseg(w, S);
     const long long N = w->N;
     float* A = w->work;                                // NF arrays
-    const dim3 grid(fl_div_up(w->nx, kSX - 2 * S), fl_div_up(w->ny, kSY),
-                    (unsigned)(nseg * NF * S));
-    k_syn_zx<NF, S><<<grid, kST, 0, s>>>(cb, low, A, N, w->nx, w->ny, w->nz, nseg, w->R);
+    const int whole = w->nx <= kRowMax;
+    const int W = whole ? 32 * fl_div_up(w->nx, 32) : kRowTile + 32;
+    const int rows = W < 256 ? 256 / W : 1;
+    const unsigned gx = whole ? 1 : fl_div_up(w->nx, kRowTile), gr = fl_div_up(w->ny, rows);
+    const int sl = stream_seg_len(w, S, (long long)gx * gr * NF * S, 1024 / (W * rows));
+    const int nseg = fl_div_up(class_len(w->nz, S, 0), sl);
+    k_syn_zx<NF, S><<<dim3(gx, gr, (unsigned)(nseg * NF * S)), dim3(W, rows), sizeof(float) * 2 * NF * W * rows, s>>>(
+        cb, low, A, N, w->nx, w->ny, w->nz, nseg, sl, whole, w->R);
     const int nsegy = fl_div_up(class_len(w->ny, S, 0), kSegY);
     const dim3 gy(fl_div_up(w->nx, 128), w->nz, (unsigned)(nsegy * S));
     k_merge_y_stream<NF, S><<<gy, 128, 0, s>>>(A, N, dst, w->nx, w->ny, w->nz, nsegy, w->R, base,
