@@ -118,8 +118,10 @@ __device__ bool slice_sum(double v, int slice, int c0, int c1, double* partials,
     return true;
 }
 
-// y = c_r^cr_power * (sum of w x along each ray), one block per ray chunk
-__global__ void __launch_bounds__(kRayChunk, 8)
+// y = c_r^cr_power * (sum of w x along each ray): the plan's general forward,
+// one block of kFanBlock threads per chunk (slice, r0) of kFanBlock / kFanParts
+// rays
+__global__ void __launch_bounds__(kFanBlock, 1024 / kFanBlock)
 k_batch_fwd(const float* __restrict__ X, const float* __restrict__ XT, float* __restrict__ Y,
             const BatchSlice* __restrict__ sl, const int2* __restrict__ chunks, int cr_power,
             int scratch, const BatchScal* __restrict__ S)
@@ -127,23 +129,17 @@ k_batch_fwd(const float* __restrict__ X, const float* __restrict__ XT, float* __
     const int2 ch = chunks[blockIdx.x];
     if (S && S[ch.x].done) return;
     const BatchSlice& b = sl[ch.x];
-    const int r = ch.y + threadIdx.x;
-    if (r >= b.na * b.nv) return;
-    float a1[1];
-    walk_fan<float, 1>(X + b.xoff, XT + b.xoff, &b.col[r].x, &b.col[r].y, b.nx, b.ny, a1,
-                       (long long)b.nx * b.ny);
-    const float acc = a1[0];
-    float cr = ray_cr(b.scale, b.colr[r], 0.0f);
-    float out = cr * acc;
-    if (cr_power == 2) out = cr * out;
-    Y[(scratch ? b.woff : b.yoff) + r] = out;
+    const int r = ch.y + threadIdx.x % (kFanBlock / kFanParts), nr = b.na * b.nv;
+    fan_forward_block<float, float>(X + b.xoff, XT + b.xoff, Y + (scratch ? b.woff : b.yoff),
+                                    b.col, b.colr, b.nx, b.ny, b.scale, cr_power, nullptr,
+                                    min(r, nr - 1), r < nr);
 }
 
 // Turn slices: the plan's turn forward, one block of kFanBlock threads per
 // chunk (slice, r0) of the rays iv < nv/G (kFanBlock / lanes rays). ypack:
 // into the batch's scratch (woff), packed per orbit; else the standard
 // layout at yoff.
-__global__ void __launch_bounds__(kFanBlock, 3)
+__global__ void __launch_bounds__(kFanBlock, 768 / kFanBlock)
 k_batch_fwd_turn(const float* __restrict__ X, const float* __restrict__ XT, float* __restrict__ Y,
                  const BatchSlice* __restrict__ sl, const int2* __restrict__ chunks,
                  int cr_power, int ypack, const BatchScal* __restrict__ S)
@@ -179,7 +175,7 @@ k_batch_transpose(const float* __restrict__ X, float* __restrict__ XT,
 // Reflection slices: the plan's reflection forward (fan_refl_forward_block),
 // one block of kFanBlock threads per chunk (slice, r0) of the walked rays
 // (slots x columns of FanReflGeom; kFanBlock / lanes rays). ypack as above.
-__global__ void __launch_bounds__(kFanBlock, 3)
+__global__ void __launch_bounds__(kFanBlock, 768 / kFanBlock)
 k_batch_fwd_refl(const float* __restrict__ X, const float* __restrict__ XT, float* __restrict__ Y,
                  const BatchSlice* __restrict__ sl, const int2* __restrict__ chunks,
                  int cr_power, int ypack, const BatchScal* __restrict__ S)
@@ -551,7 +547,7 @@ extern "C" int fl_batch_create(fl_plan* const* plans, int32_t n_plans, fl_batch*
         const BatchSlice& c = sl[i];
         for (int r = 0; r < c.na * c.nv; r += kRayChunk) wrays.push_back(make_int2(i, r));
         if (c.turns == 1)
-            for (int r = 0; r < c.na * c.nv; r += kRayChunk) rays.push_back(make_int2(i, r));
+            for (int r = 0; r < c.na * c.nv; r += kFanBlock / kFanParts) rays.push_back(make_int2(i, r));
     }
     // room for the largest walked-ray lists (16 parts per ray), which
     // fl_batch_autotune may choose
@@ -709,7 +705,7 @@ static int batch_fwd(fl_batch* b, const float* x, float* y, int cr_power, int yp
         k_batch_fwd_turn<<<b->n_ray_t_chunks, kFanBlock, 0, s2>>>(
             x, b->xt, y, b->d_sl, b->d_rays_t, cr_power, ypack, S);
     if (g)
-        k_batch_fwd<<<b->n_ray_chunks, kRayChunk, 0, s>>>(x, b->xt, y, b->d_sl, b->d_rays,
+        k_batch_fwd<<<b->n_ray_chunks, kFanBlock, 0, s>>>(x, b->xt, y, b->d_sl, b->d_rays,
                                                           cr_power, ypack, S);
     int st = fl_check_launch("batched forward");
     if (!st) st = join_from(s, s2, b->evj);

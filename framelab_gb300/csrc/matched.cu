@@ -226,8 +226,9 @@ k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
     }
 }
 
+// General fan forward (fan_forward_block).
 template <typename TX, typename TY>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(kFanBlock, 1024 / kFanBlock)
 k_fwd_fan(const TX* __restrict__ X, const TX* __restrict__ XT, TY* __restrict__ y,
           const ColEntry* __restrict__ col, const float* __restrict__ colr,
           const int* __restrict__ vframe, int nx, int ny, int na, int nv, long long nper,
@@ -235,25 +236,20 @@ k_fwd_fan(const TX* __restrict__ X, const TX* __restrict__ XT, TY* __restrict__ 
           const float* __restrict__ xscale)
 {
     if (skip && *skip) return;
-    long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= (long long)na * nv) return;
-    int iv = (int)(r / na);
-    const TX* x = X + (long long)vframe[iv] * nper;
-    const TX* xt = XT + (long long)vframe[iv] * nper;
-    float a1[1];
-    walk_fan<TX, 1>(x, xt, &col[r].x, &col[r].y, nx, ny, a1, nper);
-    float acc = a1[0];
-    float cr = ray_cr(scale, colr[r], 0.0f);
-    if (xscale) acc *= *xscale;
-    float out = cr * acc;
-    if (cr_power == 2) out = cr * out;
-    Store<TY>::st(y + r, out);
+    constexpr int nry = kFanBlock / kFanParts;
+    long long r = (long long)blockIdx.x * nry + threadIdx.x % nry;
+    const bool ray = r < (long long)na * nv;
+    if (!ray) r = (long long)na * nv - 1;
+    const int iv = (int)(r / na);
+    const long long fo = (long long)vframe[iv] * nper;
+    fan_forward_block<TX, TY>(X + fo, XT + fo, y, col, colr, nx, ny, scale, cr_power, xscale, r,
+                              ray);
 }
 
 // Fan forward of a turn plan (G = 2 or 4, one frame): blocks of kFanBlock
 // threads, L parts per ray (fan_turn_forward_block, fl_plan_fan_lanes).
 template <typename TX, typename TY, int G>
-__global__ void __launch_bounds__(kFanBlock, 3)
+__global__ void __launch_bounds__(kFanBlock, 768 / kFanBlock)
 k_fwd_fan_turn(const TX* __restrict__ X, const TX* __restrict__ XT, TY* __restrict__ y,
                const ColEntry* __restrict__ col, const float* __restrict__ colr, int nx, int ny,
                int na, int nv, float scale, int cr_power, const int* __restrict__ skip,
@@ -267,7 +263,7 @@ k_fwd_fan_turn(const TX* __restrict__ X, const TX* __restrict__ XT, TY* __restri
 // Fan reflection forms (NR = 1, 2 or 4, one frame): forward blocks of
 // kFanBlock threads, L parts per walked ray (fan_refl_forward_block).
 template <typename TX, typename TY, int NR>
-__global__ void __launch_bounds__(kFanBlock, 3)
+__global__ void __launch_bounds__(kFanBlock, 768 / kFanBlock)
 k_fwd_fan_refl(const TX* __restrict__ X, const TX* __restrict__ XT, TY* __restrict__ y,
                const ColEntry* __restrict__ col,
                const float* __restrict__ colr, int nx, int ny, int na, int nv, float scale,
@@ -1057,7 +1053,7 @@ void launch_fwd(fl_plan* p, const void* x, void* y, int cr_power, const int* ski
     } else {
         long long nr = (long long)s.na * s.nv;
         const TX* xt = fan_transposed<TX>(p, x, st);
-        k_fwd_fan<TX, TY><<<fl_div_up(nr, 128), 128, 0, st>>>(
+        k_fwd_fan<TX, TY><<<fl_div_up(nr, kFanBlock / kFanParts), kFanBlock, 0, st>>>(
             (const TX*)x, xt, (TY*)y, p->d_col, p->d_colr, p->d_view_frame, s.nx, s.ny, s.na,
             s.nv, p->n_vox_frame, s.scale, cr_power, skip, xscale);
     }

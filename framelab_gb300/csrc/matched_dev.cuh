@@ -749,13 +749,6 @@ __device__ __forceinline__ void walk_fan_parts(const TX* __restrict__ x,
     const int S = s2 - s1 + 1;
     const int q0 = L > 1 ? (lane * S) / L : 0, q1 = L > 1 ? ((lane + 1) * S) / L : S;
     if (q0 >= q1) return;
-    // first guesses at the entry of this part's first segment
-    float ag = a_in;
-    if (L > 1 && q0 > 0) {
-        const int s = pd ? s1 + q0 : s2 - q0;
-        ag = fmaxf(a_in, xabs(D, (float)(pd ? (s << SH) : min((s + 1) << SH, nD))));
-    }
-    int jx = slab_guess(X, ag, nx), jy = slab_guess(Y, ag, ny);
     const int nxy = nx * ny;                       // < 2^31 (checked at plan creation)
     // The array the walked ray's own direction reads (xt when it travels
     // mostly along x, else x) is E, the other O. Two running indices a, b
@@ -788,42 +781,40 @@ __device__ __forceinline__ void walk_fan_parts(const TX* __restrict__ x,
         const float v_in = fmaxf(fminf(tx0, tx1), fminf(ty0, ty1));
         const float v_out = fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1));
         if (!(v_in < v_out)) continue;
-        jx = slab_at(X, px, jx, lox, hix, v_in, bh, cbx);
-        jy = slab_at(Y, py, jy, loy, hiy, v_in, bh, cby);
+        // first guesses: the segment's first dominant slab, the other by its parameter
+        const float ag = __fadd_rn(bh, v_in);
+        const int jx = slab_at(X, px, xd ? (pd ? lox : hix - 1) : slab_guess(X, ag, nx), lox, hix,
+                               v_in, bh, cbx);
+        const int jy = slab_at(Y, py, xd ? slab_guess(Y, ag, ny) : (pd ? loy : hiy - 1), loy, hiy,
+                               v_in, bh, cby);
         float mx = __fsub_rn((float)(px ? jx + 1 : jx), X.kq);
         float my = __fsub_rn((float)(py ? jy + 1 : jy), Y.kq);
         float Ux = xrel(X, mx, bh, cbx), Uy = xrel(Y, my, bh, cby);
         int a = xd ? jx * ny + jy : jy * nx + jx;
         int b = xd ? jx * ny + (ny - 1 - jy) : (ny - 1 - jy) * nx + jx;
+        // The steps are straight-line code: an axis that does not step adds
+        // nothing to its plane and gets the crossing it had, and past the exit
+        // the walk runs on unseen (crossings never decrease, so a cell lies in
+        // the sub-box exactly when the walk reached it before v_out). Branches
+        // around the steps cost more: 512^2, 720 views 209 -> 194 us.
         float cur = v_in;
-        bool in = true;
         const int budget = (hix - lox) + (hiy - loy) + 2;
-        for (int it = 0; it < budget && in; it += NB) {
+        for (int it = 0; it < budget && cur < v_out; it += NB) {
             float seg[NB];
             int ia[NB], ib[NB];
             bool live[NB];
 #pragma unroll
             for (int u = 0; u < NB; u++) {
                 const float nxt = fminf(Ux, Uy);
-                live[u] = in;
+                live[u] = cur < v_out;
                 seg[u] = __fsub_rn(nxt, cur);
                 ia[u] = a; ib[u] = b;
-                if (in) {
-                    // the last voxel of the sub-box: its next crossing is the exit
-                    const bool more = nxt < v_out;
-                    if (Ux == nxt) {
-                        jx += px ? 1 : -1;
-                        mx = __fadd_rn(mx, stx); Ux = xrel(X, mx, bh, cbx);
-                        a += dax; b += dax;
-                    }
-                    if (Uy == nxt) {
-                        jy += py ? 1 : -1;
-                        my = __fadd_rn(my, sty); Uy = xrel(Y, my, bh, cby);
-                        a += day; b -= day;
-                    }
-                    cur = nxt;
-                    in = more;
-                }
+                const bool gx = Ux == nxt, gy = Uy == nxt;
+                mx = __fadd_rn(mx, gx ? stx : 0.0f); Ux = xrel(X, mx, bh, cbx);
+                my = __fadd_rn(my, gy ? sty : 0.0f); Uy = xrel(Y, my, bh, cby);
+                a += (gx ? dax : 0) + (gy ? day : 0);
+                b += (gx ? dax : 0) - (gy ? day : 0);
+                cur = nxt;
             }
             float vv[NB][NI];
 #pragma unroll
@@ -1228,19 +1219,68 @@ constexpr int kFanX = 32;
 // (nv/G views x na columns) of rays long enough for them (segments of 16
 // planes). Four threads to a ray also pay where there are rays enough: the
 // threads of a warp then walk the same part of neighbouring rays and end closer
-// together (512^2, 720 views: 262 us with whole rays, 218 with 4 parts, 263 with
-// 16; 256^2 / 360: 75, 45, 52; 128^2 / 360: 35, 21, 31; 96^2 / 180, 6,750 walks:
-// 30, 17.4, 15.5; 64^2 / 90: 21, 11.9, 12.5; 64 uneven slices: 6.49 ms, 6.51,
-// 9.65). A function of the scan alone, so a plan and a batch holding it choose
-// alike.
+// together (with blocks of 256 threads, 512^2, 720 views: 262 us with whole
+// rays, 218 with 4 parts, 263 with 16; 256^2 / 360: 75, 45, 52; 96^2 / 180,
+// 6,750 walks: 30, 17.4, 15.5; 64^2 / 90: 21, 11.9, 12.5). A function of the
+// scan alone, so a plan and a batch holding it choose alike.
 constexpr int kFanLanes = 16;
 constexpr long long kFanSplitWalks = 1LL << 13;
-constexpr int kFanBlock = 256;       // threads per block of the fan turn forward
+// Threads per block of the fan forwards. Blocks of 256 (three to an SM, and a
+// barrier over eight parts' warps) left SMs waiting for a block's last ray:
+// 512^2, 720 views 218 -> 209 us, 256^2 / 360 45 -> 42; 64 threads as 128.
+constexpr int kFanBlock = 128;
+constexpr int kFanParts = 4;         // parts per ray of the general fan forward
 
 __host__ __device__ inline int fan_turn_lanes(long long walks, int nx, int ny)
 {
     const int n = nx > ny ? nx : ny;
     return walks < kFanSplitWalks && n > 5 * (1 << kSegFan) ? kFanLanes : 4;
+}
+
+// A pointer as this thread holds it. Formed from kernel parameters and a slice's
+// or a frame's offset, the image pointers were formed anew at every gather (64
+// uneven slices: 5.42 ms, 4.31 so). Every lane of the warp must call it.
+template <typename T>
+__device__ __forceinline__ const T* held(const T* p)
+{
+    return (const T*)__shfl_sync(0xffffffffu, (unsigned long long)p, threadIdx.x & 31);
+}
+
+// One block of kFanBlock threads of the general fan forward: kFanParts threads
+// per ray, laid out and added as the parts of the turn form below (ray r of the
+// first ray r0 and tx < kFanBlock / kFanParts; a thread with ray false walks r
+// too, and stores nothing). X, XT: the ray's image. Parts shorten the longest
+// threads and bring a warp's rays closer together: 501 x 383, 701 x 451 rays
+// 208 us with one thread a ray and the stepwise branches, 203 without these
+// (walk_fan_parts), 174 with four parts (two 183, eight 179); 640 x 600,
+// 1001 x 719: 540, 534, 503; 255^2, 401 x 181: 57, 51, 37; 63 x 61, 101 x 89:
+// 18.8, 16.7, 10.7. Every thread of the block must call it.
+template <typename TX, typename TY>
+__device__ __forceinline__ void fan_forward_block(const TX* __restrict__ X,
+                                                  const TX* __restrict__ XT, TY* __restrict__ y,
+                                                  const ColEntry* __restrict__ col,
+                                                  const float* __restrict__ colr, int nx, int ny,
+                                                  float scale, int cr_power,
+                                                  const float* __restrict__ xscale, long long r,
+                                                  bool ray)
+{
+    constexpr int L = kFanParts, nry = kFanBlock / L;
+    const int tx = threadIdx.x % nry, lane = threadIdx.x / nry;
+    float acc[1];
+    walk_fan<TX, 1, L>(held(X), held(XT), &col[r].x, &col[r].y, nx, ny, acc, (long long)nx * ny,
+                       lane);
+    __shared__ float part[kFanBlock];
+    part[threadIdx.x] = acc[0];
+    __syncthreads();
+    if (lane != 0 || !ray) return;
+    float a = part[tx];
+#pragma unroll
+    for (int k = 1; k < L; k++) a += part[k * nry + tx];
+    if (xscale) a *= *xscale;
+    const float cr = ray_cr(scale, colr[r], 0.0f);
+    float out = cr * a;
+    if (cr_power == 2) out = cr * out;
+    Store<TY>::st(y + r, out);
 }
 
 // One block of kFanBlock threads of the fan turn forward (G = 2 or 4, one
@@ -1267,6 +1307,7 @@ __device__ __forceinline__ void fan_turn_forward_block(const TX* __restrict__ X,
                                                        int ypack, long long r0, int L)
 {
     const int nry = kFanBlock / L;             // rays per block
+    X = held(X); XT = held(XT);
     const int gv = nv / G;
     const int tx = threadIdx.x % nry, lane = threadIdx.x / nry;
     const long long r = r0 + tx;
@@ -1397,6 +1438,7 @@ __device__ __forceinline__ void fan_refl_forward_block(const TX* __restrict__ X,
                                                        const float* __restrict__ xscale,
                                                        int ypack, long long r0, int L)
 {
+    X = held(X); XT = held(XT);
     constexpr int NI = 2 * NR;
     const int nry = kFanBlock / L;             // rays per block
     const FanReflGeom g = fan_refl_geom(NR, nv, na);
