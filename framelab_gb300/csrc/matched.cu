@@ -35,10 +35,10 @@ namespace {
 // z-folded; the block walks only the rows ib < nb/2 and also produces each
 // ray's mirrored companion, row nb-1-ib, from the same walk. yfold selects
 // the backprojection's input layout for the output (k_weight_cone's).
-// 7 blocks per SM with the mirror: 152 x 152 x 98, 211 views 1.33 -> 0.99 ms
-// against 8 (72 registers); without it 8 and 7 are alike.
+// 7 blocks per SM (72 registers): 255^3, 179 views 11.2 ms, 12.2 with 8; with the
+// mirror 8 spilled (152 x 152 x 98, 211 views 1.33 ms, 0.99).
 template <typename TX, typename TY, bool MIRROR>
-__global__ void __launch_bounds__(128, MIRROR ? 7 : 8)
+__global__ void __launch_bounds__(128, 7)
 k_fwd_cone(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
            const float* __restrict__ colr, const RowEntry* __restrict__ row,
            const int* __restrict__ vframe, int nx, int ny, int nz, int na, int nb,
@@ -56,9 +56,9 @@ k_fwd_cone(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
     const ColEntry* ce = col + (long long)iv * na + ia;
     const RowEntry* re = row + (long long)iv * nb + ib;
     const TX* x = X + (long long)vframe[iv] * nper;
-    float accm = 0.0f;
-    float acc = walk<TX, true, false, MIRROR>(x, ce, &re->z, nx, ny, nz, nullptr,
-                                              &accm, nper);
+    ConeForm<MIRROR> f{nx * ny, make_float2(0.0f, 0.0f)};
+    walk_form(x, nper, ce, &re->z, nx, ny, MIRROR ? nz / 2 : nz, f);
+    float acc = f.acc.x, accm = f.acc.y;
     float cr = ray_cr(scale, colr[(long long)iv * na + ia], __ldg(&re->dz2));
     if (xscale) { acc *= *xscale; accm *= *xscale; }
     float out = cr * acc;
@@ -86,7 +86,7 @@ k_fwd_cone(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
 // ia) the 4 values (views iv, iv + nv/2; rows ib, nb-1-ib) side by side
 // (k_weight_packed<TY, 2>).
 template <typename TX, typename TY>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, 7)
 k_fwd_quad(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
            const float* __restrict__ colr, const RowEntry* __restrict__ row, int nx, int ny,
            int nz, int na, int nb, int nv, long long nper, float scale, int cr_power,
@@ -129,7 +129,7 @@ k_fwd_quad(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
 // ia) the 8 values (view iv + j nv/4, rows ib / nb-1-ib) side by side
 // (k_weight_packed<TY, 4>).
 template <typename TX, typename TY>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, 5)
 k_fwd_oct(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
           const float* __restrict__ colr, const RowEntry* __restrict__ row, int n, int nz,
           int na, int nb, int nv, long long nper, float scale, int cr_power,
@@ -175,11 +175,12 @@ k_fwd_oct(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restri
 // 111.2 ms at 512^3 / 720. The orbit layout answers a step with one 32-byte
 // load (two for NR = 4): 5.86 and 92.9 ms with the orbits in 2 x 2 tiles
 // (row by row 6.70 / 103.5, two or four z planes per line 7.3 / 112 and 9.4 /
-// 146; as two 16-byte loads each 7.53 / 119). 7 (NR = 4) and 9 (NR = 2) blocks
-// per SM against 6 and 8: 5.83 / 90.7; lanes in 2 x 2 quads: 5.66 / 87.7.
-// Half turn, 90 views at 256^3: 2.26 -> 2.18 ms.
+// 146; as two 16-byte loads each 7.53 / 119), 5.66 / 87.7 with the lanes in
+// 2 x 2 quads, 4.96 with the steps in batches (walk_form; 4 and 7 blocks
+// per SM -- 3, 5 or 6 fewer or more steps' registers: 5.16, 5.16, 6.6). Half
+// turn, 90 views at 256^3: 2.26, 2.18, 1.56 ms.
 template <typename TX, typename TY, int NR>
-__global__ void __launch_bounds__(128, NR == 4 ? 7 : 9)
+__global__ void __launch_bounds__(128, NR == 4 ? 4 : 7)
 k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
            const float* __restrict__ colr, const RowEntry* __restrict__ row, int nx, int ny,
            int nz, int na, int nb, int nv, long long nper, float scale, int cr_power,
@@ -323,14 +324,8 @@ k_count(int32_t* __restrict__ cnt, const ColEntry* __restrict__ col,
     int ib = (int)(q % nb);
     int iv = (int)(q / nb);
     const ColEntry* ce = col + (long long)iv * na + ia;
-    int c = 0;
-    if (three) {
-        const RowEntry* re = row + (long long)iv * nb + ib;
-        walk<float, true, true>(nullptr, ce, &re->z, nx, ny, nz, &c);
-    } else {
-        walk<float, false, true>(nullptr, ce, &ce->y, nx, ny, 1, &c);
-    }
-    cnt[r] = c;
+    const RowEntry* re = row + (long long)iv * nb + ib;
+    cnt[r] = three ? walk_count<true>(ce, &re->z, nx, ny, nz) : walk_count<false>(ce, &ce->y, nx, ny, 1);
 }
 
 // yw of the general and (MIRROR) z-mirror forms of a cone plan, rows fastest:

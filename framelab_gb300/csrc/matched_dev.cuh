@@ -34,6 +34,18 @@ __device__ __forceinline__ float2 xrel2(const AxisEntry& a, float2 m2, float bh,
                       __ffma2_rn(m2, make_float2(a.il, a.il), make_float2(cb, cb)));
 }
 
+// A pointer as this thread holds it. Formed from a kernel parameter and a
+// slice's, frame's or view's offset, a pointer is taken apart again: the offset
+// is added to the index in 64 bits at every gather (forwards of 64 uneven fan
+// slices 5.42 ms, 4.31 so; of 151 x 151 x 97, 211 views 2.02 and 1.57). Every
+// lane in mask must call it.
+template <typename T>
+__device__ __forceinline__ const T* held(const T* p, unsigned mask = 0xffffffffu)
+{
+    const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
+    return (const T*)__shfl_sync(mask, (unsigned long long)p, lane);
+}
+
 // Absolute crossing of plane k, hi part only: for estimates (which segments a
 // ray meets, first guesses of its voxels) and detector windows, never a weight.
 __device__ __forceinline__ float xabs(const AxisEntry& a, float k)
@@ -186,23 +198,18 @@ __device__ __forceinline__ void seg_walk_dom(const ColEntry* __restrict__ ce,
         // next crossings at or before the exit planes', and the exit plane's
         // crossing is computed from the same m as v_out.
         const int budget = (dhi - dlo) + (XD ? ny : nx) + (THREE ? nzr : 0) + 2;
-#pragma unroll 2
+#pragma unroll 1
         for (int it = 0; it < budget; it++) {
             const float nxt = THREE ? fminf(fminf(Ux, Uy), Uz) : fminf(Ux, Uy);
             const float seg = __fsub_rn(nxt, cur);
             const bool more = nxt < v_out;             // false at the exit (and for NaN)
-            if (Ux == nxt) {
-                jx += px ? 1 : -1;
-                mx = __fadd_rn(mx, px ? 1.0f : -1.0f); Ux = xrel(X, mx, bh, cbx);
-            }
-            if (Uy == nxt) {
-                jy += py ? 1 : -1;
-                my = __fadd_rn(my, py ? 1.0f : -1.0f); Uy = xrel(Y, my, bh, cby);
-            }
-            if (THREE && Uz == nxt) {
-                jz += pz ? 1 : -1;
-                mz = __fadd_rn(mz, pz ? 1.0f : -1.0f); Uz = xrel(Z, mz, bh, cbz);
-            }
+            if (Ux == nxt) { jx += px ? 1 : -1; mx = __fadd_rn(mx, px ? 1.0f : -1.0f); }
+            if (Uy == nxt) { jy += py ? 1 : -1; my = __fadd_rn(my, py ? 1.0f : -1.0f); }
+            if (THREE && Uz == nxt) { jz += pz ? 1 : -1; mz = __fadd_rn(mz, pz ? 1.0f : -1.0f); }
+            // straight-line: an axis that does not step gets the crossing it had
+            Ux = xrel(X, mx, bh, cbx);
+            Uy = xrel(Y, my, bh, cby);
+            if (THREE) Uz = xrel(Z, mz, bh, cbz);
             body.take(seg, more, jx, jy, jz);
             if (!more) break;
             cur = nxt;
@@ -252,60 +259,20 @@ __device__ __forceinline__ void seg_walk(const ColEntry* __restrict__ ce,
     else seg_walk_dom<THREE, false>(ce, pZ, nx, ny, nzr, s1, s2, jx, jy, jz, body);
 }
 
-// Body of the general forward and the count: the standard volume, or with
-// MIRROR the z-folded one (pairs of voxel (ix, iy, iz) and its mirror (ix,
-// iy, nz-1-iz) at pair index (iz*ny + iy)*nx + ix; acc gets the voxel's sum,
-// accm the mirror's -- the companion ray of a scan symmetric about the
-// source plane). COUNT: counts the voxels with w > 0, no loads. xlen:
-// elements available at x (checked builds verify every gather index).
-template <typename TX, bool COUNT, bool MIRROR>
-struct GenBody {
-    const TX* __restrict__ x;
-    long long xlen;
-    int nx, ny;
+// Body of the count of a ray's voxels with w > 0.
+struct CountBody {
     int cnt = 0;
-    float acc = 0.0f, xv = 0.0f;
-    float2 acc2 = make_float2(0.0f, 0.0f), xv2 = make_float2(0.0f, 0.0f);
-    __device__ __forceinline__ void load(int jx, int jy, int jz, float& s, float2& s2) const
-    {
-        if (COUNT) return;
-        const int v = (jz * ny + jy) * nx + jx;      // < 2^31 (checked at plan creation)
-        if (MIRROR) {
-            s2 = make_float2(0.0f, 0.0f);
-            if (FL_IN(2 * (long long)v + 1, xlen)) s2 = Store<TX>::ld2(x + 2 * (long long)v);
-        } else {
-            s = 0.0f;
-            if (FL_IN(v, xlen)) s = ldv(x + v);
-        }
-    }
-    __device__ __forceinline__ void at(int jx, int jy, int jz) { load(jx, jy, jz, xv, xv2); }
-    __device__ __forceinline__ void take(float seg, bool more, int jx, int jy, int jz)
-    {
-        float xn = 0.0f;
-        float2 xn2 = make_float2(0.0f, 0.0f);
-        if (more) load(jx, jy, jz, xn, xn2);
-        if (COUNT) cnt += seg > 0.0f;
-        else if (MIRROR) acc2 = __ffma2_rn(make_float2(seg, seg), xv2, acc2);
-        else acc = fmaf(seg, xv, acc);
-        xv = xn;
-        xv2 = xn2;
-    }
+    __device__ __forceinline__ void at(int, int, int) {}
+    __device__ __forceinline__ void take(float seg, bool, int, int, int) { cnt += seg > 0.0f; }
 };
 
-// The general walk (2-D with THREE = false; z-folded volume with MIRROR: the
-// ray must descend from the source plane, so it stays in iz < nz/2).
-// Returns sum over voxels of w * x; *nseg counts segments with w > 0.
-template <typename TX, bool THREE, bool COUNT, bool MIRROR = false>
-__device__ __forceinline__ float walk(const TX* __restrict__ x, const ColEntry* ce,
-                                      const AxisEntry* pZ, int nx, int ny, int nz, int* nseg,
-                                      float* accm = nullptr, long long xlen = 0)
+template <bool THREE>
+__device__ __forceinline__ int walk_count(const ColEntry* ce, const AxisEntry* pZ, int nx, int ny,
+                                          int nz)
 {
-    GenBody<TX, COUNT, MIRROR> b{x, xlen, nx, ny};
-    if (!(MIRROR && !(__ldg(&pZ->ih) < 0.0f)))      // the folded walk takes descending rays
-        seg_walk<THREE>(ce, pZ, nx, ny, THREE ? (MIRROR ? nz / 2 : nz) : 1, b);
-    if (COUNT) *nseg = b.cnt;
-    if (MIRROR) { *accm = b.acc2.y; return b.acc2.x; }
-    return b.acc;
+    CountBody b;
+    seg_walk<THREE>(ce, pZ, nx, ny, THREE ? nz : 1, b);
+    return b.cnt;
 }
 
 // Folded pair index of voxel (x, y, z) in the 4 x 4 tiled volume of a
@@ -316,35 +283,191 @@ __device__ __forceinline__ int tiled_pair(int x, int y, int zb, int nx4)
     return zb + (((y >> 2) * nx4 + (x >> 2)) << 4) + ((y & 3) << 2) + (x & 3);
 }
 
-// The z-mirror walk of a descending ray with the half-turn partner (plan
-// flag rot): besides the folded pair of voxel (ix, iy, iz) it gathers the
-// pair of voxel (nx-1-ix, ny-1-iy, iz), which the turned ray of view v + nv/2
-// crosses with the same segment. x is the tiled folded volume (nx, ny
-// multiples of 4). acc gets the (voxel, mirror) sums, accr the turned pair's.
-template <typename TX>
-struct QuadBody {
-    const TX* __restrict__ x;
-    long long xlen;
-    int nxy, nx4;
-    float2 acc = make_float2(0.0f, 0.0f), accr = make_float2(0.0f, 0.0f);
-    float2 xv = make_float2(0.0f, 0.0f), xr = make_float2(0.0f, 0.0f);
-    __device__ __forceinline__ void load(int jx, int jy, int jz, float2& a, float2& r) const
+// Steps per batch of the forms. Bound: issue slots and the L1 (neighbouring rays'
+// gathers are not dense). One step at a time behind branches, the next step's
+// values a step ahead: 256^3, 360 views (NR = 4) 5.66 ms, 90 views (NR = 2) 2.19,
+// 64^3 / 72 85 us; 4 and 2 steps at 128 and 72 registers: 4.96, 1.56, 42. NR = 4
+// by 1, 2, 3 steps (72, 96, 128 registers): 5.42, 5.16, 5.01; NR = 2 by 1, 3, 4:
+// 1.95, 1.57, 1.60. General 151 x 151 x 97, 211 views 1.65 -> 1.43 ms, 255^3 / 179
+// 12.8 -> 11.2; z-mirror 152 x 152 x 98 / 211 0.99 -> 0.85, 511 x 511 x 16 / 179
+// 1.77 -> 1.37; by two, three, six steps 1.63, 1.55, 1.50 (general; 1.56 with
+// the index formed from jx, jy, jz). Half turn 180 x 180 x 100, 178 views 1.04 ->
+// 0.76; quarter turns 180 views 0.81 -> 0.64, 128^3 / 240 0.63 -> 0.48.
+constexpr int kRefl4Batch = 4, kRefl2Batch = 2, kQuadBatch = 4, kOctBatch = 4,
+              kConeBatch = 4;
+
+// The forwards' walk: seg_walk's voxels and segments in the same order,
+// Form::NB steps at a time as straight-line code (an axis that does not step
+// gets the crossing it had; past the exit the walk runs on unseen: crossings
+// never decrease, so a voxel lies in the sub-box exactly when the walk reached it
+// before v_out), their gathers issued together. Form::DOWN: a folded volume,
+// walked by descending rays only. xlen: elements available at x (checked
+// builds verify every gather index). Form (one kernel form's gathers and sums; V
+// the values of one step):
+//   index(jx, jy, zb, k)     what load and add need of voxel (jx, jy), plane
+//                            offset zb (z times the form's plane size xy();
+//                            LINEAR: the voxel's index, kept step by step)
+//   load(x, xlen, k, v)      the (voxel, mirror) pairs
+//   add(seg, k, v)           the sums
+template <typename TX, typename Form>
+__device__ __forceinline__ void walk_form(const TX* __restrict__ xp, long long xlen,
+                                          const ColEntry* __restrict__ ce,
+                                          const AxisEntry* __restrict__ pZ, int nx, int ny,
+                                          int nzr, Form& form)
+{
+    constexpr int SH = kSegCone, NB = Form::NB, V = Form::V;
+    const float ihx = __ldg(&ce->x.ih), ilx = __ldg(&ce->x.il);
+    const float ihy = __ldg(&ce->y.ih), ily = __ldg(&ce->y.il);
+    const float ihz = __ldg(&pZ->ih), ilz = __ldg(&pZ->il);
+    const bool px = ihx > 0.0f, py = ihy > 0.0f, pz = ihz > 0.0f;
+    const bool xd = fabsf(ihx) <= fabsf(ihy), pd = xd ? px : py;
+    const int nD = xd ? nx : ny;
+    int s1 = 0, s2 = -1;
+    bool hit;
     {
-        const int zb = jz * nxy;                     // < 2^31 (checked at plan creation)
-        const int t = tiled_pair(jx, jy, zb, nx4), tr = 2 * zb + nxy - 1 - t;
-        a = make_float2(0.0f, 0.0f); r = a;
-        if (FL_IN(2 * (long long)t + 1, xlen)) a = Store<TX>::ld2(x + 2 * (long long)t);
-        if (FL_IN(2 * (long long)tr + 1, xlen)) r = Store<TX>::ld2(x + 2 * (long long)tr);
+        const AxisEntry X{__ldg(&ce->x.kq), ihx, ilx, 0.0f}, Y{__ldg(&ce->y.kq), ihy, ily, 0.0f};
+        const AxisEntry Z{__ldg(&pZ->kq), ihz, ilz, 0.0f};
+        const float x0 = xabs(X, 0.0f), x1 = xabs(X, (float)nx), y0 = xabs(Y, 0.0f),
+                    y1 = xabs(Y, (float)ny), z0 = xabs(Z, 0.0f), z1 = xabs(Z, (float)nzr);
+        const float a_in = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1));
+        const float a_out = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1));
+        hit = seg_range<SH>(xd ? X : Y, nD, a_in, a_out, s1, s2);
     }
-    __device__ __forceinline__ void at(int jx, int jy, int jz) { load(jx, jy, jz, xv, xr); }
-    __device__ __forceinline__ void take(float seg, bool more, int jx, int jy, int jz)
+    if (Form::DOWN && pz) hit = false;
+    // warp alignment, as in seg_walk
+    const unsigned am = __activemask();
+    const TX* x = held(xp, am);
+    const int key = (xd ? 2 : 0) | (pd ? 1 : 0);
+    const int lo = __reduce_min_sync(am, hit ? s1 : 0x7fffffff);
+    const int hi = __reduce_max_sync(am, hit ? s2 : -1);
+    if (!hit) return;
+    if (__match_any_sync(am, key) == am) { s1 = lo; s2 = hi; }
+    const float stx = px ? 1.0f : -1.0f, sty = py ? 1.0f : -1.0f, stz = pz ? 1.0f : -1.0f;
+    const int rowlen = Form::LINEAR ? nx : 1, xy = form.xy();
+    const int dx = px ? 1 : -1, dy = py ? rowlen : -rowlen;
+    const int dz = Form::DOWN || !pz ? -xy : xy;
+    for (int q = s1; q <= s2; q++) {
+        const int sg = pd ? q : s1 + s2 - q;
+        const AxisEntry X{__ldg(&ce->x.kq), ihx, ilx, __ldg(&ce->x.c)};
+        const AxisEntry Y{__ldg(&ce->y.kq), ihy, ily, __ldg(&ce->y.c)};
+        const AxisEntry Z{__ldg(&pZ->kq), ihz, ilz, __ldg(&pZ->c)};
+        float bh, be;
+        make_anchor<SH>(xd ? X : Y, sg, nD, bh, be);
+        const float cbx = __fsub_rn(X.c, be), cby = __fsub_rn(Y.c, be), cbz = __fsub_rn(Z.c, be);
+        const int dlo = sg << SH, dhi = min((sg + 1) << SH, nD);
+        const int lox = xd ? dlo : 0, hix = xd ? dhi : nx, loy = xd ? 0 : dlo, hiy = xd ? ny : dhi;
+        const float tx0 = xrel(X, __fsub_rn((float)lox, X.kq), bh, cbx);
+        const float tx1 = xrel(X, __fsub_rn((float)hix, X.kq), bh, cbx);
+        const float ty0 = xrel(Y, __fsub_rn((float)loy, Y.kq), bh, cby);
+        const float ty1 = xrel(Y, __fsub_rn((float)hiy, Y.kq), bh, cby);
+        const float tz0 = xrel(Z, __fsub_rn(0.0f, Z.kq), bh, cbz);
+        const float tz1 = xrel(Z, __fsub_rn((float)nzr, Z.kq), bh, cbz);
+        const float v_in = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fminf(tz0, tz1));
+        const float v_out = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
+        if (!(v_in < v_out)) continue;
+        const float ag = __fadd_rn(bh, v_in);
+        int jx = slab_at(X, px, slab_guess(X, ag, nx), lox, hix, v_in, bh, cbx);
+        int jy = slab_at(Y, py, slab_guess(Y, ag, ny), loy, hiy, v_in, bh, cby);
+        const int jz = slab_at(Z, pz, slab_guess(Z, ag, nzr), 0, nzr, v_in, bh, cbz);
+        float mx = __fsub_rn((float)(px ? jx + 1 : jx), X.kq);
+        float my = __fsub_rn((float)(py ? jy + 1 : jy), Y.kq);
+        float mz = __fsub_rn((float)(pz ? jz + 1 : jz), Z.kq);
+        float Ux = xrel(X, mx, bh, cbx), Uy = xrel(Y, my, bh, cby), Uz = xrel(Z, mz, bh, cbz);
+        int zb = jz * xy + (Form::LINEAR ? jy * nx + jx : 0);   // < 2^31 (checked at plan creation)
+        float cur = v_in;
+        const int budget = (dhi - dlo) + (xd ? ny : nx) + nzr + 2;
+        for (int it = 0; it < budget && cur < v_out; it += NB) {
+            float seg[NB];
+            int k[NB][3];
+            bool live[NB];
+#pragma unroll
+            for (int u = 0; u < NB; u++) {
+                const float nxt = fminf(fminf(Ux, Uy), Uz);
+                live[u] = cur < v_out;
+                seg[u] = __fsub_rn(nxt, cur);
+                form.index(jx, jy, zb, k[u]);
+                const bool gx = Ux == nxt, gy = Uy == nxt, gz = Uz == nxt;
+                if (gx) { mx = __fadd_rn(mx, stx); (Form::LINEAR ? zb : jx) += dx; }
+                if (gy) { my = __fadd_rn(my, sty); (Form::LINEAR ? zb : jy) += dy; }
+                if (gz) { mz = __fadd_rn(mz, stz); zb += dz; }
+                Ux = xrel(X, mx, bh, cbx); Uy = xrel(Y, my, bh, cby); Uz = xrel(Z, mz, bh, cbz);
+                cur = nxt;
+            }
+            float2 v[NB][V];
+#pragma unroll
+            for (int u = 0; u < NB; u++) {
+#pragma unroll
+                for (int j = 0; j < V; j++) v[u][j] = make_float2(0.0f, 0.0f);
+                if (live[u]) form.load(x, xlen, k[u], v[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < NB; u++)
+                if (live[u]) form.add(make_float2(seg[u], seg[u]), k[u], v[u]);
+        }
+    }
+}
+
+// The standard volume (acc.x), or with MIRROR the z-folded one: pairs of voxel
+// (ix, iy, iz) and its mirror (ix, iy, nz-1-iz) at pair index (iz*ny + iy)*nx +
+// ix; acc.y gets the mirror's sum, the companion ray of a scan symmetric about
+// the source plane.
+template <bool MIRROR>
+struct ConeForm {
+    static constexpr int NB = kConeBatch, V = 1;
+    static constexpr bool DOWN = MIRROR;
+    static constexpr bool LINEAR = true;
+    int nxy;
+    float2 acc;
+    __device__ __forceinline__ int xy() const { return nxy; }
+    __device__ __forceinline__ void index(int, int, int zb, int (&k)[3]) const
     {
-        float2 xn = make_float2(0.0f, 0.0f), xnr = xn;
-        if (more) load(jx, jy, jz, xn, xnr);
-        acc = __ffma2_rn(make_float2(seg, seg), xv, acc);
-        accr = __ffma2_rn(make_float2(seg, seg), xr, accr);
-        xv = xn;
-        xr = xnr;
+        k[0] = zb;
+    }
+    template <typename TX>
+    __device__ __forceinline__ void load(const TX* __restrict__ x, long long xlen,
+                                         const int (&k)[3], float2 (&v)[V]) const
+    {
+        if (MIRROR) {
+            if (FL_IN(2 * (long long)k[0] + 1, xlen)) v[0] = Store<TX>::ld2(x + 2 * (long long)k[0]);
+        } else {
+            if (FL_IN(k[0], xlen)) v[0].x = ldv(x + k[0]);
+        }
+    }
+    __device__ __forceinline__ void add(float2 w, const int (&)[3], const float2 (&v)[V])
+    {
+        if (MIRROR) acc = __ffma2_rn(w, v[0], acc);
+        else acc.x = fmaf(w.x, v[0].x, acc.x);
+    }
+};
+
+// Half turn (plan flag rot): besides the folded pair of voxel (ix, iy, iz) the
+// walk gathers the pair of voxel (nx-1-ix, ny-1-iy, iz), which the turned ray
+// of view v + nv/2 crosses with the same segment. x is the tiled folded volume
+// (nx, ny multiples of 4). acc[0]: the (voxel, mirror) sums, acc[1] the turned
+// pair's.
+struct QuadForm {
+    static constexpr int NB = kQuadBatch, V = 2;
+    static constexpr bool DOWN = true, LINEAR = false;
+    int nxy, nx4;
+    float2 acc[2];
+    __device__ __forceinline__ int xy() const { return nxy; }
+    __device__ __forceinline__ void index(int jx, int jy, int zb, int (&k)[3]) const
+    {
+        k[0] = tiled_pair(jx, jy, zb, nx4);          // < 2^31 (checked at plan creation)
+        k[1] = 2 * zb + nxy - 1 - k[0];
+    }
+    template <typename TX>
+    __device__ __forceinline__ void load(const TX* __restrict__ x, long long xlen,
+                                         const int (&k)[3], float2 (&v)[V]) const
+    {
+#pragma unroll
+        for (int j = 0; j < V; j++)
+            if (FL_IN(2 * (long long)k[j] + 1, xlen)) v[j] = Store<TX>::ld2(x + 2 * (long long)k[j]);
+    }
+    __device__ __forceinline__ void add(float2 w, const int (&)[3], const float2 (&v)[V])
+    {
+#pragma unroll
+        for (int j = 0; j < V; j++) acc[j] = __ffma2_rn(w, v[j], acc[j]);
     }
 };
 
@@ -353,49 +476,43 @@ __device__ __forceinline__ void walk_quad(const TX* __restrict__ x, const ColEnt
                                           const AxisEntry* pZ, int nx, int ny, int nz,
                                           float2* acc, float2* accr, long long xlen)
 {
-    QuadBody<TX> b{x, xlen, nx * ny, nx >> 2};
-    if (__ldg(&pZ->ih) < 0.0f) seg_walk<true>(ce, pZ, nx, ny, nz / 2, b);
-    *acc = b.acc;
-    *accr = b.accr;
+    QuadForm f{nx * ny, nx >> 2, {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)}};
+    walk_form(x, xlen, ce, pZ, nx, ny, nz / 2, f);
+    *acc = f.acc[0];
+    *accr = f.acc[1];
 }
 
-// The z-mirror walk with all four quarter turns (plan flag rot4, nx == ny ==
-// n, a multiple of 4): per step it gathers the folded pairs of voxel (ix, iy)
-// and of its turns R^j (ix, iy), R (x, y) = (n-1-y, x), which the ray of view
-// v + j nv/4 at the same column and row crosses with the same segment. x is
-// the tiled folded volume. acc[j] gets the (voxel, mirror) sums of turn j.
-template <typename TX>
-struct OctBody {
-    const TX* __restrict__ x;
-    long long xlen;
+// All four quarter turns (plan flag rot4, nx == ny == n, a multiple of 4): per
+// step the folded pairs of voxel (ix, iy) and of its turns R^j (ix, iy), R (x, y)
+// = (n-1-y, x), which the ray of view v + j nv/4 at the same column and row
+// crosses with the same segment. x is the tiled folded volume. acc[j] gets the
+// (voxel, mirror) sums of turn j.
+struct OctForm {
+    static constexpr int NB = kOctBatch, V = 4;
+    static constexpr bool DOWN = true, LINEAR = false;
     int n, nn, n4;
-    float2 acc[4], xv[4];
-    __device__ __forceinline__ void load(int jx, int jy, int jz, float2 (&o)[4]) const
+    float2 acc[4];
+    __device__ __forceinline__ int xy() const { return nn; }
+    __device__ __forceinline__ void index(int jx, int jy, int zb, int (&k)[3]) const
     {
-        const int zb = jz * nn;
-        int q[4];                                    // turns 2, 3 are turns 0, 1 by pi
-        q[0] = tiled_pair(jx, jy, zb, n4);
-        q[1] = tiled_pair(n - 1 - jy, jx, zb, n4);
-        q[2] = 2 * zb + nn - 1 - q[0];
-        q[3] = 2 * zb + nn - 1 - q[1];
+        k[0] = tiled_pair(jx, jy, zb, n4);
+        k[1] = tiled_pair(n - 1 - jy, jx, zb, n4);
+        k[2] = 2 * zb + nn - 1;                      // turns 2, 3 are turns 0, 1 by pi
+    }
+    template <typename TX>
+    __device__ __forceinline__ void load(const TX* __restrict__ x, long long xlen,
+                                         const int (&k)[3], float2 (&v)[V]) const
+    {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            o[j] = make_float2(0.0f, 0.0f);
-            if (FL_IN(2 * (long long)q[j] + 1, xlen)) o[j] = Store<TX>::ld2(x + 2 * (long long)q[j]);
+        for (int j = 0; j < V; j++) {
+            const int q = j < 2 ? k[j] : k[2] - k[j - 2];
+            if (FL_IN(2 * (long long)q + 1, xlen)) v[j] = Store<TX>::ld2(x + 2 * (long long)q);
         }
     }
-    __device__ __forceinline__ void at(int jx, int jy, int jz) { load(jx, jy, jz, xv); }
-    __device__ __forceinline__ void take(float seg, bool more, int jx, int jy, int jz)
+    __device__ __forceinline__ void add(float2 w, const int (&)[3], const float2 (&v)[V])
     {
-        float2 xn[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) xn[j] = make_float2(0.0f, 0.0f);
-        if (more) load(jx, jy, jz, xn);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            acc[j] = __ffma2_rn(make_float2(seg, seg), xv[j], acc[j]);
-            xv[j] = xn[j];
-        }
+        for (int j = 0; j < V; j++) acc[j] = __ffma2_rn(w, v[j], acc[j]);
     }
 };
 
@@ -404,13 +521,13 @@ __device__ __forceinline__ void walk_oct(const TX* __restrict__ x, const ColEntr
                                          const AxisEntry* pZ, int n, int nz, float2 (&acc)[4],
                                          long long xlen)
 {
-    OctBody<TX> b;
-    b.x = x; b.xlen = xlen; b.n = n; b.nn = n * n; b.n4 = n >> 2;
+    OctForm f;
+    f.n = n; f.nn = n * n; f.n4 = n >> 2;
 #pragma unroll
-    for (int j = 0; j < 4; j++) { b.acc[j] = make_float2(0.0f, 0.0f); b.xv[j] = b.acc[j]; }
-    if (__ldg(&pZ->ih) < 0.0f) seg_walk<true>(ce, pZ, n, n, nz / 2, b);
+    for (int j = 0; j < 4; j++) f.acc[j] = make_float2(0.0f, 0.0f);
+    walk_form(x, xlen, ce, pZ, n, n, nz / 2, f);
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[j] = b.acc[j];
+    for (int j = 0; j < 4; j++) acc[j] = f.acc[j];
 }
 
 // Orbit index of voxel (x, y, z) in the folded volume of a reflection form
@@ -478,22 +595,42 @@ __device__ __forceinline__ void ld_orbit<__nv_bfloat16>(const __nv_bfloat16* __r
 // the pairs' places and exchanged when the ray crosses the middle of x or y (at
 // most once each). Every image's sum adds the same terms in the same order as
 // with one gather per image.
-template <typename TX, int NR>
-struct ReflBody {
-    const TX* __restrict__ x;
-    long long xlen;
-    int nx, ny, hx, hy, hxy;
-    int flips = 0;                           // of the current voxel (bit 0 x, bit 1 y)
-    float2 A[4], B[4], va[4], vb[4];         // sums and values of the two orbits
-    __device__ __forceinline__ void load(int jx, int jy, int jz, float2 (&a)[4],
-                                         float2 (&b)[4]) const
+template <int NR>
+struct ReflForm {
+    static constexpr int NB = NR == 4 ? kRefl4Batch : kRefl2Batch, V = NR == 4 ? 8 : 4;
+    static constexpr bool DOWN = true, LINEAR = false;
+    int nx, ny, hx, hy;
+    int flips = 0;                           // of the sums' places (bit 0 x, bit 1 y)
+    float2 A[4], B[4];                       // sums of the two orbits
+    __device__ __forceinline__ int xy() const { return hx * hy; }
+    __device__ __forceinline__ void index(int jx, int jy, int zb, int (&k)[3]) const
     {
-        const int xx = min(jx, nx - 1 - jx), yy = min(jy, ny - 1 - jy), zb = jz * hxy;
-        const int q = orbit_index(xx, yy, zb, hx);
-        if (FL_IN(8 * (long long)q + 7, xlen)) ld_orbit<TX>(x + 8 * (long long)q, a);
-        if (NR == 4) {
-            const int t = orbit_index(yy, xx, zb, hx);
-            if (FL_IN(8 * (long long)t + 7, xlen)) ld_orbit<TX>(x + 8 * (long long)t, b);
+        const int xx = min(jx, nx - 1 - jx), yy = min(jy, ny - 1 - jy);
+        k[0] = orbit_index(xx, yy, zb, hx);
+        k[1] = NR == 4 ? orbit_index(yy, xx, zb, hx) : 0;
+        k[2] = (jx >= hx ? 1 : 0) | (jy >= hy ? 2 : 0);
+    }
+    template <typename TX>
+    __device__ __forceinline__ void load(const TX* __restrict__ x, long long xlen,
+                                         const int (&k)[3], float2 (&v)[V]) const
+    {
+#pragma unroll
+        for (int o = 0; o < V / 4; o++) {
+            float2 t[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) t[j] = make_float2(0.0f, 0.0f);
+            if (FL_IN(8 * (long long)k[o] + 7, xlen)) ld_orbit<TX>(x + 8 * (long long)k[o], t);
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[4 * o + j] = t[j];
+        }
+    }
+    __device__ __forceinline__ void add(float2 w, const int (&k)[3], const float2 (&v)[V])
+    {
+        quadrant(k[2]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            A[j] = __ffma2_rn(w, v[j], A[j]);
+            if (NR == 4) B[j] = __ffma2_rn(w, v[V - 4 + j], B[j]);
         }
     }
     // the sums follow the voxel into the quadrant of flips f (bit 0 x, bit 1 y)
@@ -517,26 +654,6 @@ struct ReflBody {
         }
         flips = f;
     }
-    __device__ __forceinline__ int flips_of(int jx, int jy) const
-    {
-        return (jx >= hx ? 1 : 0) | (jy >= hy ? 2 : 0);
-    }
-    __device__ __forceinline__ void at(int jx, int jy, int jz)
-    {
-        load(jx, jy, jz, va, vb);
-        quadrant(flips_of(jx, jy));
-    }
-    __device__ __forceinline__ void take(float seg, bool more, int jx, int jy, int jz)
-    {
-        const float2 w = make_float2(seg, seg);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            A[j] = __ffma2_rn(w, va[j], A[j]);
-            if (NR == 4) B[j] = __ffma2_rn(w, vb[j], B[j]);
-        }
-        if (more) load(jx, jy, jz, va, vb);
-        if (more) quadrant(flips_of(jx, jy));
-    }
 };
 
 template <typename TX, int NR>
@@ -544,13 +661,11 @@ __device__ __forceinline__ void walk_refl(const TX* __restrict__ x, const ColEnt
                                           const AxisEntry* pZ, int nx, int ny, int nz,
                                           float2 (&acc)[2 * NR], long long xlen)
 {
-    ReflBody<TX, NR> b;
-    b.x = x; b.xlen = xlen; b.nx = nx; b.ny = ny;
-    b.hx = nx >> 1; b.hy = ny >> 1; b.hxy = b.hx * b.hy;
+    ReflForm<NR> b;
+    b.nx = nx; b.ny = ny; b.hx = nx >> 1; b.hy = ny >> 1;
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-        b.A[j] = b.B[j] = b.va[j] = b.vb[j] = make_float2(0.0f, 0.0f);
-    if (__ldg(&pZ->ih) < 0.0f) seg_walk<true>(ce, pZ, nx, ny, nz / 2, b);
+    for (int j = 0; j < 4; j++) b.A[j] = b.B[j] = make_float2(0.0f, 0.0f);
+    walk_form(x, xlen, ce, pZ, nx, ny, nz / 2, b);
     b.quadrant(0);                           // A, B by the images' own flips
     if (NR == 4) {
         acc[0] = b.A[0]; acc[2 % (2 * NR)] = b.A[3];          // I, R^2
@@ -810,10 +925,9 @@ __device__ __forceinline__ void walk_fan_parts(const TX* __restrict__ x,
                 seg[u] = __fsub_rn(nxt, cur);
                 ia[u] = a; ib[u] = b;
                 const bool gx = Ux == nxt, gy = Uy == nxt;
-                mx = __fadd_rn(mx, gx ? stx : 0.0f); Ux = xrel(X, mx, bh, cbx);
-                my = __fadd_rn(my, gy ? sty : 0.0f); Uy = xrel(Y, my, bh, cby);
-                a += (gx ? dax : 0) + (gy ? day : 0);
-                b += (gx ? dax : 0) - (gy ? day : 0);
+                if (gx) { mx = __fadd_rn(mx, stx); a += dax; b += dax; }
+                if (gy) { my = __fadd_rn(my, sty); a += day; b -= day; }
+                Ux = xrel(X, mx, bh, cbx); Uy = xrel(Y, my, bh, cby);
                 cur = nxt;
             }
             float vv[NB][NI];
@@ -1235,15 +1349,6 @@ __host__ __device__ inline int fan_turn_lanes(long long walks, int nx, int ny)
 {
     const int n = nx > ny ? nx : ny;
     return walks < kFanSplitWalks && n > 5 * (1 << kSegFan) ? kFanLanes : 4;
-}
-
-// A pointer as this thread holds it. Formed from kernel parameters and a slice's
-// or a frame's offset, the image pointers were formed anew at every gather (64
-// uneven slices: 5.42 ms, 4.31 so). Every lane of the warp must call it.
-template <typename T>
-__device__ __forceinline__ const T* held(const T* p)
-{
-    return (const T*)__shfl_sync(0xffffffffu, (unsigned long long)p, threadIdx.x & 31);
 }
 
 // One block of kFanBlock threads of the general fan forward: kFanParts threads

@@ -74,7 +74,7 @@ constexpr int kReflWarps = 4;       // 2 x 2 blocks of columns per thread block
 // turn), 0.207 ms at 64^3 / 72. Lanes along z with one column per warp: 9.34,
 // 140, 2.91, 0.102; 2 x 2 columns: 7.22, 102, 2.11, 0.203; with the views of a
 // large input in chunks and vector stores of the packed input: 6.94, 98.7, 2.08,
-// 0.100. Slower or no faster: two rows per iteration (8.9 ms at 256^3), 3 and 5
+// 0.100; the row table's pointer held (held): 6.79 at 256^3. Slower or no faster: two rows per iteration (8.9 ms at 256^3), 3 and 5
 // blocks per SM (7.5, 10.6), blocks of 8 and 16 warps (7.4), even and odd rows
 // kept apart so that the lanes' loads are dense (7.26; 108 at 512^3), the next
 // row's table entry loaded ahead (7.7), a run-time lane count for FULL (+10 %).
@@ -152,7 +152,7 @@ k_adj_refl(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
         refl_view(g, w, vt, base, alim);
         const ViewEntry ve = view[vt];
         const ColEntry* cv = col + (long long)vt * na;
-        const AxisEntry* rv = rowz + (long long)vt * nb;
+        const AxisEntry* rv = held(rowz + (long long)vt * nb, wm);
         const TW* yv = yw + base;
         // the images' detector windows, image (lane mod NI) in each lane
         int alo, ahi;
