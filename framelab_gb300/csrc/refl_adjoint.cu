@@ -74,10 +74,12 @@ constexpr int kReflWarps = 4;       // 2 x 2 blocks of columns per thread block
 // turn), 0.207 ms at 64^3 / 72. Lanes along z with one column per warp: 9.34,
 // 140, 2.91, 0.102; 2 x 2 columns: 7.22, 102, 2.11, 0.203; with the views of a
 // large input in chunks and vector stores of the packed input: 6.94, 98.7, 2.08,
-// 0.100; the row table's pointer held (held): 6.79 at 256^3. Slower or no faster: two rows per iteration (8.9 ms at 256^3), 3 and 5
-// blocks per SM (7.5, 10.6), blocks of 8 and 16 warps (7.4), even and odd rows
-// kept apart so that the lanes' loads are dense (7.26; 108 at 512^3), the next
-// row's table entry loaded ahead (7.7), a run-time lane count for FULL (+10 %).
+// 0.100; the row table's pointer held (held): 6.79 at 256^3; NR = 2 with 2 x 2
+// columns at 7 blocks per SM (4: 2.04): 1.94 at 256^3 / 90. Slower or no faster:
+// two rows per iteration (8.9 ms at 256^3), 3 and 5 blocks per SM (7.5, 10.6),
+// blocks of 8 and 16 warps (7.4), even and odd rows kept apart so that the lanes'
+// loads are dense (7.26; 108 at 512^3), the next row's table entry loaded ahead
+// (7.7), a run-time lane count for FULL (+10 %).
 // View chunks: the walked views w0 .. w1 only. A launch that is not the
 // first continues the sums it finds in X (FP32, either layout) and one that
 // is not the last leaves them there, so a sequence of launches over
@@ -89,7 +91,7 @@ constexpr int kReflWarps = 4;       // 2 x 2 blocks of columns per thread block
 // volume's half height would leave many lanes without a voxel), so a warp takes
 // 32 >> lanes blocks side by side; a constant 5 with FULL.
 template <typename TX, int PB, typename TW, int NR, bool FULL>
-__global__ void __launch_bounds__(kReflWarps * 32, PB == 2 ? 4 : 7)
+__global__ void __launch_bounds__(kReflWarps * 32, PB == 2 && NR == 4 ? 4 : 7)
 k_adj_refl(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __restrict__ col,
            const AxisEntry* __restrict__ rowz, const ViewEntry* __restrict__ view, DetGrid G,
            int nx, int ny, int nz, int na, int nb, int nv, float dz,
