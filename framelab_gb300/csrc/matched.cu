@@ -179,8 +179,9 @@ k_fwd_oct(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restri
 // 2 x 2 quads, 4.96 with the steps in batches (walk_form; 4 and 7 blocks
 // per SM -- 3, 5 or 6 fewer or more steps' registers: 5.16, 5.16, 6.6). Half
 // turn, 90 views at 256^3: 2.26, 2.18, 1.56 ms.
-template <typename TX, typename TY, int NR>
-__global__ void __launch_bounds__(128, NR == 4 ? 4 : 7)
+// NB steps a batch (the rule at the launch).
+template <typename TX, typename TY, int NR, int NB>
+__global__ void __launch_bounds__(128, NB == kRefl4Batch ? 4 : 7)
 k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restrict__ col,
            const float* __restrict__ colr, const RowEntry* __restrict__ row, int nx, int ny,
            int nz, int na, int nb, int nv, long long nper, float scale, int cr_power,
@@ -202,7 +203,7 @@ k_fwd_refl(const TX* __restrict__ X, TY* __restrict__ y, const ColEntry* __restr
     const ColEntry* ce = col + (long long)vt * na + a;
     const RowEntry* re = row + (long long)vt * nb + ib;
     float2 acc[2 * NR];
-    walk_refl<TX, NR>(X, ce, &re->z, nx, ny, nz, acc, nper);
+    walk_refl<TX, NR, NB>(X, ce, &re->z, nx, ny, nz, acc, nper);
     const float cr = ray_cr(scale, colr[(long long)vt * na + a], __ldg(&re->dz2));
     const float xs = xscale ? *xscale : 1.0f;
     float o[2][2 * NR];                 // the orbit's two planes of 2 NR values
@@ -991,12 +992,19 @@ void launch_fwd(fl_plan* p, const void* x, void* y, int cr_power, const int* ski
         const int NR = fl_plan_refl(p);
         const ReflGeom g = refl_geom(NR, s.nv, s.na, s.nb);
         dim3 grid(fl_div_up(s.na, fb.x), g.slots, fl_div_up(s.nb / 2, fb.y));
-#define FL_FWD_REFL(NR_)                                                                     \
-    k_fwd_refl<TX, TY, NR_><<<grid, fb, 0, st>>>(                                            \
+        // 16-bit volumes of the quarter turns: four steps' conversions spill, so
+        // one step a batch (256^3, 360 views, FP16 6.82 -> 4.46 ms; two 5.63) unless
+        // the blocks are fewer than fit at once, where latency counts (64^3 / 72:
+        // 45 us by four, 55 by one)
+        constexpr int many = sizeof(TX) == 2 ? 1 : kRefl4Batch;
+        const long long blocks = (long long)grid.x * grid.y * grid.z;
+#define FL_FWD_REFL(NR_, NB_)                                                                \
+    k_fwd_refl<TX, TY, NR_, NB_><<<grid, fb, 0, st>>>(                                       \
         (const TX*)x, (TY*)y, p->d_col, p->d_colr, p->d_row, s.nx, s.ny, s.nz, s.na, s.nb, s.nv, \
         p->n_vox_frame, s.scale, cr_power, skip, xscale, yfold)
-        if (NR == 4) FL_FWD_REFL(4);
-        else FL_FWD_REFL(2);
+        if (NR == 4 && blocks <= 4 * 152) FL_FWD_REFL(4, kRefl4Batch);
+        else if (NR == 4) FL_FWD_REFL(4, many);
+        else FL_FWD_REFL(2, kRefl2Batch);
 #undef FL_FWD_REFL
     } else if (s.ndim == 3 && p->zmirror && p->rot && p->rot4) {
         dim3 grid(fl_div_up(s.na, fb.x), s.nv / 4, fl_div_up(s.nb / 2, fb.y));

@@ -595,9 +595,10 @@ __device__ __forceinline__ void ld_orbit<__nv_bfloat16>(const __nv_bfloat16* __r
 // the pairs' places and exchanged when the ray crosses the middle of x or y (at
 // most once each). Every image's sum adds the same terms in the same order as
 // with one gather per image.
-template <int NR>
+template <int NR, int STEPS>
 struct ReflForm {
-    static constexpr int NB = NR == 4 ? kRefl4Batch : kRefl2Batch, V = NR == 4 ? 8 : 4;
+    static constexpr int NB = STEPS;
+    static constexpr int V = NR == 4 ? 8 : 4;
     static constexpr bool DOWN = true, LINEAR = false;
     int nx, ny, hx, hy;
     int flips = 0;                           // of the sums' places (bit 0 x, bit 1 y)
@@ -656,12 +657,12 @@ struct ReflForm {
     }
 };
 
-template <typename TX, int NR>
+template <typename TX, int NR, int NB>
 __device__ __forceinline__ void walk_refl(const TX* __restrict__ x, const ColEntry* ce,
                                           const AxisEntry* pZ, int nx, int ny, int nz,
                                           float2 (&acc)[2 * NR], long long xlen)
 {
-    ReflForm<NR> b;
+    ReflForm<NR, NB> b;
     b.nx = nx; b.ny = ny; b.hx = nx >> 1; b.hy = ny >> 1;
 #pragma unroll
     for (int j = 0; j < 4; j++) b.A[j] = b.B[j] = make_float2(0.0f, 0.0f);
