@@ -96,11 +96,11 @@ k_adj_cone(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
         const int W = 1 << lg;
         for (int v0 = 0; v0 < min(ZL, nvf - jb); v0 += ZL >> lg) {
             const int vm = g0 + v0 + (sub >> lg);
-            const int lo = __shfl_sync(gm, alo, vm), hi = __shfl_sync(gm, ahi, vm);
+            const int lo = __shfl_sync(gm, alo, vm), span = __shfl_sync(gm, ahi - alo, vm);
             const int ivm = __shfl_sync(gm, iv, vm);
             for (int j0 = 0; j0 < maxw; j0 += W) {      // once, or W = ZL and one view
-                const int ia = lo + j0 + (sub & (W - 1));
-                bool ok = ia <= hi && FL_IN(ia, na);
+                const int j = j0 + (sub & (W - 1)), ia = (int)((unsigned)lo + j);
+                bool ok = j <= span && FL_IN(ia, na);   // (lo + j can wrap; not where ok)
                 __syncwarp(gm);
                 if (ok) {
                     const ColEntry ce = col[(long long)ivm * na + ia];

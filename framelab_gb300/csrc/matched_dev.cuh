@@ -1130,7 +1130,10 @@ __device__ __forceinline__ void column_window(const DetGrid& G, float c, float s
     // fl_plan_create allows between y_det and the uniform grid
     f0 = fmaxf(ceilf(f0 - 0.02f), 0.0f);
     f1 = fminf(floorf(f1 + 0.02f), (float)(na - 1));
-    lo = (int)f0; hi = (int)f1;                   // empty when lo > hi
+    // empty when lo > hi; lo is as large as 2^31 - 1 where the shadow lies that far
+    // beside a very fine detector (hi is na - 1 then): hi - lo does not wrap, lo plus
+    // a lane's number may
+    lo = (int)f0; hi = (int)f1;
 }
 
 // Fan adjoint of a PX x PY block of pixels with lower corner (ix0, iy0): for

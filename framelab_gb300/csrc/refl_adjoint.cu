@@ -163,6 +163,7 @@ k_adj_refl(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
             refl_corner<NR, PB>(sub % NI, X0, Y0, nx, ny, bx, by);
             column_window(G, ve.c, ve.s, (float)(bx - hx), (float)(by - hy), (float)PB, (float)PB,
                           na, alo, ahi, dmin, dmax);
+            alo = min(alo, na);                         // lane numbers are added to it
             ahi = min(ahi, alim - 1);
         }
         const int maxw = __reduce_max_sync(wm, ahi - alo + 1);
