@@ -577,7 +577,9 @@ k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
             const float g = fdiv(SD, fmul(fadd(xr, SO), dy_det));
             amax = (int)floorf(fadd(fsub(fmul(fadd(yr, 1.0f), g), y_os), (float)na2));
             amin = (int)floorf(fadd(fsub(fmul(fsub(yr, 1.0f), g), y_os), (float)na2));
-            amin = max(amin, 0); amax = min(amax, na - 1);
+            // into [0, na] and [-1, na - 1]: both ends can be as large as an int holds
+            // (a very fine panel, a source inside the volume), and lanes are added
+            amin = min(max(amin, 0), na); amax = max(min(amax, na - 1), -1);
         }
         const int maxw = __reduce_max_sync(gm, amax - amin + 1);
         if (maxw <= 0) continue;

@@ -54,3 +54,19 @@ def test_reflection_backprojection(run):
     assert P.reflect and P.rotations == 4
     P.set_tuning("adj_run", run)
     _check(P, PAR.snapped(p, 4, True))
+
+
+# the source outside the volume and inside it (windows of negative width)
+@pytest.mark.parametrize("SO", [30.0, 3.0])
+def test_version_1_backprojection(SO):
+    """Bit for bit the reference's (its window's conversions to int saturate)."""
+    import torch
+    from framelab_gb300.projector import Plan
+    p = G.cone_para(12, 12, 20, 6, 14, 40, L=(12.0, 12.0, 20.0), SO=SO, OD=30.0, Ly=6 * PITCH,
+                    Lz=40.0)
+    P = Plan(p)
+    y = np.random.default_rng(6).standard_normal(P.n_rays).astype(np.float32)
+    x = P.adjoint(torch.from_numpy(y).cuda(), model="chord_ref").cpu().numpy().reshape(-1)
+    want = O.cone_adj_f32(y, p, threads=os.cpu_count() or 1)
+    assert np.any(want)
+    assert np.array_equal(x, want)
