@@ -79,8 +79,10 @@ k_adj_cone(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
             iv = views[jb + sub];
             const ViewEntry ve = view[iv];
             float dmin, dmax;
-            column_window(G, ve.c, ve.s, (float)(X0 - nx / 2), (float)(Y0 - ny / 2), (float)PB,
-                          (float)PB, na, alo, ahi, dmin, dmax);
+            // (the part of the block inside the grid: a source beside the grid's
+            // corner may stand in the rest)
+            column_window(G, ve.c, ve.s, (float)(X0 - nx / 2), (float)(Y0 - ny / 2),
+                          (float)min(PB, nx - X0), (float)min(PB, ny - Y0), na, alo, ahi, dmin, dmax);
             // rows of the group's heights at the block's depths, a row to spare
             const float za = (float)(zc - nz / 2) * dz - ve.sz;
             const float zb = (float)(min(zc + ZL, nzw) - nz / 2) * dz - ve.sz;

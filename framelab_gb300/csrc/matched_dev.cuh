@@ -1178,8 +1178,10 @@ __device__ __forceinline__ void fan_view_gather(float (&acc)[PY][PX], const floa
                                                 int ix0, int iy0, int nx, int ny, int na)
 {
     int lo, hi; float dmin, dmax;
-    column_window(G, ve.c, ve.s, (float)(ix0 - nx / 2), (float)(iy0 - ny / 2), (float)PX,
-                  (float)PY, na, lo, hi, dmin, dmax);
+    // the part of the block inside the grid (a source beside the grid's corner may
+    // stand in the rest)
+    column_window(G, ve.c, ve.s, (float)(ix0 - nx / 2), (float)(iy0 - ny / 2),
+                  (float)min(PX, nx - ix0), (float)min(PY, ny - iy0), na, lo, hi, dmin, dmax);
     const ColEntry* cv = col + (long long)iv * na;
     const float* yv = yw + (long long)iv * na;
     for (int ia = lo; ia <= hi; ia++) {
