@@ -741,7 +741,8 @@ k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
 // (c1, k1) min(rs, rz); then whichever crossing comes first, |rs - rz|; then (c2,
 // k2) 1 - max(rs, rz). These are the reference's cases 11 (the first alone), 12
 // and 21 (the first two) and 22 (all three) with their expressions: 1 - rz is rs
-// - rz at rs = 1, and a weight of 1 leaves l as it is.
+// - rz at rs = 1, and a weight of 1 leaves l as it is. A weight of 0 (a slab that
+// ends exactly on a plane) still reads its cell, which may not be finite.
 __device__ __forceinline__ float gao_slab(float acc, float p1, float p2, float q1, float q2,
                                           float l, int ns, int nz, const float* __restrict__ x,
                                           int ss, int zs, int base)
@@ -753,7 +754,7 @@ __device__ __forceinline__ float gao_slab(float acc, float p1, float p2, float q
     float rs = 1.0f, rz = 1.0f;
     if (dc) rs = fdiv(fsub((float)c2, p1), fsub(p2, p1));
     if (dk) rz = fdiv(fsub((float)k2, q1), fsub(q2, q1));
-    const bool zfirst = rs > rz;                    // the z crossing comes first
+    const bool zfirst = !dc || rs > rz;             // the z crossing comes first, or alone
     const bool t1 = c1 > -1 && k1 > -1;
     const bool t2 = (dc || dk) && (zfirst ? c1 > -1 && k2 < nz : c2 < ns && k1 > -1);
     const bool t3 = dc && dk && c2 < ns && k2 < nz;
