@@ -1484,9 +1484,11 @@ __device__ __forceinline__ void fan_turn_adjoint_block(TX* __restrict__ X,
     const int tx = threadIdx.x, g = threadIdx.y, bx = ix0 + P * tx;
     __shared__ float part[kTurnGroups][G * P * P][kFanX];
     // NG = 16: one group per thread, the second eight added to the first's
-    // sums; NG = 8: both groups of a pair in turn
+    // sums after a barrier that every row reaches; NG = 8: both groups of a pair
+    // in turn
 #pragma unroll 1
-    for (int h = g; h < kTurnViews; h += NG) {
+    for (int k = 0; k < kTurnViews / NG; k++) {
+        const int h = g + k * NG;
         float acc[G][P][P];
 #pragma unroll
         for (int m = 0; m < G; m++)
@@ -1496,19 +1498,25 @@ __device__ __forceinline__ void fan_turn_adjoint_block(TX* __restrict__ X,
                 for (int i = 0; i < P; i++) acc[m][j][i] = 0.0f;
         if (bx < hx)
             fan_turn_gather<G, P>(acc, ywp, col, view, D, bx, iy0, nx, ny, na, nv, h, kTurnViews);
-        const bool add = h >= kTurnGroups;
-        if (NG > kTurnGroups && add) __syncthreads();  // the first eight are there (uniform in a warp)
-        float(*mine)[kFanX] = part[h % kTurnGroups];
+        auto put = [&](bool add) {
+            float(*mine)[kFanX] = part[h % kTurnGroups];
 #pragma unroll
-        for (int m = 0; m < G; m++)
+            for (int m = 0; m < G; m++)
 #pragma unroll
-            for (int j = 0; j < P; j++)
+                for (int j = 0; j < P; j++)
 #pragma unroll
-                for (int i = 0; i < P; i++) {
-                    float& q = mine[(m * P + j) * P + i][tx];
-                    q = add ? q + acc[m][j][i] : acc[m][j][i];
-                }
-        if (NG > kTurnGroups && !add) __syncthreads();
+                    for (int i = 0; i < P; i++) {
+                        float& q = mine[(m * P + j) * P + i][tx];
+                        q = add ? q + acc[m][j][i] : acc[m][j][i];
+                    }
+        };
+        if (NG <= kTurnGroups) {
+            put(k > 0);
+        } else {
+            if (h < kTurnGroups) put(false);
+            __syncthreads();
+            if (h >= kTurnGroups) put(true);
+        }
     }
     __syncthreads();
     if (g != 0) return;
@@ -1827,7 +1835,8 @@ __device__ __forceinline__ void fan_refl_adjoint_block(TX* __restrict__ X,
     const int X0 = PB * bx, Y0 = PB * by;
     float(*part)[2 * NV][kFanX] = reinterpret_cast<float(*)[2 * NV][kFanX]>(smem);
 #pragma unroll 1
-    for (int h = g; h < kTurnViews; h += NG) {        // as in fan_turn_adjoint_block
+    for (int k = 0; k < kTurnViews / NG; k++) {       // as in fan_turn_adjoint_block
+        const int h = g + k * NG;
         float P[NR][PB][PB], Q[NR][PB][PB];
 #pragma unroll
         for (int j = 0; j < NR; j++)
@@ -1837,21 +1846,27 @@ __device__ __forceinline__ void fan_refl_adjoint_block(TX* __restrict__ X,
                 for (int a = 0; a < PB; a++) { P[j][b][a] = 0.0f; Q[j][b][a] = 0.0f; }
         if (prim)
             fan_refl_gather<NR, PB>(P, Q, ywp, col, view, D, X0, Y0, nx, ny, na, nv, h, kTurnViews);
-        const bool add = h >= kTurnGroups;
-        if (NG > kTurnGroups && add) __syncthreads();
-        float(*mine)[kFanX] = part[h % kTurnGroups];
+        auto put = [&](bool add) {
+            float(*mine)[kFanX] = part[h % kTurnGroups];
 #pragma unroll
-        for (int j = 0; j < NR; j++)
+            for (int j = 0; j < NR; j++)
 #pragma unroll
-            for (int b = 0; b < PB; b++)
+                for (int b = 0; b < PB; b++)
 #pragma unroll
-                for (int a = 0; a < PB; a++) {
-                    float& p = mine[(j * PB + b) * PB + a][tx];
-                    float& q = mine[NV + (j * PB + b) * PB + a][tx];
-                    p = add ? p + P[j][b][a] : P[j][b][a];
-                    q = add ? q + Q[j][b][a] : Q[j][b][a];
-                }
-        if (NG > kTurnGroups && !add) __syncthreads();
+                    for (int a = 0; a < PB; a++) {
+                        float& p = mine[(j * PB + b) * PB + a][tx];
+                        float& q = mine[NV + (j * PB + b) * PB + a][tx];
+                        p = add ? p + P[j][b][a] : P[j][b][a];
+                        q = add ? q + Q[j][b][a] : Q[j][b][a];
+                    }
+        };
+        if (NG <= kTurnGroups) {
+            put(k > 0);
+        } else {
+            if (h < kTurnGroups) put(false);
+            __syncthreads();
+            if (h >= kTurnGroups) put(true);
+        }
     }
     __syncthreads();
     if (g != 0 || !prim) return;
