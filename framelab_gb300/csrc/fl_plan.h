@@ -55,7 +55,7 @@ struct fl_plan {
     float *d_cos_det2, *d_sin_det2; // [na+1] bin-edge trig (finite-beam backprojector)
     float *d_fb_edges;             // [nv*na*6] finite-beam edge lines (Px, Py, Pd) x 2
     int32_t *d_view_frame, *d_idY, *d_Nv;
-    cudaMemPool_t pool;            // cone: stream-ordered scratch of single calls (kept, freed with the plan)
+    cudaMemPool_t pool;            // stream-ordered scratch of single calls (fl_plan_scratch; null until one asks)
     float zdet_min, zdet_max;      // smallest non-zero and largest |z_det| (cone)
     // matched-model tables (device); rows nv and nv + 1 (two extra views) hold
     // view nv/8 at the exact angle pi/4 and view nv/4 at the exact angle pi/2
@@ -265,6 +265,12 @@ bool fl_tma_available();
 // plan's forwards gave up its bounded wait since the last check; reads the
 // flag after synchronising the stream. FL_OK for plans without the flag.
 int fl_plan_take_timeouts(fl_plan* p, cudaStream_t s);
+
+// `bytes` of device memory for one call, in stream order (the caller frees it with
+// cudaFreeAsync on st): calls on several streams get memory of their own. Null
+// where there is none: while st is captured (a captured call then holds no memory
+// of its graph's), or when it cannot be had.
+void* fl_plan_scratch(fl_plan* p, size_t bytes, cudaStream_t st);
 
 // internal launchers
 int fl_ref_forward(fl_plan* p, const float* x, float* y, cudaStream_t st);

@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -104,21 +105,47 @@ static void free_plan_arrays(fl_plan* p)
     if (p->pool) cudaMemPoolDestroy(p->pool);
 }
 
-// A memory pool of the current device that keeps what it was given until it is
-// destroyed: concurrent calls get memory of their own, a call after another on
-// one stream the same memory again.
-static int make_pool(cudaMemPool_t* pool)
+// What an idle pool keeps over a synchronisation; more goes back to the device.
+// Version-1 backprojection of 164 MB (128^3, 200 views of 512 x 400), synchronised after
+// each call: 27.3 ms, 27.0 with everything kept; of 15 MB 4.58 both ways.
+static constexpr uint64_t kPoolKeep = 64ull << 20;
+
+// The plan's memory pool on the current device, made by the first call that wants
+// one (null: it cannot be had).
+static cudaMemPool_t plan_pool(fl_plan* p)
 {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (p->pool) return p->pool;
+    // another thread may be capturing a stream in the global mode
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
     cudaMemPoolProps pr;
     std::memset(&pr, 0, sizeof pr);
     pr.allocType = cudaMemAllocationTypePinned;
     pr.location.type = cudaMemLocationTypeDevice;
-    int st = fl_check_cuda(cudaGetDevice(&pr.location.id), "cudaGetDevice");
-    if (!st) st = fl_check_cuda(cudaMemPoolCreate(pool, &pr), "cudaMemPoolCreate");
-    uint64_t keep = ~0ull;
-    if (!st) st = fl_check_cuda(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep),
-                                "cudaMemPoolSetAttribute");
-    return st;
+    uint64_t keep = kPoolKeep;
+    cudaMemPool_t pool = nullptr;
+    if (cudaGetDevice(&pr.location.id) == cudaSuccess && cudaMemPoolCreate(&pool, &pr) == cudaSuccess) {
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+            p->pool = pool;
+        else
+            cudaMemPoolDestroy(pool);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return p->pool;
+}
+
+void* fl_plan_scratch(fl_plan* p, size_t bytes, cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    void* w = nullptr;
+    const bool plain = cudaStreamIsCapturing(st, &cap) == cudaSuccess;
+    if (plain && cap != cudaStreamCaptureStatusNone) return nullptr;
+    cudaMemPool_t pool = plain ? plan_pool(p) : nullptr;
+    if (pool && fl_malloc_async(&w, bytes, pool, st) == cudaSuccess) return w;
+    cudaGetLastError();                          // the caller does without
+    return nullptr;
 }
 
 // Nudge a direction component away from zero so 1/d stays finite; the ray
@@ -635,7 +662,6 @@ extern "C" int fl_plan_create(const fl_scan* scan, fl_plan** out)
     if (!st) st = upload(&p->d_idY, idY.data(), idY.size());
     if (!st) st = upload(&p->d_Nv, Nvv.data(), nt);
     if (!st && s.ndim == 3) {
-        st = make_pool(&p->pool);
         p->zdet_min = 3.0e38f;
         for (int ib = 0; ib < nb; ib++) {
             const float z = std::fabs(s.z_det[ib]);

@@ -478,13 +478,19 @@ k_ref_fan_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
     x[(long long)it * nx * ny + (long long)iy * nx + ix] = fmul(acc, scale);
 }
 
-// Rows-fastest copy of a cone sinogram for the backprojection below: yt[(iv na +
-// ia) nb + ib] = y[(iv nb + ib) na + ia], 32 x 32 tiles through shared memory;
-// *bad is set when a value is not finite.
+// Prepares a cone sinogram for the backprojection below: whether every value is
+// finite (flag[0 .. nflag), all 0 before, becomes 1 when one is not), and with RF the
+// rows-fastest copy yt[(iv na + ia) nb + ib] = y[(iv nb + ib) na + ia], 32 x 32 tiles
+// through shared memory. Without scratch the flag is the backprojection's own
+// output, every voxel of it, read by its voxel's lane before it is written. Blocks
+// that find such a value write the same flags; one that sees that another has begun
+// leaves it to that one.
+template <bool RF, typename F>
 __global__ void __launch_bounds__(256)
-k_ref_rows_fastest(const float* __restrict__ y, float* __restrict__ yt, int* bad, int na, int nb)
+k_ref_prepare(const float* __restrict__ y, float* __restrict__ yt, int na, int nb, F* flag,
+              long long nflag)
 {
-    __shared__ float tile[32][33];
+    __shared__ float tile[RF ? 32 : 1][33];
     const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
     const long long base = (long long)blockIdx.z * na * nb;
     bool fin = true;
@@ -492,14 +498,17 @@ k_ref_rows_fastest(const float* __restrict__ y, float* __restrict__ yt, int* bad
         const int ia = a0 + threadIdx.x, ib = b0 + k;
         if (ia >= na || ib >= nb) continue;
         const float v = y[base + (long long)ib * na + ia];
-        tile[k][threadIdx.x] = v;
+        if (RF) tile[k][threadIdx.x] = v;
         fin = fin && isfinite(v);
     }
-    if (!__syncthreads_and(fin) && threadIdx.x == 0 && threadIdx.y == 0) *bad = 1;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int ia = a0 + k, ib = b0 + threadIdx.x;
-        if (ia < na && ib < nb) yt[base + (long long)ia * nb + ib] = tile[threadIdx.x][k];
-    }
+    const bool all = __syncthreads_and(fin);
+    if (RF)
+        for (int k = threadIdx.y; k < 32; k += 8) {
+            const int ia = a0 + k, ib = b0 + threadIdx.x;
+            if (ia < na && ib < nb) yt[base + (long long)ia * nb + ib] = tile[threadIdx.x][k];
+        }
+    if (all || __syncthreads_or(*(volatile F*)flag != F(0))) return;    // (all or none of the block)
+    for (long long k = threadIdx.y * 32 + threadIdx.x; k < nflag; k += 256) flag[k] = F(1);
 }
 
 constexpr int kChordWarps = 4;     // neighbouring voxel columns per thread block
@@ -515,7 +524,7 @@ constexpr int kChordWarps = 4;     // neighbouring voxel columns per thread bloc
 // Rays that miss the voxel are not evaluated. The reference's window is about
 // 5 x 6 rays per voxel and view at a magnification of two, of which about 5
 // meet it; the others get l = 0 from find_l_3d and add an exact zero (unless a
-// value is not finite: *bad turns the skipping off). A line that misses the
+// value is not finite: k_ref_prepare turns the skipping off). A line that misses the
 // voxel's box grown by a margin m on every side passes none of the reference's
 // face tests: a test computes u = s (h - r) + r' for a slope s of the direction
 // (a, b, c) and offsets r, r' of the source, with an error of at most 2^-22
@@ -529,8 +538,8 @@ constexpr int kChordWarps = 4;     // neighbouring voxel columns per thread bloc
 //   in z:  every point of the line inside the grown square lies within 0.88 of
 //          the one nearest its centre, at t0: |rz + c t0| > 1/2 + m + |c| k,
 //          k = 0.88 / |(a, b)|.
-// zmin, zmax: the smallest non-zero and the largest |z_det|. Y has its rows
-// fastest.
+// zmin, zmax: the smallest non-zero and the largest |z_det|. RF: Y has its
+// rows fastest and *bad is the flag, else its columns (k_ref_prepare).
 // Bound: issue (82-85 %; 871 warp instructions per column of 32 voxels and
 // view). 128^3, 120 views, 192 x 160 panel: 27.6 ms with a thread per voxel,
 // the window's columns set up by each and every ray of it evaluated; 14.2 with
@@ -538,6 +547,7 @@ constexpr int kChordWarps = 4;     // neighbouring voxel columns per thread bloc
 // and no division for faces that fail in the plane; 8.30 with chord_two; 6.43
 // with the margin of 0.02 and without the per-ray test where chord_two applies.
 // 6 and 10 blocks per SM 6.68 and 6.61. 200^3, 40 views, 400 x 300: 51.8 -> 10.6.
+template <bool RF>
 __global__ void __launch_bounds__(kChordWarps * 32, 8)
 k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
                      const int* __restrict__ bad, const float* __restrict__ cos_phi,
@@ -557,7 +567,9 @@ k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
     const int iz = ((int)(blockIdx.z % zruns) << lz) + sub, it = blockIdx.z / zruns;
     if (ix >= nx) return;                               // whole groups
     const bool on = iz < nz;
-    const bool skip = !*bad;
+    const bool skip = RF ? !*bad
+                         : x[(long long)it * nx * ny * nz + ((long long)min(iz, nz - 1) * ny + iy) * nx + ix] == 0.0f;
+    if (!RF) __syncwarp(gm);                            // read before any lane stores its sum
     const float SD = fadd(SO, OD);
     const int na2 = na / 2, nb2 = nb / 2, nx2 = nx / 2, ny2 = ny / 2, nz2 = nz / 2;
     const long long nd = (long long)na * nb;
@@ -697,7 +709,7 @@ k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
                 for (int ib = bmin; ib <= bmax; ib++) {
                     const float z2 = fadd(__ldg(zdet + ib), z1);
                     const float cz = fsub(z2, z1);
-                    const float* yb = yv + ib;
+                    const float* yb = yv + (RF ? (long long)ib : (long long)ib * na);
                     if (wide > W) {                     // more columns than lanes: one by one
                         const float cOD = fmul(c, OD), sOD = fmul(s, OD);
                         for (int ia2 = ak; ia2 < ak + wide; ia2++) {
@@ -705,7 +717,7 @@ k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
                             const float l = chord_box(x1, y1, z1, fsub(cOD, fmul(s, u)),
                                                       fadd(sOD, fmul(c, u)), z2, 1.0f, 1.0f, 1.0f,
                                                       xc, yc, zc);
-                            acc = fadd(acc, fmul(l, __ldg(yb + (long long)ia2 * nb)));
+                            acc = fadd(acc, fmul(l, __ldg(yb + (RF ? (long long)ia2 * nb : (long long)ia2))));
                         }
                         continue;
                     }
@@ -720,7 +732,7 @@ k_ref_cone_chord_adj(float* __restrict__ x, const float* __restrict__ Y,
                             : (q.flags & kAxis)
                                 ? chord_box(x1, y1, z1, q.x2, q.y2, z2, 1.0f, 1.0f, 1.0f, xc, yc, zc)
                                 : chord_box_col(q, cz, rx, ry, rz);
-                        acc = fadd(acc, fmul(l, __ldg(yb + (long long)q.ia * nb)));
+                        acc = fadd(acc, fmul(l, __ldg(yb + (RF ? (long long)q.ia * nb : (long long)q.ia))));
                     }
                 }
             }
@@ -1081,15 +1093,19 @@ int fl_ref_adjoint(fl_plan* p, const float* y, float* x, cudaStream_t st)
     } else {
         if ((long long)s.nz * s.nt > 65535)
             return fl_set_error(FL_ERR_UNSUPPORTED, "reference backprojector: nz * nt > 65535");
-        // scratch of this call, in stream order: the non-finite flag and the
-        // rows-fastest copy of y (a warp's lanes read neighbouring rows)
-        void* w = nullptr;
-        FL_CUDA(fl_malloc_async(&w, 256 + (size_t)p->n_rays * sizeof(float), p->pool, st));
+        // scratch of this call: the flag and a rows-fastest copy of y (a warp's lanes
+        // then read neighbouring rows). Without it (fl_plan_scratch) they read y as it
+        // is, for the same bits (128^3, 120 views, 192 x 160 panel, source at four half
+        // widths: 4.58 ms and 4.95 without; 200 views, 512 x 400: 27.3 and 32.6)
+        void* w = fl_plan_scratch(p, 256 + (size_t)p->n_rays * sizeof(float), st);
         int* bad = (int*)w;
-        float* yt = (float*)((char*)w + 256);
-        int e = fl_check_cuda(cudaMemsetAsync(bad, 0, sizeof(int), st), "cudaMemsetAsync");
-        const dim3 tg(fl_div_up(s.na, 32), fl_div_up(s.nb, 32), s.nv);
-        if (!e) k_ref_rows_fastest<<<tg, dim3(32, 8), 0, st>>>(y, yt, bad, s.na, s.nb);
+        float* yt = w ? (float*)((char*)w + 256) : nullptr;
+        int e = fl_check_cuda(w ? cudaMemsetAsync(bad, 0, sizeof(int), st)
+                                : cudaMemsetAsync(x, 0, (size_t)p->n_vox * sizeof(float), st),
+                              "cudaMemsetAsync");
+        const dim3 tg(fl_div_up(s.na, 32), fl_div_up(s.nb, 32), s.nv), tb(32, 8);
+        if (w) k_ref_prepare<true><<<tg, tb, 0, st>>>(y, yt, s.na, s.nb, bad, 1);
+        else k_ref_prepare<false><<<tg, tb, 0, st>>>(y, yt, s.na, s.nb, x, p->n_vox);
         // 16 or 8 lanes per voxel column where that leaves at least a quarter
         // fewer lanes without a voxel
         int lz = 5;
@@ -1097,14 +1113,15 @@ int fl_ref_adjoint(fl_plan* p, const float* y, float* x, cudaStream_t st)
         while (lz > 3 && 4 * lanes(lz - 1) <= 3 * lanes(lz)) lz--;
         const int zruns = fl_div_up(s.nz, 1 << lz);
         const dim3 grid(fl_div_up(s.nx, kChordWarps << (5 - lz)), s.ny, zruns * s.nt);
+        auto* k = w ? k_ref_cone_chord_adj<true> : k_ref_cone_chord_adj<false>;
         if (!e)
-            k_ref_cone_chord_adj<<<grid, kChordWarps * 32, 0, st>>>(
-                x, yt, bad, p->d_cos_phi, p->d_sin_phi, p->d_sd_z, p->d_y_det, p->d_z_det, p->d_idY,
+            k<<<grid, kChordWarps * 32, 0, st>>>(
+                x, w ? yt : y, bad, p->d_cos_phi, p->d_sin_phi, p->d_sd_z, p->d_y_det, p->d_z_det, p->d_idY,
                 p->d_Nv, p->tmp_size, s.SO, s.OD, s.scale, s.dy_det, s.y_os, s.dz_det, s.dz, s.nx,
                 s.ny, s.nz, s.na, s.nb, p->zdet_min, p->zdet_max, p->det_kind != -2, p->v0,
                 1.0f / p->dv, zruns, lz);
         if (!e) e = fl_check_launch("reference chord backprojection");
-        const int f = fl_check_cuda(cudaFreeAsync(w, st), "cudaFreeAsync");
+        const int f = w ? fl_check_cuda(cudaFreeAsync(w, st), "cudaFreeAsync") : FL_OK;
         return e ? e : f;
     }
     return fl_check_launch("reference chord backprojection");
