@@ -1377,9 +1377,11 @@ int fl_matched_adjoint_wt(fl_plan* p, const void* yw, int wt, void* x, int xt, c
 // below is timed (CUDA events, one launch after one untimed) on the plan's own
 // geometry, with the plan's scratch as input and output, and the fastest kept
 // for the forward and for the backprojection.
-// * Cone plans: the 128-thread block shapes of both kernels, for the reflection
-//   backprojection warps of one or 2 x 2 columns and its view chunks instead. A
-//   voxel's sum does not depend on these, so neither do the projections.
+// * Cone plans: the 128-thread block shapes of the forward and of the turns'
+//   backprojections, for the reflection backprojection warps of one or 2 x 2
+//   columns and its view chunks instead (the general and z-mirror ones have
+//   nothing to choose). A voxel's sum does not depend on these, so neither do the
+//   projections.
 // * Fan plans: the parts per walked ray of the turn forward (1, 4, 16: the
 //   order of a ray's additions, within FP32 rounding) and the pixel block of
 //   the backprojections (1 or 2: the same bits).
@@ -1423,29 +1425,28 @@ extern "C" int fl_plan_autotune(fl_plan* p, void* stream, int32_t* shapes)
     };
     if (cone) {
         static const int cand[4][2] = {{8, 16}, {16, 8}, {32, 4}, {4, 32}};
-        // the reflection backprojection has no block shape; it tries warps of
-        // 2 x 2 columns and of one (FL_TUNE_ADJ_RUN)
-        const bool refl = fl_plan_refl(p) != 0;
+        // block shapes: of the forwards, and of the turns' backprojections. The
+        // reflection backprojection tries warps of 2 x 2 columns and of one
+        // (FL_TUNE_ADJ_RUN); the general and z-mirror ones have nothing to try.
+        const int form = fl_plan_form(p);
+        const bool refl = fl_plan_refl(p) != 0, turns = form == FL_FORM_HALF || form == FL_FORM_QUARTER;
         for (int pass = 0; pass < 2 && !st; pass++) {
             const bool fwd = pass == 0;
+            if (!fwd && !turns && !refl) break;
             float best = 3.0e38f;
-            int bi = 0, br = 0;
-            for (int c = 0; c < (!fwd && refl ? 1 : 4) && !st; c++)
-                for (int r = !fwd && refl ? 1 : 0; r < (!fwd && refl ? 3 : 1) && !st; r++) {
-                    if (fwd) { p->fwd_bx = cand[c][0]; p->fwd_by = cand[c][1]; }
-                    else {
-                        p->adj_bx = cand[c][0]; p->adj_by = cand[c][1];
-                        p->adj_run = r;
-                    }
-                    float ms = 0.0f;
-                    st = timed(fwd, ms);
-                    if (!st && ms < best) { best = ms; bi = c; br = r; }
-                }
-            if (fwd) { p->fwd_bx = cand[bi][0]; p->fwd_by = cand[bi][1]; }
-            else {
-                p->adj_bx = cand[bi][0]; p->adj_by = cand[bi][1];
-                p->adj_run = br;
+            int bi = 0;
+            auto set = [&](int c) {
+                if (fwd) { p->fwd_bx = cand[c][0]; p->fwd_by = cand[c][1]; }
+                else if (refl) p->adj_run = c + 1;
+                else { p->adj_bx = cand[c][0]; p->adj_by = cand[c][1]; }
+            };
+            for (int c = 0; c < (!fwd && refl ? 2 : 4) && !st; c++) {
+                set(c);
+                float ms = 0.0f;
+                st = timed(fwd, ms);
+                if (!st && ms < best) { best = ms; bi = c; }
             }
+            set(bi);
         }
         // then the view chunks of the reflection backprojection (FP32 output)
         if (!st && fl_plan_refl(p) && p->zmirror) {
@@ -1491,7 +1492,8 @@ extern "C" int fl_plan_autotune(fl_plan* p, void* stream, int32_t* shapes)
     if (shapes) {
         if (cone) {
             shapes[0] = p->fwd_bx; shapes[1] = p->fwd_by;
-            shapes[2] = p->adj_bx; shapes[3] = p->adj_by;
+            shapes[2] = p->adj_bx ? p->adj_bx : 8;    // (8 x 16 where nothing has a shape)
+            shapes[3] = p->adj_bx ? p->adj_by : 16;
         } else {
             shapes[0] = fl_plan_fan_lanes(p); shapes[1] = 0;
             shapes[2] = fl_plan_fan_block(p); shapes[3] = fl_plan_fan_groups(p);

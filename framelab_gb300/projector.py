@@ -237,8 +237,10 @@ class Plan:
     def autotune(self, stream=None) -> dict:
         """Times the launch variants of this plan's matched projector kernels
         on its own geometry and keeps the fastest (``fl_plan_autotune``).
-        Cone plans: the block shapes (and, on a reflection plan, the columns
-        per side of a backprojection warp's block and its view chunks); the
+        Cone plans: the block shapes of the forward and of the turns'
+        backprojections; on a reflection plan the backprojection's columns per
+        side of a warp's block (reported as ``adjoint_voxels_per_thread``) and its
+        view chunks instead (``adjoint_rows_per_iteration`` selects nothing). The
         projections do not change. Fan plans: the parts per walked ray of the turn forward
         (the order of a ray's additions) and the backprojection's pixel block
         (the same bits). Plans without a matched backprojection report

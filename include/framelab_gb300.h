@@ -234,17 +234,18 @@ int fl_plan_query(const fl_plan *plan, int option, int *value);
 /* Launch-shape autotuner for a plan's matched projector kernels: times each
  * candidate on the plan's own geometry, one launch each on `stream` after one
  * untimed, and keeps the fastest for the forward and for the backprojection.
- * Cone plans: the 128-thread block shapes (8x16, 16x8, 32x4, 4x32) of both
- * kernels (on reflection plans the backprojection's FL_TUNE_ADJ_RUN and
- * FL_TUNE_ADJ_CHUNKS instead). Fan plans: the parts per walked ray of the
- * turn and reflection forwards (FL_TUNE_FAN_PARTS: 1, 4, 16), the pixel block
- * of the backprojections (FL_TUNE_FAN_BLOCK: 1 or 2) and the view groups of
- * the turn and reflection backprojections (FL_TUNE_FAN_GROUPS: 8 or 16). Only
- * the fan parts change any bit of a result (the order of a ray's additions, not
- * the matrix). Synchronises `stream`; uses the
- * plan's scratch buffers. shapes (optional, [4]): the chosen forward x, y and
- * backprojection x, y of a cone plan; for a fan plan the parts count, 0, the
- * pixel block and the view groups. */
+ * Cone plans: the 128-thread block shapes (8x16, 16x8, 32x4, 4x32) of the
+ * forward and of the half- and quarter-turn backprojections (on reflection plans
+ * the backprojection's FL_TUNE_ADJ_RUN and FL_TUNE_ADJ_CHUNKS instead; general
+ * and z-mirror backprojections have nothing to choose and report 8x16). Fan
+ * plans: the parts per walked ray of the turn and reflection forwards
+ * (FL_TUNE_FAN_PARTS: 1, 4, 16), the pixel block of the backprojections
+ * (FL_TUNE_FAN_BLOCK: 1 or 2) and the view groups of the turn and reflection
+ * backprojections (FL_TUNE_FAN_GROUPS: 8 or 16). Only the fan parts change any
+ * bit of a result (the order of a ray's additions, not the matrix). Synchronises
+ * `stream`; uses the plan's scratch buffers. shapes (optional, [4]): the chosen
+ * forward x, y and backprojection x, y of a cone plan; for a fan plan the parts
+ * count, 0, the pixel block and the view groups. */
 int fl_plan_autotune(fl_plan *plan, void *stream, int32_t *shapes);
 /* FL_TUNE_ADJ_RUN: columns per side of the block of voxel columns a warp of the
  * reflection backprojection owns (1 or 2; by default 2 once such warps fill the
