@@ -209,19 +209,13 @@ void launch(fl_plan* p, const void* yw, void* x, const int* skip, int xfold, cud
     const fl_scan& s = p->s;
     const int nzw = MIRROR ? s.nz / 2 : s.nz;
     // as for the reflection form (refl_adjoint.cu): 2 x 2 columns per warp once
-    // such warps fill the GPU; 16 or 8 lanes per block where that leaves at
-    // least a quarter fewer lanes without a voxel and still fills it
+    // such warps fill the GPU
     auto warps = [&](int pb, int lz) {
         return ((long long)fl_div_up(s.nx, pb) * fl_div_up(s.ny, pb) * fl_div_up(nzw, 1 << lz) * s.nt) >>
                (5 - lz);
     };
-    auto lanes_log2 = [&](int pb) {
-        auto lanes = [&](int lz) { return fl_div_up(nzw, 1 << lz) << lz; };
-        int lz = 5;
-        while (lz > 3 && 4 * lanes(lz - 1) <= 3 * lanes(lz) && warps(pb, lz - 1) >= 10 * 152) lz--;
-        return lz;
-    };
-    const int PB = warps(2, lanes_log2(2)) >= 10 * 152 ? 2 : 1, lz = lanes_log2(PB);
+    auto lanes_log2 = [&](int pb) { return adj_lanes_log2(p, nzw, [&](int lz) { return warps(pb, lz); }); };
+    const int PB = warps(2, lanes_log2(2)) >= adj_full_warps(p) ? 2 : 1, lz = lanes_log2(PB);
     const int zruns = fl_div_up(nzw, 1 << lz);
     const dim3 grid(fl_div_up(s.nx, (2 * PB) << (5 - lz)), fl_div_up(s.ny, 2 * PB), zruns * s.nt);
     auto* k = PB == 2 ? (lz == 5 ? k_adj_cone<TX, 2, TW, MIRROR, true> : k_adj_cone<TX, 2, TW, MIRROR, false>)

@@ -57,6 +57,7 @@ struct fl_plan {
     int32_t *d_view_frame, *d_idY, *d_Nv;
     cudaMemPool_t pool;            // stream-ordered scratch of single calls (fl_plan_scratch; null until one asks)
     float zdet_min, zdet_max;      // smallest non-zero and largest |z_det| (cone)
+    int sms;                       // multiprocessors of the device (launch rules)
     // matched-model tables (device); rows nv and nv + 1 (two extra views) hold
     // view nv/8 at the exact angle pi/4 and view nv/4 at the exact angle pi/2
     // for the reflection forms

@@ -644,6 +644,10 @@ extern "C" int fl_plan_create(const fl_scan* scan, fl_plan** out)
     for (int j = 0; j < Nvv[0] && p->views_natural; j++)
         if (idY[j] != j) p->views_natural = 0;
 
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || p->sms < 1)
+        p->sms = 152;
     int st = FL_OK;
     if (!st) st = upload(&p->d_sd_phi, phi.data(), nv);
     if (!st) st = upload(&p->d_sd_z, sdz.data(), nv);

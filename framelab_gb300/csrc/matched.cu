@@ -1002,7 +1002,7 @@ void launch_fwd(fl_plan* p, const void* x, void* y, int cr_power, const int* ski
     k_fwd_refl<TX, TY, NR_, NB_><<<grid, fb, 0, st>>>(                                       \
         (const TX*)x, (TY*)y, p->d_col, p->d_colr, p->d_row, s.nx, s.ny, s.nz, s.na, s.nb, s.nv, \
         p->n_vox_frame, s.scale, cr_power, skip, xscale, yfold)
-        if (NR == 4 && blocks <= 4 * 152) FL_FWD_REFL(4, kRefl4Batch);
+        if (NR == 4 && blocks <= 4LL * p->sms) FL_FWD_REFL(4, kRefl4Batch);
         else if (NR == 4) FL_FWD_REFL(4, many);
         else FL_FWD_REFL(2, kRefl2Batch);
 #undef FL_FWD_REFL

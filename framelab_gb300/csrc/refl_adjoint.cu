@@ -336,21 +336,9 @@ long long warp_count(const fl_plan* p, int PB, int lz)
     return (blocks * fl_div_up(s.nz / 2, 1 << lz)) >> (5 - lz);
 }
 
-// Enough of them to fill the GPU: ten per SM.
-constexpr long long kFullWarps = 10 * 152;
-
-// log2 of the lanes per block of columns: 32 lanes, or 16 or 8 where that
-// leaves at least a quarter fewer of them without a voxel and still fills the
-// GPU (512 x 512 x 32, 90 views: 1.94 ms with 32 lanes, 1.18 with 16; 64 x 64 x
-// 16, 360 views: 0.53 with 32, 0.69 with 8).
 int lanes_log2(const fl_plan* p, int PB)
 {
-    const int nzw = p->s.nz / 2;
-    auto lanes = [&](int lz) { return fl_div_up(nzw, 1 << lz) << lz; };
-    int lz = 5;
-    while (lz > 3 && 4 * lanes(lz - 1) <= 3 * lanes(lz) && warp_count(p, PB, lz - 1) >= kFullWarps)
-        lz--;
-    return lz;
+    return adj_lanes_log2(p, p->s.nz / 2, [&](int lz) { return warp_count(p, PB, lz); });
 }
 
 template <typename TX, typename TW>
@@ -391,7 +379,7 @@ void launch(fl_plan* p, const void* yw, void* x, const int* skip, int xfold, cud
 int fl_plan_adj_run(const fl_plan* p)
 {
     if (p->adj_run) return p->adj_run;
-    return warp_count(p, 2, lanes_log2(p, 2)) >= kFullWarps ? 2 : 1;
+    return warp_count(p, 2, lanes_log2(p, 2)) >= adj_full_warps(p) ? 2 : 1;
 }
 
 void fl_matched_adjoint_refl(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
