@@ -213,7 +213,7 @@ struct Pass {
 // block. Every value is the same fmaf chain as in the separable pass kernels
 // above (taps in order, filters in order), so both forms give identical bits.
 constexpr int kSX = 32, kSY = 8, kST = kSX * kSY;   // column tile, threads per block
-constexpr int kRowMax = 512, kRowTile = 256;         // k_syn_zx: longest whole row; columns of a part
+constexpr int kRowMax = 512;                         // k_syn_zx: longest whole row
 constexpr int kMaxStreamStep = 8;                    // dilations the streaming kernels take
 
 // element of a plane: a base that all threads share and a 32-bit byte offset,
@@ -233,6 +233,11 @@ __host__ __device__ inline int class_len(int nz, int s, int r)
 // resident blocks of k_ana_stream per SM: three, and two where 27 values of v
 // are held as well as the window
 __host__ __device__ constexpr int ana_resident(int nf, int mode) { return nf == 3 && mode == 1 ? 2 : 3; }
+
+// resident threads of k_syn_zx per SM. Four bands a thread (Haar) leave too few loads
+// in flight with two blocks of 512: 200^3, one level 114 us with 1024 threads, 98
+// with 1536 (a slice more ahead 107, two 101); 256^3 193 and 170.
+__host__ __device__ constexpr int syn_threads(int nf) { return nf == 2 ? 1536 : 1024; }
 
 // One analysis level: the y and x passes of each slice in shared memory, the
 // z pass from the register window, fused with the coefficient write (MODE 0)
@@ -360,7 +365,7 @@ k_ana_stream(const float* __restrict__ in, int nx, int ny, int nz, int nseg, int
 // arrays, then along x into the NF arrays A_i), band 0 taken from `low` when
 // non-null. Threads along x hold aligned runs of columns: a whole row where it
 // fits in kRowMax threads (`whole`, several rows a block when it is short),
-// else kRowTile columns and one warp more for the columns beside them. The x
+// else a tile of them and one warp more for the columns beside it. The x
 // taps come from shared memory. blockIdx.z = seg + nseg (i + NF r).
 // The 27 bands' reads bound it; issue slots came next. Warps of 32 - 2S outputs
 // whose taps came by shuffles read rows from unaligned columns, and moving the
@@ -368,13 +373,13 @@ k_ana_stream(const float* __restrict__ in, int nx, int ny, int nz, int nseg, int
 // slice: 256^3, two levels, with the y merge 916 -> 759 us. Copies into a ring in
 // shared memory, four slices deep, were slower (968 us).
 template <int NF, int S>
-__global__ void __launch_bounds__(kRowMax, 2)
+__global__ void __launch_bounds__(kRowMax, syn_threads(NF) / kRowMax)
 k_syn_zx(BandPtrs bands, const float* __restrict__ low, float* __restrict__ A, long long N,
          int nx, int ny, int nz, int nseg, int seg_len, int whole, Filters R)
 {
     constexpr int NB = NF * NF;                        // bands per thread
     extern __shared__ float s_bm[];                    // [2][NF][rows][blockDim.x]
-    const int W = blockDim.x, rows = blockDim.y, tx = threadIdx.x;
+    const int W = blockDim.x, rows = blockDim.y, tx = threadIdx.x, T = W - 32;
     const int y = blockIdx.y * rows + threadIdx.y;
     const int seg = blockIdx.z % nseg, ir = blockIdx.z / nseg, i = ir % NF, r = ir / NF;
     const int nfirst = seg * seg_len, nend = min(nfirst + seg_len, class_len(nz, S, r));
@@ -389,11 +394,11 @@ k_syn_zx(BandPtrs bands, const float* __restrict__ low, float* __restrict__ A, l
         out_ok = out_ok && tx < nx;
     } else {
         // the last warp holds the S columns before the tile, then the S after it
-        const int x0 = blockIdx.x * kRowTile, h = tx - kRowTile;
-        const int off = h < 0 ? tx : h < S ? h - S : min(h - S, S - 1) + kRowTile;
+        const int x0 = blockIdx.x * T, h = tx - T;
+        const int off = h < 0 ? tx : h < S ? h - S : min(h - S, S - 1) + T;
         x = wrapi(x0 + off, nx);
-        left = h < 0 ? (tx < S ? kRowTile + tx : tx - S) : tx;
-        right = h < 0 ? (tx + S < kRowTile ? tx + S : tx + S + S) : tx;
+        left = h < 0 ? (tx < S ? T + tx : tx - S) : tx;
+        right = h < 0 ? (tx + S < T ? tx + S : tx + S + S) : tx;
         out_ok = out_ok && h < 0 && x0 + off < nx;
     }
     const long long plane = (long long)ny * nx;
@@ -715,6 +720,20 @@ static int stream_seg_len(const fl_framelet* w, int step, long long columns, int
     return best;
 }
 
+// Columns of a tile of k_syn_zx for rows longer than kRowMax: the width whose tiles
+// take the least of an SM's resident threads per row (256 left 28 % of its columns
+// outside rows of 600: linear bank, 600 x 40 x 300, one level 223 us, 194 with 224;
+// rows of 520 82 us, 70 with 192; of 768 the same 3 x 256).
+static int syn_tile(int nx, int threads)
+{
+    int best = 0, bp = 0, bb = 1;
+    for (int t = 256; t >= 96; t -= 32) {
+        const int parts = fl_div_up(nx, t), blocks = threads / (t + 32);
+        if (!best || (long long)parts * bb < (long long)bp * blocks) { best = t; bp = parts; bb = blocks; }
+    }
+    return best;
+}
+
 template <int NF, int S>
 static void ana_stream(fl_framelet* w, const float* in, const BandPtrs& cb, const BandPtrs& tb,
                        float* low_out, int last, int mode, float tau, cudaStream_t s)
@@ -736,10 +755,11 @@ static void syn_stream(fl_framelet* w, const BandPtrs& cb, const float* low, flo
     const long long N = w->N;
     float* A = w->work;                                // NF arrays
     const int whole = w->nx <= kRowMax;
-    const int W = whole ? 32 * fl_div_up(w->nx, 32) : kRowTile + 32;
+    const int T = whole ? 0 : syn_tile(w->nx, syn_threads(NF));
+    const int W = whole ? 32 * fl_div_up(w->nx, 32) : T + 32;
     const int rows = W < 256 ? 256 / W : 1;
-    const unsigned gx = whole ? 1 : fl_div_up(w->nx, kRowTile), gr = fl_div_up(w->ny, rows);
-    const int sl = stream_seg_len(w, S, (long long)gx * gr * NF * S, 1024 / (W * rows));
+    const unsigned gx = whole ? 1 : fl_div_up(w->nx, T), gr = fl_div_up(w->ny, rows);
+    const int sl = stream_seg_len(w, S, (long long)gx * gr * NF * S, syn_threads(NF) / (W * rows));
     const int nseg = fl_div_up(class_len(w->nz, S, 0), sl);
     k_syn_zx<NF, S><<<dim3(gx, gr, (unsigned)(nseg * NF * S)), dim3(W, rows), sizeof(float) * 2 * NF * W * rows, s>>>(
         cb, low, A, N, w->nx, w->ny, w->nz, nseg, sl, whole, w->R);
