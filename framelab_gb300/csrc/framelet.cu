@@ -739,11 +739,29 @@ static void ana_stream(fl_framelet* w, const float* in, const BandPtrs& cb, cons
                        float* low_out, int last, int mode, float tau, cudaStream_t s)
 {
     const unsigned gx = fl_div_up(w->nx, kSX), gy = fl_div_up(w->ny, kSY);
-    const int sl = stream_seg_len(w, S, (long long)gx * gy * S, ana_resident(NF, mode));
+    // Rows that are no multiple of the 32-byte sector: neighbouring tiles share sectors
+    // of every one of the 27 bands, and with three blocks an SM L2 writes them before
+    // both halves are there (160 x 150 x 170: 190 us, 140 with two blocks; 180^3 219,
+    // 143; 128 x 129 x 130 94, 75; 252 x 256 x 256 522, 422). Rows off 16 bytes in
+    // volumes far larger than L2 do best with one (250 x 256 x 256 647, 560, 486;
+    // 161 x 100 x 100 with one 64, two 60). Aligned rows want three (200^3 157, two
+    // 167), as do Haar's eight bands. Unused shared memory holds the others off.
+    int resident = ana_resident(NF, mode);
+    size_t hold = 0;
+    if (NF == 3 && mode == 0 && w->nx % 8 != 0) {
+        const bool one = w->nx % 4 != 0 && w->N * 4 * w->nbands > (400LL << 20);
+        hold = one ? 120000 : 76000;
+        if (cudaFuncSetAttribute(k_ana_stream<NF, S, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hold) ==
+            cudaSuccess)
+            resident = one ? 1 : 2;
+        else
+            hold = 0;
+    }
+    const int sl = stream_seg_len(w, S, (long long)gx * gy * S, resident);
     const int nseg = fl_div_up(class_len(w->nz, S, 0), sl);
     const dim3 grid(gx, gy, (unsigned)(nseg * S));
     if (mode == 0)
-        k_ana_stream<NF, S, 0><<<grid, kST, 0, s>>>(in, w->nx, w->ny, w->nz, nseg, sl, w->D, cb, tb, low_out, last, tau);
+        k_ana_stream<NF, S, 0><<<grid, kST, hold, s>>>(in, w->nx, w->ny, w->nz, nseg, sl, w->D, cb, tb, low_out, last, tau);
     else
         k_ana_stream<NF, S, 1><<<grid, kST, 0, s>>>(in, w->nx, w->ny, w->nz, nseg, sl, w->D, cb, tb, low_out, last, tau);
 }
