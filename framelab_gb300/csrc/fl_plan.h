@@ -245,8 +245,8 @@ int fl_plan_fan_lanes(const fl_plan* p);
 // of thread blocks on 152 SMs.
 int fl_plan_fan_block(const fl_plan* p);
 // Thread rows of a fan plan's turn and reflection backprojections (8 or 16):
-// the plan's setting (FL_TUNE_FAN_GROUPS), else 16 (batches take 8; the bits
-// are the same).
+// the plan's setting (FL_TUNE_FAN_GROUPS), else 16 where the blocks fit the GPU at
+// once or the views are many (batches take 8; the bits are the same).
 int fl_plan_fan_groups(const fl_plan* p);
 // View chunks of a cone plan's reflection backprojection where the output is
 // FP32: the plan's setting (FL_TUNE_ADJ_CHUNKS), else one per half gigabyte of

@@ -932,10 +932,24 @@ int fl_plan_adj_chunks(const fl_plan* p, bool f32_out)
 
 int fl_plan_fan_groups(const fl_plan* p)
 {
-    // 256^2, 360 views: 74.1 us with 8 thread rows, 53.9 with 16; 640^2, 720
-    // views: 322, 313; 64^2, 90 views: 19.1, 14.7
     if (p->fan_groups) return p->fan_groups;
-    return p->s.ndim == 2 && fl_plan_turns(p) > 1 ? kTurnViews : kTurnGroups;
+    const fl_scan& s = p->s;
+    const int T = fl_plan_turns(p), NR = fl_plan_refl(p);
+    if (s.ndim != 2 || T == 1) return kTurnGroups;
+    // 16 rows halve a thread's views and double the threads. They pay where their
+    // blocks all fit at once (two to an SM; the octant's 2 x 2 one, by its registers):
+    // 256^2, 360 views: 74.1 us with 8 thread rows, 53.9 with 16; 64^2, 90 views: 19.1,
+    // 14.7; 384^2, 96 views 28.6, 26.8; and in up to six times as many where the
+    // views are many (512^2, 360 views: 135, 128; 700^2 / 182, half turn and reflection
+    // 131, 125). Beyond, and with rows that few views leave idle, 8: 512^2, 32 views
+    // 20.6, 24.7; 700^2 / 96 65, 72; with the reflection too 642^2 / 24 19.5, 26.7 and
+    // 1024^2 / 360 342, 383.
+    const int P = NR ? fan_refl_pblock(NR, s.nx, s.ny) : fl_plan_fan_block(p);
+    const int hx = T == 2 ? s.nx : s.nx / 2, hy = s.ny / 2;      // primary pixels
+    const long long blocks = (long long)fl_div_up(hx, P * kFanX) * fl_div_up(hy, P);
+    const long long fit = (NR == 4 && P == 2 ? 1LL : 2LL) * p->sms;
+    const int walked = NR ? fan_refl_geom(NR, s.nv, s.na).slots : s.nv / T;
+    return blocks <= fit || (blocks <= 6 * fit && walked > 2 * kTurnViews) ? kTurnViews : kTurnGroups;
 }
 
 int fl_plan_fan_block(const fl_plan* p)
@@ -947,7 +961,7 @@ int fl_plan_fan_block(const fl_plan* p)
     long long blocks2;
     if (T > 1) {
         const int hx = T == 2 ? s.nx : s.nx / 2, hy = s.ny / 2;
-        blocks2 = (long long)fl_div_up(hx, 2) * fl_div_up(hy, 2) * fl_plan_fan_groups(p);
+        blocks2 = (long long)fl_div_up(hx, 2) * fl_div_up(hy, 2) * (p->fan_groups ? p->fan_groups : kTurnViews);
     } else {
         blocks2 = (long long)fl_div_up(s.nx, 2) * ((s.ny + 1) / 2) * s.nt * kFanGroups;
     }

@@ -267,10 +267,11 @@ enum { FL_TUNE_ADJ_RUN = 16, FL_TUNE_ADJ_ROWS = 17 };
  * fl_plan_query reads the values in effect. */
 enum { FL_TUNE_FAN_PARTS = 18, FL_TUNE_FAN_BLOCK = 19 };
 /* FL_TUNE_FAN_GROUPS: thread rows of a fan plan's turn and reflection
- * backprojections, 8 or 16 (the default of these forms; 8 for the general form,
- * which has groups of its own): a pixel block's views are split into sixteen
- * interleaved groups, one or two to a thread, added as (S_0 + S_8) + (S_1 + S_9)
- * + ... at the end, so the results do not depend on it. Batches take 8.
+ * backprojections, 8 or 16 (by default 16 for small images and for many views of
+ * larger ones; 8 for the general form, which has groups of its own): a pixel
+ * block's views are split into sixteen interleaved groups, one or two to a
+ * thread, added as (S_0 + S_8) + (S_1 + S_9) + ... at the end, so the results do
+ * not depend on it. Batches take 8.
  * fl_plan_autotune times both on turn and reflection plans. */
 enum { FL_TUNE_FAN_GROUPS = 20 };
 /* FL_TUNE_ADJ_CHUNKS: the reflection backprojection of a cone plan runs as
