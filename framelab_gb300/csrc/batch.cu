@@ -3,8 +3,9 @@
 //
 // The slices' matched-model tables stay where their plans put them; a batch
 // holds one descriptor per slice and three work lists:
-//  * rays:   chunks of 128 consecutive rays of one slice (forward, weighting),
-//  * pixels: chunks of 2 image rows x 256 columns of one slice (adjoint),
+//  * rays:   chunks of consecutive rays of one slice: 32, four threads each
+//            (forward), and 128 (weighting),
+//  * pixels: chunks of 2 image rows x 64 columns of one slice (adjoint),
 //  * vector: chunks of kVecChunk elements of one slice's image (CGLS algebra).
 // Each operator is ONE launch over its list, whatever the mix of sizes; the ray
 // and pixel lists are ordered by decreasing per-item cost (walk length, view
@@ -13,9 +14,9 @@
 // single-scan kernels (the same device code, matched_dev.cuh), so each slice's
 // result is bit-identical to its own plan's. A slice whose plan uses the half
 // or quarter turn (fl_plan_turns when the batch is created) goes through the
-// plan's turn kernels instead, on two more lists (32 rays of the views
-// iv < nv/G; 32 primary pixels); its adjoint input is packed per orbit, as
-// the plan's. So does a slice whose plan uses a reflection form (with or
+// plan's turn kernels instead, on two more lists (32 rays of the views iv < nv/G,
+// or 8 of 16 parts each; 32 primary pixel blocks); its adjoint input is packed per
+// orbit, as the plan's. So does a slice whose plan uses a reflection form (with or
 // without a turn): walked rays and primary pixels of that form.
 //
 // CGLS (solveCGLS.m:6-31) runs per slice, all slices in lockstep: every slice

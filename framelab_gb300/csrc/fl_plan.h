@@ -230,7 +230,10 @@ inline int fl_plan_refl(const fl_plan* p)
 // voxel (x < nx/2, y < ny/2, z < nz/2) under the flips of x, y and z side by
 // side, (voxel, z mirror) pairs ordered by (flip y, flip x), at 8 times
 // orbit_index (matched_dev.cuh: 2 x 2 tiles of orbits).
-// For other plans both layouts are the standard ones.
+// Elsewhere the layouts are the standard ones: the volume of a general cone plan
+// (its adjoint input has its rows fastest, as above), and the image of a fan plan,
+// whose adjoint input is standard in the general form and packed per orbit on turn
+// and reflection plans (matched_dev.cuh).
 enum {
     FL_LAY_X_FOLDED = 1,   // the volume operand is z-folded
     FL_LAY_Y_ADJ = 2       // the forward writes the adjoint-input layout
@@ -241,8 +244,8 @@ enum {
 // values when it is built).
 int fl_plan_fan_lanes(const fl_plan* p);
 // Pixels per thread side of a fan plan's backprojection (1 or 2): the plan's
-// setting (FL_TUNE_FAN_BLOCK), else 2 once the 2 x 2 blocks make four waves
-// of thread blocks on 152 SMs.
+// setting (FL_TUNE_FAN_BLOCK), else 2 once the 2 x 2 blocks and their view groups
+// make 32,768 threads.
 int fl_plan_fan_block(const fl_plan* p);
 // Thread rows of a fan plan's turn and reflection backprojections (8 or 16):
 // the plan's setting (FL_TUNE_FAN_GROUPS), else 16 where the blocks fit the GPU at

@@ -13,9 +13,12 @@
 // smallest next crossing (an incremental Siddon walk); the segment it
 // accumulates inside V is exactly w_rV above.
 //
-// Adjoint: one thread per voxel column gathers over the rays whose detector
-// window covers the column and evaluates the same w_rV from the same table
-// entries in the same frame -- the exact transpose, with no atomics.
+// Adjoint: a gather over the rays whose detector window covers a voxel column
+// (cone: the lanes of a warp along z share a block of columns, cone_adjoint.cu and
+// refl_adjoint.cu, or on turn plans a thread has a column and its turns; fan: a
+// thread has a pixel or a 2 x 2 block and one view group), evaluating the same
+// w_rV from the same table entries in the same frame -- the exact transpose,
+// with no atomics.
 #include <algorithm>
 
 #include <type_traits>
@@ -1154,8 +1157,7 @@ void launch_adj(fl_plan* p, const float* yw, void* x, const int* skip, int xfold
 #undef FL_ADJ_FAN_REFL_G
 #undef FL_ADJ_FAN_REFL
     } else if (fl_plan_turns(p) > 1) {
-        // 2 x 2 primary blocks once there are at least 4 waves of them, else
-        // one primary pixel per thread (the same bits)
+        // 2 x 2 primary blocks or primary pixels (fl_plan_fan_block; the same bits)
         const int T = fl_plan_turns(p);
         const int hx = T == 2 ? s.nx : s.nx / 2, hy = s.ny / 2;
         const int NG = fl_plan_fan_groups(p);
@@ -1482,7 +1484,7 @@ extern "C" int fl_plan_autotune(fl_plan* p, void* stream, int32_t* shapes)
         const bool turn = fl_plan_turns(p) > 1;
         for (int pass = 0; pass < 2 && !st; pass++) {
             const bool fwd = pass == 0;
-            if (fwd && !turn) continue;            // the general forward has no parts
+            if (fwd && !turn) continue;            // the general forward always has kFanParts
             float best = 3.0e38f;
             int bi = 0;
             // backprojection: pixel block 1 or 2 x view groups 8 or 16 (turn

@@ -66,8 +66,8 @@ constexpr int kReflWarps = 4;       // 2 x 2 blocks of columns per thread block
 // every lane takes the candidates one after another and visits the detector
 // rows that meet its own voxels, neighbours of the next lane's. A row's orbit
 // is loaded once for the block's columns.
-// Bound: latency, with no unit saturated (256^3, 360 views: L1 data pipe 63 %,
-// issue 49 %, 16 warps per SM at 128 registers). The form before it gave every
+// Bound: latency, with no unit saturated (256^3, 360 views: L1 data pipe 64.6 %,
+// issue 46 %, 16 warps per SM at 128 registers). The form before it gave every
 // thread a column of its own and every lane another (72 %, 54 %, 143 warp
 // instructions per weight, the column setup repeated in each thread): 10.36 ms
 // at 256^3 / 360 views, 152.4 ms at 512^3 / 720, 2.84 ms at 256^3 / 90 (half
