@@ -751,7 +751,9 @@ static void ana_stream(fl_framelet* w, const float* in, const BandPtrs& cb, cons
     if (NF == 3 && mode == 0 && w->nx % 8 != 0) {
         const bool one = w->nx % 4 != 0 && w->N * 4 * w->nbands > (400LL << 20);
         hold = one ? 120000 : 76000;
-        if (cudaFuncSetAttribute(k_ana_stream<NF, S, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hold) ==
+        // the larger one always: the attribute is the kernel's, and another thread's
+        // call between this and the launch must not lower it
+        if (cudaFuncSetAttribute(k_ana_stream<NF, S, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120000) ==
             cudaSuccess)
             resident = one ? 1 : 2;
         else
