@@ -198,18 +198,26 @@ __device__ __forceinline__ void seg_walk_dom(const ColEntry* __restrict__ ce,
         // next crossings at or before the exit planes', and the exit plane's
         // crossing is computed from the same m as v_out.
         const int budget = (dhi - dlo) + (XD ? ny : nx) + (THREE ? nzr : 0) + 2;
-#pragma unroll 1
+        // only the axes that step get a new crossing: without gathers this is
+        // shorter than walk_form's straight-line steps (the count of 512^3, 720
+        // views: 380 ms with those, 325; 256^2, 360 views 89 us, 80)
+#pragma unroll 2
         for (int it = 0; it < budget; it++) {
             const float nxt = THREE ? fminf(fminf(Ux, Uy), Uz) : fminf(Ux, Uy);
             const float seg = __fsub_rn(nxt, cur);
             const bool more = nxt < v_out;             // false at the exit (and for NaN)
-            if (Ux == nxt) { jx += px ? 1 : -1; mx = __fadd_rn(mx, px ? 1.0f : -1.0f); }
-            if (Uy == nxt) { jy += py ? 1 : -1; my = __fadd_rn(my, py ? 1.0f : -1.0f); }
-            if (THREE && Uz == nxt) { jz += pz ? 1 : -1; mz = __fadd_rn(mz, pz ? 1.0f : -1.0f); }
-            // straight-line: an axis that does not step gets the crossing it had
-            Ux = xrel(X, mx, bh, cbx);
-            Uy = xrel(Y, my, bh, cby);
-            if (THREE) Uz = xrel(Z, mz, bh, cbz);
+            if (Ux == nxt) {
+                jx += px ? 1 : -1;
+                mx = __fadd_rn(mx, px ? 1.0f : -1.0f); Ux = xrel(X, mx, bh, cbx);
+            }
+            if (Uy == nxt) {
+                jy += py ? 1 : -1;
+                my = __fadd_rn(my, py ? 1.0f : -1.0f); Uy = xrel(Y, my, bh, cby);
+            }
+            if (THREE && Uz == nxt) {
+                jz += pz ? 1 : -1;
+                mz = __fadd_rn(mz, pz ? 1.0f : -1.0f); Uz = xrel(Z, mz, bh, cbz);
+            }
             body.take(seg, more, jx, jy, jz);
             if (!more) break;
             cur = nxt;
