@@ -32,7 +32,7 @@ constexpr int kConeWarps = 4;      // 2 x 2 blocks of columns per thread block
 // columns in increasing order) and the detector rows that can meet its voxels,
 // evaluating w_rV as the forward walk does. A row's value is loaded once for
 // the block's columns, and neighbouring lanes load neighbouring rows.
-// lanes: log2 of the lanes per block (5, 4 or 3), a constant 5 with FULL.
+// lanes: log2 of the lanes per block (5 .. 2), a constant 5 with FULL.
 // Bound: issue and latency. The form before it (one thread per column and run
 // of 8 voxels, its own column set-up per view) issued 90 warp instructions per
 // useful weight of a circular scan and 183 of a helix, whose views mostly miss a
@@ -93,7 +93,7 @@ k_adj_cone(TX* __restrict__ X, const TW* __restrict__ yw, const ColEntry* __rest
         }
         const int maxw = __reduce_max_sync(gm, ahi - alo + 1);
         if (maxw <= 0) continue;
-        int lg = PB == 1 ? 2 : 3;                       // 4 .. ZL candidates per view
+        int lg = FULL ? (PB == 1 ? 2 : 3) : min(PB == 1 ? 2 : 3, lz);   // 4 .. ZL candidates per view
         while (lg < lz && (1 << lg) < maxw) lg++;
         const int W = 1 << lg;
         for (int v0 = 0; v0 < min(ZL, nvf - jb); v0 += ZL >> lg) {
@@ -214,7 +214,7 @@ void launch(fl_plan* p, const void* yw, void* x, const int* skip, int xfold, cud
         return ((long long)fl_div_up(s.nx, pb) * fl_div_up(s.ny, pb) * fl_div_up(nzw, 1 << lz) * s.nt) >>
                (5 - lz);
     };
-    auto lanes_log2 = [&](int pb) { return adj_lanes_log2(p, nzw, [&](int lz) { return warps(pb, lz); }); };
+    auto lanes_log2 = [&](int pb) { return adj_lanes_log2(p, nzw, 2, [&](int lz) { return warps(pb, lz); }); };
     const int PB = warps(2, lanes_log2(2)) >= adj_full_warps(p) ? 2 : 1, lz = lanes_log2(PB);
     const int zruns = fl_div_up(nzw, 1 << lz);
     const dim3 grid(fl_div_up(s.nx, (2 * PB) << (5 - lz)), fl_div_up(s.ny, 2 * PB), zruns * s.nt);

@@ -257,7 +257,7 @@ int fl_plan_fan_groups(const fl_plan* p);
 int fl_plan_adj_chunks(const fl_plan* p, bool f32_out);
 // Columns per side of the block a warp of the reflection backprojection owns
 // (1 or 2): the plan's setting (FL_TUNE_ADJ_RUN), else 2 once there are ten
-// warps of 2 x 2 columns per SM.
+// warps of 2 x 2 columns per SM and less than a third as many as of one.
 int fl_plan_adj_run(const fl_plan* p);
 
 // The fan forward's transposed copy of x by TMA (fan_tma.cu): false, with
@@ -300,6 +300,11 @@ void fl_matched_adjoint_refl(fl_plan* p, const void* yw, int wt, void* x, int xt
 // the general and z-mirror forms' kernels (cone_adjoint.cu)
 void fl_matched_adjoint_cone(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
                              int xfold, cudaStream_t st);
+// the kernels of the reflection, general and z-mirror forms for volumes of few
+// heights (flat_adjoint.cu), and whether they take a plan's
+void fl_matched_adjoint_flat(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,
+                             int xfold, cudaStream_t st);
+bool fl_plan_adj_flat(const fl_plan* p);
 // volume (all frames) to the z-folded layout, or back with unfold = 1
 int fl_matched_fold(fl_plan* p, const void* src, void* dst, int dtype, int unfold,
                     cudaStream_t st);

@@ -15,7 +15,8 @@
 //
 // Adjoint: a gather over the rays whose detector window covers a voxel column
 // (cone: the lanes of a warp along z share a block of columns, cone_adjoint.cu and
-// refl_adjoint.cu, or on turn plans a thread has a column and its turns; fan: a
+// refl_adjoint.cu, or a thread has a column, flat_adjoint.cu, or on turn plans a
+// column and its turns; fan: a
 // thread has a pixel or a 2 x 2 block and one view group), evaluating the same
 // w_rV from the same table entries in the same frame -- the exact transpose,
 // with no atomics.
@@ -608,7 +609,7 @@ k_adj_fan_turn(TX* __restrict__ X, const float* __restrict__ ywp,
 
 // ---------------------------------------------------------------------------
 // Half- and quarter-turn backprojections (the general, z-mirror and reflection
-// forms: cone_adjoint.cu, refl_adjoint.cu). One thread per voxel column and a
+// forms: cone_adjoint.cu, refl_adjoint.cu, flat_adjoint.cu). One thread per voxel column and a
 // run of TZ voxels in z. Per view, the thread finds the detector columns whose
 // rays can cross its column (projection of the column's four corners), and per
 // such column the xy crossing interval [l, h] of the ray family. For each voxel
@@ -1098,7 +1099,9 @@ void launch_adj_cone(fl_plan* p, const TW* yw, void* x, const int* skip, int xfo
     {
         const int nzw = s.nz / 2;
         int zruns;
-        if (fl_plan_refl(p)) {
+        if (fl_plan_adj_flat(p)) {
+            fl_matched_adjoint_flat(p, yw, dtype_of<TW>(), x, dtype_of<TX>(), skip, xfold, st);
+        } else if (fl_plan_refl(p)) {
             fl_matched_adjoint_refl(p, yw, dtype_of<TW>(), x, dtype_of<TX>(), skip, xfold, st);
         } else if (p->zmirror && p->rot && p->rot4) {
             // runs of 2: the four columns' 16 accumulators keep 8 blocks per SM
@@ -1534,6 +1537,7 @@ FL_OOB_ACCESSOR(fl_oob_matched)
 extern "C" unsigned long long fl_oob_batch(int reset);
 extern "C" unsigned long long fl_oob_refl(int reset);
 extern "C" unsigned long long fl_oob_cone(int reset);
+extern "C" unsigned long long fl_oob_flat(int reset);
 
 extern "C" int fl_debug_bounds(int64_t* violations, int reset)
 {
@@ -1541,7 +1545,7 @@ extern "C" int fl_debug_bounds(int64_t* violations, int reset)
 #ifdef FL_BOUNDS_CHECK
     FL_CUDA(cudaDeviceSynchronize());
     *violations = (int64_t)(fl_oob_matched(reset) + fl_oob_batch(reset) +
-                            fl_oob_refl(reset) + fl_oob_cone(reset));
+                            fl_oob_refl(reset) + fl_oob_cone(reset) + fl_oob_flat(reset));
     return fl_set_error(FL_OK, "");
 #else
     *violations = 0;

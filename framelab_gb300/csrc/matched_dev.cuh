@@ -717,6 +717,23 @@ __host__ __device__ inline ReflGeom refl_geom(int NR, int nv, int na, int nb)
     return g;
 }
 
+// Column of image k of voxel column (ix, iy) on a reflection form, in the order
+// the backprojection takes them: C_k = S^k V0 for k < NR, then D_k = S^(k-NR) M
+// V0, with S = R^(4/NR), R (x, y) = (n-1-y, x), M (x, y) = (x, ny-1-y).
+template <int NR>
+__device__ __forceinline__ void refl_column(int k, int ix, int iy, int nx, int ny, int& px,
+                                            int& py)
+{
+    const int y0 = k < NR ? iy : ny - 1 - iy, t = k % NR;
+    if (NR == 4) {
+        px = t == 0 ? ix : t == 1 ? nx - 1 - y0 : t == 2 ? nx - 1 - ix : y0;
+        py = t == 0 ? y0 : t == 1 ? ix : t == 2 ? ny - 1 - y0 : ny - 1 - ix;
+    } else {
+        px = t == 0 ? ix : nx - 1 - ix;
+        py = t == 0 ? y0 : ny - 1 - y0;
+    }
+}
+
 // Fan reflection forms (fl_plan::refl on a fan plan, NR = 1, 2 or 4): with
 // M (x, y) = (x, ny-1-y), S = the identity (NR = 1), the half turn R^2 (NR =
 // 2) or the quarter turn R (NR = 4) and q = nv/NR, the walked views v = 0 ..
@@ -1098,18 +1115,18 @@ inline DetGrid det_grid(const fl_plan* p)
 }
 
 // Lanes per block of columns of the cone backprojections with lanes along z, as a
-// log2: 32 lanes, or 16 or 8 where that leaves at least a quarter fewer of them
+// log2: 32 lanes, or fewer (down to 2^least) where that leaves at least a quarter fewer of them
 // without one of the nzw voxels and the warps (a function of the log2) still fill the
 // GPU, ten per SM (reflection form, 512 x 512 x 32, 90 views: 1.94 ms with 32 lanes,
 // 1.18 with 16; 64 x 64 x 16, 360 views: 0.53 with 32, 0.69 with 8).
 inline long long adj_full_warps(const fl_plan* p) { return 10LL * p->sms; }
 
 template <typename Warps>
-inline int adj_lanes_log2(const fl_plan* p, int nzw, Warps warps)
+inline int adj_lanes_log2(const fl_plan* p, int nzw, int least, Warps warps)
 {
     auto lanes = [&](int lz) { return fl_div_up(nzw, 1 << lz) << lz; };
     int lz = 5;
-    while (lz > 3 && 4 * lanes(lz - 1) <= 3 * lanes(lz) && warps(lz - 1) >= adj_full_warps(p)) lz--;
+    while (lz > least && 4 * lanes(lz - 1) <= 3 * lanes(lz) && warps(lz - 1) >= adj_full_warps(p)) lz--;
     return lz;
 }
 

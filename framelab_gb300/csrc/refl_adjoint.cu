@@ -8,23 +8,6 @@
 
 namespace {
 
-// Column of image k of voxel column (ix, iy) on a reflection form, in the order
-// the backprojection takes them: C_k = S^k V0 for k < NR, then D_k = S^(k-NR) M
-// V0, with S = R^(4/NR), R (x, y) = (n-1-y, x), M (x, y) = (x, ny-1-y).
-template <int NR>
-__device__ __forceinline__ void refl_column(int k, int ix, int iy, int nx, int ny, int& px,
-                                            int& py)
-{
-    const int y0 = k < NR ? iy : ny - 1 - iy, t = k % NR;
-    if (NR == 4) {
-        px = t == 0 ? ix : t == 1 ? nx - 1 - y0 : t == 2 ? nx - 1 - ix : y0;
-        py = t == 0 ? y0 : t == 1 ? ix : t == 2 ? ny - 1 - y0 : ny - 1 - ix;
-    } else {
-        px = t == 0 ? ix : nx - 1 - ix;
-        py = t == 0 ? y0 : ny - 1 - y0;
-    }
-}
-
 // Lower corner of image k of the PB x PB block of columns at (X0, Y0).
 template <int NR, int PB>
 __device__ __forceinline__ void refl_corner(int k, int X0, int Y0, int nx, int ny, int& bx,
@@ -66,8 +49,8 @@ constexpr int kReflWarps = 4;       // 2 x 2 blocks of columns per thread block
 // every lane takes the candidates one after another and visits the detector
 // rows that meet its own voxels, neighbours of the next lane's. A row's orbit
 // is loaded once for the block's columns.
-// Bound: latency, with no unit saturated (256^3, 360 views: L1 data pipe 64.6 %,
-// issue 46 %, 16 warps per SM at 128 registers). The form before it gave every
+// Bound: latency, with no unit saturated (256^3, 360 views: L1 data pipe 64.7 %,
+// issue 47 %, 16 warps per SM at 128 registers). The form before it gave every
 // thread a column of its own and every lane another (72 %, 54 %, 143 warp
 // instructions per weight, the column setup repeated in each thread): 10.36 ms
 // at 256^3 / 360 views, 152.4 ms at 512^3 / 720, 2.84 ms at 256^3 / 90 (half
@@ -338,7 +321,7 @@ long long warp_count(const fl_plan* p, int PB, int lz)
 
 int lanes_log2(const fl_plan* p, int PB)
 {
-    return adj_lanes_log2(p, p->s.nz / 2, [&](int lz) { return warp_count(p, PB, lz); });
+    return adj_lanes_log2(p, p->s.nz / 2, 3, [&](int lz) { return warp_count(p, PB, lz); });
 }
 
 template <typename TX, typename TW>
@@ -375,11 +358,14 @@ void launch(fl_plan* p, const void* yw, void* x, const int* skip, int xfold, cud
 // 2 x 2 columns per warp load a row's orbit once for all of them, but make a
 // quarter of the warps: they pay once those fill the GPU (160^3, 200 views:
 // 1.46 ms against 1.59 with one column; 128^3, 120 views, 1,056 warps: 0.74
-// against 0.49).
+// against 0.49). A warp takes three times as long, so not where more of its lanes
+// have no voxel than one column's would (256 x 256 x 24, 360 views: 1.00 ms with 32
+// lanes, 0.71 with 16 and one column).
 int fl_plan_adj_run(const fl_plan* p)
 {
     if (p->adj_run) return p->adj_run;
-    return warp_count(p, 2, lanes_log2(p, 2)) >= adj_full_warps(p) ? 2 : 1;
+    const long long w2 = warp_count(p, 2, lanes_log2(p, 2)), w1 = warp_count(p, 1, lanes_log2(p, 1));
+    return w2 >= adj_full_warps(p) && 3 * w2 < w1 ? 2 : 1;
 }
 
 void fl_matched_adjoint_refl(fl_plan* p, const void* yw, int wt, void* x, int xt, const int* skip,

@@ -249,7 +249,8 @@ int fl_plan_query(const fl_plan *plan, int option, int *value);
 int fl_plan_autotune(fl_plan *plan, void *stream, int32_t *shapes);
 /* FL_TUNE_ADJ_RUN: columns per side of the block of voxel columns a warp of the
  * reflection backprojection owns (1 or 2; by default 2 once such warps fill the
- * GPU). fl_plan_autotune times both and keeps the faster; fl_plan_option sets it
+ * GPU; volumes of few heights take a column per thread instead, with
+ * FL_TUNE_ADJ_CHUNKS at most 1). fl_plan_autotune times both and keeps the faster; fl_plan_option sets it
  * (other values are refused), fl_plan_query reads the value in effect. The
  * results do not depend on it. FL_TUNE_ADJ_ROWS (1 .. 3) is accepted and read
  * back, and selects nothing: the kernel's row loop has one form. */
