@@ -258,7 +258,8 @@ void launch(fl_plan* p, const void* yw, void* x, const int* skip, int xfold, cud
 // 211, two 248, 284; 192^2, 45 views, three 98, 90, four 98, 109; 384^2 six 300, 285;
 // 512^2 six 480, 471; half turn with the reflection, 90 views, 192^2 one 107, 109, two
 // 112, 154; 256^2 three 168, 158, four 168, 170; 512^2 six 465, 452; quarter turns,
-// 48 views, 256^2 two 102, 98, six 109, 121; 512^2 four 212, 175).
+// 48 views, 256^2 two 102, 98, six 109, 121; 512^2 four 212, 175). Where the
+// runs of all frames are more than a grid's z holds, the lanes' one run per frame fits.
 bool fl_plan_adj_flat(const fl_plan* p)
 {
     const fl_scan& s = p->s;
@@ -266,6 +267,7 @@ bool fl_plan_adj_flat(const fl_plan* p)
     if (s.ndim != 3 || (!NR && p->zmirror && p->rot) || (NR && p->adj_chunks > 1)) return false;
     const int h = p->zmirror ? s.nz / 2 : s.nz;
     const long long area = (long long)s.nx * s.ny * s.nt / (NR ? 2 : 1);
+    if ((long long)fl_div_up(h, NR ? kFlatRefl : kFlatCone) * s.nt > 65535) return false;
     return area >= (1 << 14) && h <= (area < (1 << 15) ? 1 : area < (1 << 16) ? 3 : 6);
 }
 

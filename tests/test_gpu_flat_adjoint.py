@@ -78,3 +78,20 @@ def test_frames():
         want = O.exact_adjoint(one.reshape(-1), q, threads=os.cpu_count() or 1).reshape(-1)
         e = np.linalg.norm(x[t] - want) / np.linalg.norm(want)
         assert e < 5e-6, (t, e)
+
+
+def test_more_frames_than_two_runs_each_fit_a_grid():
+    """5 heights are two runs a frame; 32768 frames of one view, their sum is one frame's."""
+    import torch
+    from framelab_gb300.projector import Plan
+    n, nv = 8, 32768
+    q = _para(n, 5, n, 6, nv)
+    p = dict(q, nt=np.uint32(nv), id_X=np.arange(nv, dtype=np.uint32),
+             id_Y=np.arange(nv, dtype=np.uint32).reshape(1, nv), Nv=np.ones(nv, np.uint32),
+             tmp_size=np.uint32(1))
+    P = Plan(p)
+    r = np.random.default_rng(7).standard_normal(P.n_rays).astype(np.float32)
+    x = P.adjoint(torch.from_numpy(r).cuda()).double().reshape(nv, -1).sum(0).cpu().numpy()
+    want = O.exact_adjoint(r, q, threads=os.cpu_count() or 1).reshape(-1)
+    e = np.linalg.norm(x - want) / np.linalg.norm(want)
+    assert e < 5e-6, e
